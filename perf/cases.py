@@ -1,0 +1,692 @@
+"""What the engine is measured on: steps of serving, through the engine's own entry points.
+
+Every case is work that a server of this engine does all day: a prompt that is computed, a batch of requests that
+decodes one token each, a portion of a prompt beside decoding requests, a short generation from prompt to last token.
+A pass goes through ``LLM.model_runner`` as the engine's request loop does (``run`` for steps with prompt tokens, which
+reads the chosen tokens at once; ``launch`` for decode steps, whose tokens are read after the next step was launched),
+from host token lists to float32 logits on the device.  The tokens of a decode step are given instead of fed back, so
+that two implementations whose logits differ in the last bits still compute the same thing.
+
+Weights are random, by the engine's own rule for random weights (one draw per tensor of the checkpoint, seeded by name).
+Models are the configurations that ``bench.py`` names, cut to a few layers: the 8B-shaped Qwen3 to 6 layers and the
+0.6B-shaped one to 8, with the vocabulary cut in the same proportion so that the head keeps its share of a step, and
+the designs of width 1,024 and 2,048 to their one round of four layers.  Of the seven designs four stand here; the other
+three run the same kernels in other places (mixtures of experts, latents, windows, filters, recurrences with a decay).
+"""
+from __future__ import annotations
+
+import hashlib
+import json
+import math
+import os
+import random
+import tempfile
+
+import torch
+
+PAGE = 256
+BUDGET = 8192           # tokens of one step while contexts are being filled
+
+
+# ---------------------------------------------------------------- models
+def _qwen3(hidden, layers, heads, kv_heads, ff, vocab, tied):
+    return dict(architectures=["Qwen3ForCausalLM"], model_type="qwen3", hidden_size=hidden, num_hidden_layers=layers,
+                num_attention_heads=heads, num_key_value_heads=kv_heads, head_dim=128, intermediate_size=ff,
+                vocab_size=vocab, rope_theta=1000000.0, rms_norm_eps=1e-6, tie_word_embeddings=tied,
+                max_position_embeddings=40960, torch_dtype="bfloat16", hidden_act="silu", attention_bias=False)
+
+
+def _muvonex(width):
+    heads, ff = width // 128, width * 11 // 4
+    mlp = dict(kind="dense", ff=ff)
+    delta = dict(type="delta", mlp=mlp, mixer=dict(heads=heads, kv_heads=heads // 2, dim=128, vdim=128, conv=4))
+    par = dict(type="parallel", mlp=mlp, mixer=dict(
+        left=dict(heads=heads, kv_heads=heads // 4, dim=128, vdim=128, scale=128 ** -0.5,
+                  rot=dict(base=500000.0, dims=128, scaling=dict(factor=8.0, low=1.0, high=4.0, original=8192))),
+        right=dict(heads=2 * heads, groups=1, state=128, vdim=64, conv=4, norm_groups=1),
+        left_scale=1.0, right_scale=1.0))
+    return dict(architecture="Muvonex", vocab=32000, width=width, embedding=dict(scale=1.0), norm=dict(eps=1e-6),
+                residual_mult=1.0, layers=[delta, delta, delta, par], dtype="bfloat16")
+
+
+def _nomudra(width):
+    heads, ff = width // 128, width * 11 // 4
+    moe = dict(kind="moe", router=dict(experts=16, identity=2, top=4, groups=dict(count=3, keep=2)),
+               expert=dict(ff=ff * 2 // 11, limit=7.0), shared=dict(ff=ff * 3 // 11, limit=7.0))
+    attention = dict(type="attention", mlp=moe, mixer=dict(
+        heads=heads, kv_heads=heads // 4, dim=128, vdim=128, scale=128 ** -0.5, rot=dict(base=500000.0, dims=64),
+        mask=dict(size=4096)))
+    mlstm = dict(type="mlstm", mlp=moe, mixer=dict(heads=heads // 2, dim=128, vdim=256, gate_cap=15.0))
+    return dict(architecture="Nomudra", vocab=32000, width=width, norm=dict(eps=1e-6),
+                layers=[attention, mlstm, attention, mlstm], dtype="bfloat16")
+
+
+def _ginodra(width):
+    heads, ff = width // 128, width * 11 // 4
+    dense = dict(kind="dense", ff=ff * 3 // 2)
+    latent = dict(type="latent_attention", mlp=dense, mixer=dict(
+        heads=heads, dim=128, rot_dim=64, vdim=128, q_rank=width * 3 // 8, kv_rank=512, scale=192 ** -0.5,
+        rot=dict(base=10000.0, dims=64)))
+    window = dict(heads=heads, kv_heads=heads // 4, dim=128, vdim=128, scale=128 ** -0.5, mask=dict(size=1024))
+    delta = dict(type="general_delta", mlp=dense, mixer=dict(heads=width // 64, dim=64, decay_rank=64))
+    return dict(architecture="Ginodra", vocab=32000, width=width, norm=dict(eps=1e-6, groups=4), residual_mult=1.0,
+                canon=dict(taps=3), logit_scale=1.0, logit_softcap=30.0, dtype="bfloat16",
+                layers=[latent, dict(type="attention", mlp=dense, mixer=window), delta,
+                        dict(type="attention", mlp=dense, mixer=dict(window, kv_from=1))])
+
+
+MODELS = {
+    "qwen3_8b": _qwen3(4096, 6, 32, 8, 12288, 25344, False),
+    "qwen3_0.6b": _qwen3(1024, 8, 16, 8, 3072, 43392, True),
+    "muvonex_1k": _muvonex(1024), "muvonex_2k": _muvonex(2048),
+    "nomudra_1k": _nomudra(1024), "nomudra_2k": _nomudra(2048),
+    "ginodra_1k": _ginodra(1024), "ginodra_2k": _ginodra(2048),
+}
+
+
+# ---------------------------------------------------------------- cases
+# kind        one pass
+# prompt      ``requests`` prompts of ``shortest`` to ``longest`` tokens in one step; the logits of each one's last token
+# decode      one decode step of ``requests`` requests that hold ``shortest`` to ``longest`` tokens
+# mixed       one step: ``portion`` tokens of a prompt behind the ``before`` that are cached, beside a decode step as above
+# generate    ``requests`` prompts in one step, then ``new`` decode steps; the logits of every step
+def _case(name, model, kind, requests, shortest, longest, dtype="bfloat16", portion=0, before=0, new=0):
+    case = dict(model=model, kind=kind, requests=requests, shortest=shortest, longest=longest, dtype=dtype,
+                portion=portion, before=before, new=new)
+    return dict(case, name=name) if name else case
+
+
+def listed():
+    return [
+        # the smallest call: one short chat on the small model, where launches and latency count
+        _case("small_chat_decode_1", "qwen3_0.6b", "decode", 1, 181, 181),
+        # the headline: eight requests around 2,048 tokens of context on the 8B-shaped layers
+        _case("decode_8", "qwen3_8b", "decode", 8, 2048, 2060),
+        # a busy server: 64 requests of unlike length
+        _case("decode_64", "qwen3_8b", "decode", 64, 130, 2900),
+        # the largest decode batch: continuous batching on the small model, contexts from 64 to 4,096
+        _case("small_decode_256", "qwen3_0.6b", "decode", 256, 64, 4095),
+        # time to first token of one 2,048-token prompt
+        _case("prompt_2048", "qwen3_8b", "prompt", 1, 2048, 2048),
+        # chunked prefill: a portion of a long prompt beside requests that decode
+        _case("portion_beside_23", "qwen3_8b", "mixed", 23, 200, 2500, portion=1001, before=1024),
+        # the 32-bit path, as used to check a checkpoint's numerics: a few ragged prompts
+        _case("float32_prompts", "qwen3_0.6b", "prompt", 3, 37, 210, dtype="float32"),
+        # one long prompt through gated delta rules, a state space and attention with a sink
+        _case("muvonex_prompt_4096", "muvonex_2k", "prompt", 1, 4096, 4096),
+        # eight short chats from prompt to answer on the same model
+        _case("muvonex_generate_8", "muvonex_2k", "generate", 8, 19, 300, new=16),
+        # several documents at once through a mixture of experts, chunked attention and mLSTMs
+        _case("nomudra_prompts_5", "nomudra_2k", "prompt", 5, 333, 1501),
+        # 48 chats at once on the same model: prompts, then decode steps that touch every expert
+        _case("nomudra_generate_48", "nomudra_2k", "generate", 48, 11, 150, new=12),
+        # latents, windows and the generalised delta rule: medium prompts, then answers
+        _case("ginodra_generate_6", "ginodra_2k", "generate", 6, 301, 1403, new=16),
+    ]
+
+
+def _spread(rng, low, high):
+    """A whole number between the two, spread over its logarithm."""
+    return int(round(math.exp(rng.uniform(math.log(low), math.log(high)))))
+
+
+def draw(rng):
+    kind = rng.choice(["decode", "decode", "prompt", "prompt", "mixed", "generate", "generate", "float32"])
+    if kind == "decode":
+        model = rng.choice(["qwen3_8b", "qwen3_0.6b"])
+        n = _spread(rng, 1, 64 if model == "qwen3_8b" else 256)
+        longest = _spread(rng, 100, 2900 if model == "qwen3_8b" else min(4095, 540000 // n))
+        return _case(None, model, "decode", n, max(1, int(longest * rng.uniform(0.05, 1.0))), longest)
+    if kind == "mixed":
+        n = _spread(rng, 1, 48)
+        longest = _spread(rng, 100, 2500)
+        return _case(None, "qwen3_8b", "mixed", n, max(1, int(longest * rng.uniform(0.05, 1.0))), longest,
+                     portion=_spread(rng, 16, 1500), before=rng.choice([0, _spread(rng, 16, 2000)]))
+    if kind == "float32":
+        longest = _spread(rng, 16, 210)
+        return _case(None, "qwen3_0.6b", "prompt", rng.randint(1, 3), max(1, longest // rng.randint(1, 4)), longest,
+                     dtype="float32")
+    if kind == "prompt":
+        model = rng.choice(["qwen3_8b", "qwen3_0.6b", "muvonex_1k", "muvonex_2k", "nomudra_1k", "nomudra_2k",
+                            "ginodra_1k", "ginodra_2k"])
+        n = _spread(rng, 1, 8)
+        longest = _spread(rng, 16, (2048 if model == "qwen3_8b" else 4096) // n)
+        return _case(None, model, "prompt", n, max(2, int(longest * rng.uniform(0.2, 1.0))), longest)
+    model = rng.choice(["qwen3_0.6b", "muvonex_1k", "muvonex_2k", "nomudra_1k", "nomudra_2k", "ginodra_1k", "ginodra_2k"])
+    n = _spread(rng, 1, 48)
+    longest = _spread(rng, 8, 4096 // n if n < 16 else 150)
+    return _case(None, model, "generate", n, max(2, int(longest * rng.uniform(0.1, 1.0))), longest, new=rng.randint(4, 16))
+
+
+def _lengths(case):
+    """The requests' lengths: evenly spread between the shortest and the longest, in a mixed order."""
+    n, low, high = case["requests"], case["shortest"], case["longest"]
+    lens = [high if n == 1 else low + (high - low) * i // (n - 1) for i in range(n)]
+    random.Random(n).shuffle(lens)
+    return lens
+
+
+def _tokens(case, seed):
+    """Token ids of every request: all that it holds at the end of a pass; and those of the prompt that is cut up."""
+    gen = torch.Generator().manual_seed(seed)
+    cfg = MODELS[case["model"]]
+    vocab = cfg.get("vocab_size") or cfg["vocab"]
+    extra = {"decode": 1, "mixed": 1, "prompt": 0, "generate": case["new"]}[case["kind"]]
+    rows = [torch.randint(0, vocab, (n + extra,), generator=gen).tolist() for n in _lengths(case)]
+    cut = torch.randint(0, vocab, (case["before"] + case["portion"],), generator=gen).tolist()
+    return rows, cut
+
+
+def prepare(case, seed):
+    from nanohybrid_vlm_b200 import LLM
+    from nanohybrid_vlm_b200.engine import StepItem
+
+    rows, cut = _tokens(case, seed)
+    held = [len(r) for r in rows] + ([len(cut)] if cut else [])
+    pages = sum(-(-(n + 1) // PAGE) for n in held) + 2
+    with tempfile.TemporaryDirectory() as folder:
+        with open(os.path.join(folder, "config.json"), "w") as f:
+            json.dump(MODELS[case["model"]], f)
+        llm = LLM(folder, random_weights_seed=seed, kvcache_block_size=PAGE, num_kvcache_blocks=pages,
+                  max_model_len=max(4352, max(held) + 1), max_num_seqs=max(8, len(held)), max_num_batched_tokens=BUDGET,
+                  dtype=case["dtype"])
+    runner, kind = llm.model_runner, case["kind"]
+    state = dict(llm=llm, runner=runner, kind=kind, rows=rows, flight=None, new=case["new"])
+    ids = list(range(len(rows)))
+    if kind in ("decode", "mixed"):
+        # the contexts, filled as a server fills them: whole prompts, several to a step
+        fill = [(i, r[:-1]) for i, r in enumerate(rows)] + ([("cut", cut[:case["before"]])] if case["before"] else [])
+        step, room = [], BUDGET
+        for req, tokens in fill:
+            runner.cache.allocate(req, len(tokens) + (1 if req != "cut" else case["portion"]))
+            if len(tokens) > room:
+                runner.step(step)
+                step, room = [], BUDGET
+            step.append(StepItem(req, tokens, 0, []))
+            room -= len(tokens)
+        if step:
+            runner.step(step)
+        items = [StepItem(i, [r[-1]], len(r) - 1, [0]) for i, r in enumerate(rows)]
+        sampling = [(0.0, i, len(r)) for i, r in enumerate(rows)]
+        if kind == "mixed":
+            if not case["before"]:
+                runner.cache.allocate("cut", case["portion"])
+            items.insert(0, StepItem("cut", cut[case["before"]:], case["before"], [case["portion"] - 1]))
+            sampling.insert(0, (0.0, len(rows), len(cut)))
+        state.update(items=items, sampling=sampling)
+    else:
+        new = case["new"]
+        first = [StepItem(i, r[:len(r) - new], 0, [len(r) - new - 1]) for i, r in zip(ids, rows)]
+        state.update(ids=ids, first=first, first_sampling=[(0.0, i, len(r) - new) for i, r in zip(ids, rows)])
+    return state
+
+
+def run(state):
+    runner, kind = state["runner"], state["kind"]
+    if kind == "mixed":
+        runner.run(state["items"], state["sampling"])
+        return runner.last_logits
+    if kind == "decode":
+        flight = runner.launch(state["items"], state["sampling"])
+        logits = runner.last_logits
+        if state["flight"] is not None:
+            state["flight"].read()          # the tokens of the step before, as the request loop reads them
+        state["flight"] = flight
+        return logits
+    from nanohybrid_vlm_b200.engine import StepItem
+    for i, r in zip(state["ids"], state["rows"]):
+        runner.cache.allocate(i, len(r))
+    runner.run(state["first"], state["first_sampling"])
+    out, flight, new = [runner.last_logits], None, state["new"]
+    for k in range(new):
+        starts = [len(r) - new + k for r in state["rows"]]
+        items = [StepItem(i, [r[s]], s, [0]) for i, r, s in zip(state["ids"], state["rows"], starts)]
+        launched = runner.launch(items, [(0.0, i, s + 1) for i, s in zip(state["ids"], starts)])
+        out.append(runner.last_logits.clone())
+        if flight is not None:
+            flight.read()
+        flight = launched
+    if flight is not None:
+        flight.read()
+    for i in state["ids"]:
+        runner.cache.free(i)
+    return out
+
+
+# ---------------------------------------------------------------- what a pass cannot do without
+def _layer_numbers(cfg):
+    """Per layer: weights that every token uses, (experts, weights of one, used by a token), bytes of a cached token,
+    bytes of a request's state, multiply-adds of the mixer per token beside its matrices, attention (heads, d, dv, reach)."""
+    if "architectures" in cfg:
+        W, H, G, d, ff = (cfg["hidden_size"], cfg["num_attention_heads"], cfg["num_key_value_heads"], cfg["head_dim"],
+                          cfg["intermediate_size"])
+        return [((H + 2 * G) * d * W + H * d * W + 3 * ff * W, None, 4 * G * d, 0, 0, (H, d, d, None))] \
+            * cfg["num_hidden_layers"]
+    W, out = cfg["width"], []
+    for layer in cfg["layers"]:
+        m, mlp, kind = layer["mixer"], layer["mlp"], layer["type"]
+        cached = state = scan = 0
+        att = None
+        if kind == "delta":
+            H, G, d, dv = m["heads"], m["kv_heads"], m["dim"], m["vdim"]
+            mix, state, scan = (2 * G * d + 3 * H * dv + 2 * H) * W, 4 * H * d * dv, 3 * H * d * dv
+        elif kind == "parallel":
+            a, s = m["left"], m["right"]
+            H, G, d = a["heads"], a["kv_heads"], a["dim"]
+            inner = s["heads"] * s["vdim"]
+            mix = (2 * H * d + 2 * G * d + 3 * inner + 2 * s["groups"] * s["state"] + s["heads"]) * W
+            cached, att = 4 * G * d, (H, d, d, None)
+            state, scan = 4 * inner * s["state"], 2 * inner * s["state"]
+        elif kind == "mlstm":
+            H, d, dv = m["heads"], m["dim"], m["vdim"]
+            mix, state, scan = (2 * H * d + 3 * H * dv + 2 * H) * W, 4 * H * d * (dv + 1), 2 * H * d * (dv + 1)
+        elif kind == "latent_attention":
+            H, d, r, dv, q, c = m["heads"], m["dim"], m["rot_dim"], m["vdim"], m["q_rank"], m["kv_rank"]
+            mix = (q + c + r + H + H * dv) * W + H * (d + r) * q + H * (d + dv) * c
+            cached, att = 2 * (c + r), (H, d + r, dv, None)
+        elif kind == "general_delta":
+            n, d = m["heads"] * m["dim"], m["dim"]
+            mix, state, scan = (6 * n + m["decay_rank"]) * W + n * m["decay_rank"], 4 * n * d, 4 * n * d
+        else:
+            H, G, d = m["heads"], m["kv_heads"], m["dim"]
+            nomudra = "rot" in m
+            mix = (2 * H * d + (H * d if nomudra else H) + (0 if m.get("kv_from") is not None else (1 if nomudra else 2)
+                                                               * G * d)) * W
+            cached, att = 4 * G * d, (H, d, d, m["mask"]["size"])
+        moe = None
+        if mlp["kind"] == "moe":
+            r = mlp["router"]
+            moe = (r["experts"], 3 * mlp["expert"]["ff"] * W, r["top"])
+            mix += (r["experts"] + r["identity"] + 1) * W + 3 * mlp["shared"]["ff"] * W
+        else:
+            mix += (2 if "canon" in cfg else 3) * mlp["ff"] * W
+        out.append((mix, moe, cached, state, scan, att))
+    return out
+
+
+def _step_work(cfg, item, spans, rows):
+    """Bytes and operations of one step whose requests bring the tokens [start, end) of ``spans``."""
+    W, V = (cfg.get("hidden_size") or cfg["width"]), (cfg.get("vocab_size") or cfg["vocab"])
+    T = sum(e - s for s, e in spans)
+    moved, flops = V * W * item + T * W * item + rows * V * 4, 2.0 * rows * V * W
+    for weights, moe, cached, state, scan, att in _layer_numbers(cfg):
+        flops += 2.0 * T * (weights + scan)
+        moved += weights * item + sum(state * (2 if s else 1) for s, _ in spans)
+        if moe is not None:
+            experts, size, top = moe
+            flops += 2.0 * T * top * size
+            moved += min(experts, T * top) * size * item
+        if att is not None:
+            H, d, dv, reach = att
+            for s, e in spans:
+                keys = sum(min(p + 1, reach) for p in range(s, e)) if reach else (s + 1 + e) * (e - s) / 2
+                flops += 2.0 * H * (d + dv) * keys
+                seen = e if reach is None else min(e, e - s + reach - 1)
+                moved += (seen + e - s) * cached * item / 2
+    return moved, flops
+
+
+def work(case):
+    cfg, item = MODELS[case["model"]], (2 if case["dtype"] == "bfloat16" else 4)
+    lens, kind = _lengths(case), case["kind"]
+    if kind in ("decode", "mixed"):
+        steps = [[(n, n + 1) for n in lens]]
+        if kind == "mixed":
+            steps[0].append((case["before"], case["before"] + case["portion"]))
+    else:
+        steps = [[(0, n) for n in lens]] + [[(n + k, n + k + 1) for n in lens] for k in range(case["new"])]
+    totals = [_step_work(cfg, item, spans, len(spans)) for spans in steps]
+    return {"bytes": sum(m for m, _ in totals), "flops": sum(f for _, f in totals)}
+
+
+def tolerance(case):
+    """About four times what the same step shows with its sums in another order (a batch against its requests one by one,
+    a prompt against its portions), at most 0.03.  Random layers of the 8B width are the most sensitive: 0.017 there,
+    0.010 at the 0.6B width, 0.005 (Muvonex), 0.0015 (Nomudra, whose router may choose another expert for single tokens:
+    the largest difference of one value is large).  In 32 bits the sums agree to 2e-6 with 64 bits."""
+    if case["dtype"] == "float32":
+        return {"rel": 1e-5, "max": 1e-4}
+    design = case["model"].split("_")[0]
+    return {"qwen3": {"rel": 0.03, "max": 0.4}, "muvonex": {"rel": 0.02, "max": 0.2},
+            "nomudra": {"rel": 0.008, "max": 0.5}, "ginodra": {"rel": 0.02, "max": 0.2}}[design]
+
+
+# ---------------------------------------------------------------- the same in 64 bits
+class _Weights:
+    """The tensors of a random model by the engine's rule: every tensor of the checkpoint is one float32 draw from a
+    generator on the device seeded by (seed, name), rounded to the model's type."""
+
+    def __init__(self, seed, dtype):
+        self.seed, self.dtype, self.kept = seed, dtype, {}
+
+    def __call__(self, name, *shape, std=0.02, mean=0.0, exact=False):
+        if name not in self.kept:
+            digest = hashlib.sha256(f"{self.seed}:{name}".encode()).digest()
+            gen = torch.Generator(device="cuda").manual_seed(int.from_bytes(digest[:8], "little") & 0x7FFFFFFFFFFFFFFF)
+            t = torch.empty(shape, dtype=torch.float32, device="cuda").normal_(0.0, std, generator=gen) + mean
+            self.kept[name] = (t if exact else t.to(self.dtype)).double()
+        return self.kept[name]
+
+    def norm(self, name, *shape):
+        return self(name, *shape, std=0.01, mean=1.0)
+
+    def small(self, name, *shape, exact=False):
+        return self(name, *shape, std=0.01, exact=exact)
+
+
+def _unit_rms(x, eps):
+    return x / torch.sqrt((x * x).mean(-1, keepdim=True) + eps)
+
+
+def _rotate(x, pos, freq):
+    """x [T, heads, d]: the first 2 * len(freq) elements of a head turn, element i with element i + len(freq)."""
+    half = len(freq)
+    ang = pos[:, None].double() * torch.tensor(freq, dtype=torch.float64, device=x.device)[None, :]
+    c, s = ang.cos()[:, None], ang.sin()[:, None]
+    a, b = x[..., :half], x[..., half:2 * half]
+    return torch.cat([a * c - b * s, b * c + a * s, x[..., 2 * half:]], -1)
+
+
+def _freq(dims, base, bands=None):
+    out = [base ** (-2.0 * i / dims) for i in range(dims // 2)]
+    for i, f in enumerate(out if bands else []):
+        length = 2.0 * math.pi / f
+        if length > bands["original"] / bands["low"]:
+            out[i] = f / bands["factor"]
+        elif length >= bands["original"] / bands["high"]:
+            s = (bands["original"] / length - bands["low"]) / (bands["high"] - bands["low"])
+            out[i] = (1.0 - s) * f / bands["factor"] + s * f
+    return out
+
+
+def _attend(q, k, v, scale, reach=None, chunk=None, sink=None, slope=None):
+    """q [T, H, d], k [T, G, d], v [T, G, dv] of one request, causal."""
+    T, H, G = q.shape[0], q.shape[1], k.shape[1]
+    out = torch.empty(T, H, v.shape[-1], dtype=torch.float64, device=q.device)
+    j = torch.arange(T, device=q.device)
+    for r0 in range(0, T, 1024):
+        i = j[r0:r0 + 1024, None]
+        hidden = (j[None] > i)
+        if reach:
+            hidden |= i - j[None] >= reach
+        if chunk:
+            hidden |= i // chunk != j[None] // chunk
+        for g in range(G):
+            heads = slice(g * (H // G), (g + 1) * (H // G))
+            s = torch.einsum("ihd,jd->hij", q[r0:r0 + 1024, heads], k[:, g]) * scale
+            if slope is not None:
+                s = s - slope[heads, None, None] * (i - j[None])
+            s = s.masked_fill(hidden, -math.inf)
+            if sink is not None:
+                s = torch.cat([s, sink[heads, None, None].expand(-1, s.shape[1], 1)], -1)
+            p = torch.softmax(s, -1)[..., :T]
+            out[r0:r0 + 1024, heads] = torch.einsum("hij,jd->ihd", p, v[:, g])
+    return out
+
+
+def _taps(x, spans, weight, bias=None):
+    """A causal filter over time, one per channel, for every request by itself; the last tap meets the current token."""
+    out = torch.empty_like(x)
+    K = weight.shape[1]
+    for a, b in spans:
+        padded = torch.cat([x.new_zeros(K - 1, x.shape[1]), x[a:b]])
+        out[a:b] = sum(padded[j:j + b - a] * weight[:, j] for j in range(K))
+    return out if bias is None else out + bias
+
+
+def _padded(x, spans):
+    """Packed rows as [longest, requests, ...], zeros behind the shorter ones."""
+    return torch.nn.utils.rnn.pad_sequence([x[a:b] for a, b in spans])
+
+
+def _packed(x, spans):
+    return torch.cat([x[:b - a, i] for i, (a, b) in enumerate(spans)])
+
+
+def _per_request(spans, fn, *tensors):
+    return torch.cat([fn(*(t[a:b] for t in tensors)) for a, b in spans])
+
+
+def _silu(x):
+    return x * torch.sigmoid(x)
+
+
+def _qwen3_exact(cfg, w, ids, pos, spans, rows):
+    W, H, G, d, ff, eps = (cfg["hidden_size"], cfg["num_attention_heads"], cfg["num_key_value_heads"], cfg["head_dim"],
+                           cfg["intermediate_size"], cfg["rms_norm_eps"])
+    table = w("model.embed_tokens.weight", cfg["vocab_size"], W)
+    x = table[ids]
+    freq = _freq(d, cfg["rope_theta"])
+    for i in range(cfg["num_hidden_layers"]):
+        p = f"model.layers.{i}."
+        h = _unit_rms(x, eps) * w.norm(p + "input_layernorm.weight", W)
+        q, k, v = ((h @ w(p + f"self_attn.{n}_proj.weight", m * d, W).T).view(-1, m, d)
+                   for n, m in (("q", H), ("k", G), ("v", G)))
+        q = _rotate(_unit_rms(q, eps) * w.norm(p + "self_attn.q_norm.weight", d), pos, freq)
+        k = _rotate(_unit_rms(k, eps) * w.norm(p + "self_attn.k_norm.weight", d), pos, freq)
+        o = _per_request(spans, lambda *t: _attend(*t, d ** -0.5), q, k, v)
+        x = x + o.reshape(-1, H * d) @ w(p + "self_attn.o_proj.weight", W, H * d).T
+        if i == cfg["num_hidden_layers"] - 1:
+            x = x[rows]
+        h = _unit_rms(x, eps) * w.norm(p + "post_attention_layernorm.weight", W)
+        x = x + (_silu(h @ w(p + "mlp.gate_proj.weight", ff, W).T) * (h @ w(p + "mlp.up_proj.weight", ff, W).T)) \
+            @ w(p + "mlp.down_proj.weight", W, ff).T
+        w.kept = {"model.embed_tokens.weight": table}
+    x = _unit_rms(x, eps) * w.norm("model.norm.weight", W)
+    return x @ (table if cfg["tie_word_embeddings"] else w("lm_head.weight", cfg["vocab_size"], W)).T
+
+
+def _muvonex_exact(cfg, w, ids, pos, spans, rows):
+    W, eps = cfg["width"], cfg["norm"]["eps"]
+    x = w("embed", cfg["vocab"], W)[ids]
+    for i, layer in enumerate(cfg["layers"]):
+        h = _unit_rms(x, eps) * (1.0 + w.small(f"l{i}.norm1", W))
+        m, p = layer["mixer"], f"l{i}.mix."
+        if layer["type"] == "delta":
+            H, G, d, dv, K = m["heads"], m["kv_heads"], m["dim"], m["vdim"], m["conv"]
+            q, k, v = (_silu(_taps(h @ w(p + n, r * c, W).T, spans, w(p + n + ".conv", r * c, K))).view(-1, r, c)
+                       for n, r, c in (("q", G, d), ("k", G, d), ("v", H, dv)))
+            q = q / torch.sqrt((q * q).sum(-1, keepdim=True) + 1e-6) * d ** -0.5
+            k = k / torch.sqrt((k * k).sum(-1, keepdim=True) + 1e-6)
+            beta = torch.sigmoid(h @ w(p + "b", H, W).T)
+            decay = torch.exp(-torch.exp(w.small(p + "A_log", H, exact=True)) * torch.nn.functional.softplus(
+                h @ w(p + "a", H, W).T + w.small(p + "dt_bias", H, exact=True), threshold=100.0))
+            q, k = (_padded(t.repeat_interleave(H // G, 1), spans) for t in (q, k))
+            v, beta, decay = (_padded(t, spans) for t in (v, beta, decay))
+            S = x.new_zeros(len(spans), H, d, dv)
+            o = torch.empty_like(v)
+            for t in range(len(v)):
+                S = S * decay[t][..., None, None]
+                u = beta[t][..., None] * (v[t] - torch.einsum("bhd,bhdv->bhv", k[t], S))
+                S = S + k[t][..., None] * u[..., None, :]
+                o[t] = torch.einsum("bhd,bhdv->bhv", q[t], S)
+            o = _unit_rms(_packed(o, spans), eps) * w.norm(p + "norm", dv)
+            y = (o.reshape(-1, H * dv) * _silu(h @ w(p + "g", H * dv, W).T)) @ w(p + "o", W, H * dv).T
+        else:
+            a, s, q_, r_ = m["left"], m["right"], p + "left.", p + "right."
+            H, G, d = a["heads"], a["kv_heads"], a["dim"]
+            freq = _freq(a["rot"]["dims"], a["rot"]["base"], a["rot"]["scaling"])
+            q, k, v = ((h @ w(q_ + n, r * d, W).T).view(-1, r, d) for n, r in (("q", H), ("k", G), ("v", G)))
+            q, k = _unit_rms(_rotate(q, pos, freq), eps), _unit_rms(_rotate(k, pos, freq), eps)
+            sink = w(q_ + "sink", H, exact=True)
+            o = _per_request(spans, lambda *t: _attend(*t, a["scale"], sink=sink), q, k, v)
+            y = m["left_scale"] * (o.reshape(-1, H * d) @ w(q_ + "o", W, H * d).T)
+            H, P, N, G = s["heads"], s["vdim"], s["state"], s["groups"]
+            n = H * P
+            z, c, dt = (h @ w(r_ + "in", 2 * n + 2 * G * N + H, W).T).split([n, n + 2 * G * N, H], -1)
+            c = _silu(_taps(c, spans, w(r_ + "conv", n + 2 * G * N, s["conv"]), w.small(r_ + "conv.b", n + 2 * G * N)))
+            u, B, C = c.split([n, G * N, G * N], -1)
+            dt = torch.nn.functional.softplus(dt + w.small(r_ + "dt_bias", H, exact=True), threshold=100.0)
+            rate = torch.exp(w.small(r_ + "A_log", H, exact=True))
+            u = u.reshape(-1, H, P)
+            B, C = (t.reshape(-1, G, N).repeat_interleave(H // G, 1) for t in (B, C))
+            up, Bp, Cp, dp = (_padded(t, spans) for t in (u, B, C, dt))
+            S, o = x.new_zeros(len(spans), H, N, P), torch.empty_like(up)
+            for t in range(len(up)):
+                S = S * torch.exp(-rate * dp[t])[..., None, None] + (dp[t][..., None] * Bp[t])[..., None] * up[t][..., None, :]
+                o[t] = torch.einsum("bhn,bhnp->bhp", Cp[t], S)
+            o = _packed(o, spans) + w(r_ + "D", H, std=0.01, mean=1.0, exact=True)[:, None] * u
+            o = (o.reshape(-1, n) * _silu(z)).view(-1, s["norm_groups"], n // s["norm_groups"])
+            o = _unit_rms(o, eps).reshape(-1, n) * w.norm(r_ + "norm", n)
+            y = y + m["right_scale"] * (o @ w(r_ + "o", W, n).T)
+        ff, p = layer["mlp"]["ff"], f"l{i}.mlp."
+        g = torch.nn.functional.gelu(h @ w(p + "gate", ff, W).T, approximate="tanh")
+        x = x + cfg["residual_mult"] * (y + (g * (h @ w(p + "up", ff, W).T)) @ w(p + "down", W, ff).T)
+    return (_unit_rms(x[rows], eps) * (1.0 + w.small("final.norm", W))) @ w("embed", cfg["vocab"], W).T
+
+
+def _nomudra_exact(cfg, w, ids, pos, spans, rows):
+    W, eps = cfg["width"], cfg["norm"]["eps"]
+
+    def norm(x, name):
+        return torch.tanh(w(name + ".alpha", std=0.05, mean=0.5) * x) * w.norm(name, W) + w.small(name + ".b", W)
+
+    def unit(h, p, ff, limit):
+        g = (h @ w(p + "gate", ff, W).T).clamp(max=limit)
+        return (g * torch.sigmoid(1.702 * g) * ((h @ w(p + "up", ff, W).T).clamp(-limit, limit) + 1.0)) \
+            @ w(p + "down", W, ff).T
+
+    x = norm(w("embed", cfg["vocab"], W)[ids], "embed.norm")
+    for i, layer in enumerate(cfg["layers"]):
+        h, m, p = norm(x, f"l{i}.norm1"), layer["mixer"], f"l{i}.mix."
+        if layer["type"] == "attention":
+            H, G, d = m["heads"], m["kv_heads"], m["dim"]
+            freq = _freq(m["rot"]["dims"], m["rot"]["base"])
+            q = (h @ w(p + "q", H * d, W).T + w.small(p + "q.b", H * d)).view(-1, H, d)
+            k = (h @ w(p + "k", G * d, W).T + w.small(p + "k.b", G * d)).view(-1, G, d)
+            o = _per_request(spans, lambda *t: _attend(*t, m["scale"], chunk=m["mask"]["size"]),
+                             _rotate(q, pos, freq), _rotate(k, pos, freq), k)
+            o = o.reshape(-1, H * d) * torch.sigmoid(h @ w(p + "g", H * d, W).T)
+            y = o @ w(p + "o", W, H * d).T + w.small(p + "o.b", W)
+        else:
+            H, d, dv, cap = m["heads"], m["dim"], m["vdim"], m["gate_cap"]
+            q, k, v = ((h @ w(p + n, H * c, W).T).view(-1, H, c) for n, c in (("q", d), ("k", d), ("v", dv)))
+            gi, gf = (cap * torch.tanh((h @ w(p + n, H, W).T + w(p + n + ".b", H, std=1.0, exact=True)) / cap)
+                      for n in ("i", "f"))
+            gf = torch.nn.functional.logsigmoid(gf)
+            q, k, v, gi, gf = (_padded(t, spans) for t in (q * d ** -0.5, k, v, gi, gf))
+            S, n = x.new_zeros(len(spans), H, d, dv), x.new_zeros(len(spans), H, d)
+            top, o = x.new_zeros(len(spans), H), torch.empty_like(v)
+            for t in range(len(v)):
+                new = torch.maximum(gf[t] + top, gi[t])
+                keep, take = torch.exp(gf[t] + top - new)[..., None], torch.exp(gi[t] - new)[..., None]
+                S = keep[..., None] * S + (take * k[t])[..., None] * v[t][..., None, :]
+                n, top = keep * n + take * k[t], new
+                den = torch.maximum((n * q[t]).sum(-1).abs(), torch.exp(-top)) + 1e-6
+                o[t] = torch.einsum("bhd,bhdv->bhv", q[t], S) / den[..., None]
+            o = _unit_rms(_packed(o, spans), eps).reshape(-1, H * dv) * w.norm(p + "norm", H * dv)
+            y = (o * torch.sigmoid(h @ w(p + "g", H * dv, W).T)) @ w(p + "o", W, H * dv).T
+        x = x + norm(y, f"l{i}.norm1b")
+        h, mlp, p = norm(x, f"l{i}.norm2"), layer["mlp"], f"l{i}.mlp."
+        r = mlp["router"]
+        N, groups = r["experts"] + r["identity"], r["groups"]
+        score = torch.softmax(h @ w(p + "router", N, W).T, -1)
+        choice = score + w.small(p + "correction", N, exact=True)
+        best = choice.view(-1, groups["count"], N // groups["count"]).amax(-1).topk(groups["keep"], -1).indices
+        allowed = torch.zeros(len(h), groups["count"], dtype=torch.bool, device=h.device).scatter_(1, best, True)
+        allowed = allowed.repeat_interleave(N // groups["count"], 1)
+        chosen = choice.masked_fill(~allowed, -math.inf).topk(r["top"], -1).indices
+        weight = score.gather(1, chosen)
+        weight = weight / (weight.sum(-1, keepdim=True) + 1e-20)
+        y = unit(h, p + "shared.", mlp["shared"]["ff"], mlp["shared"]["limit"]) \
+            * torch.sigmoid(h @ w(p + "shared.sg", 1, W).T)
+        for e in range(N):
+            at, slot = (chosen == e).nonzero(as_tuple=True)
+            if len(at):
+                got = h[at] if e >= r["experts"] else unit(h[at], p + f"e{e}.", mlp["expert"]["ff"], mlp["expert"]["limit"])
+                y[at] += weight[at, slot][:, None] * got
+        x = x + norm(y, f"l{i}.norm2b")
+    return norm(x[rows], "final.norm") @ w("head", cfg["vocab"], W).T
+
+
+def _ginodra_exact(cfg, w, ids, pos, spans, rows):
+    W, eps, groups = cfg["width"], cfg["norm"]["eps"], cfg["norm"]["groups"]
+
+    def norm(x, name):
+        return _unit_rms(x.view(-1, groups, W // groups), eps).reshape(-1, W) * w.norm(name, W)
+
+    def filtered(h, name):
+        return h + _taps(h, spans, w(name, W, cfg["canon"]["taps"], std=0.3))
+
+    x, kept = w("embed", cfg["vocab"], W)[ids], {}
+    for i, layer in enumerate(cfg["layers"]):
+        plain = norm(x, f"l{i}.norm1")
+        h, m, p = filtered(plain, f"l{i}.canon1"), layer["mixer"], f"l{i}.mix."
+        if layer["type"] == "latent_attention":
+            H, d, r, dv, rank = m["heads"], m["dim"], m["rot_dim"], m["vdim"], m["kv_rank"]
+            freq = _freq(m["rot"]["dims"], m["rot"]["base"])
+            q = _unit_rms(h @ w(p + "dq", m["q_rank"], W).T, eps) * w.norm(p + "dq.norm", m["q_rank"])
+            q = (q @ w(p + "uq", H * (d + r), m["q_rank"]).T).view(-1, H, d + r)
+            q = torch.cat([q[..., :d], _rotate(q[..., d:], pos, freq)], -1)
+            c, kr = (h @ w(p + "dkv", rank + r, W).T).split([rank, r], -1)
+            c = _unit_rms(c, eps) * w.norm(p + "dkv.norm", rank)
+            k = torch.cat([(c @ w(p + "uk", H * d, rank).T).view(-1, H, d),
+                           _rotate(kr[:, None], pos, freq).expand(-1, H, -1)], -1)
+            v = (c @ w(p + "uv", H * dv, rank).T).view(-1, H, dv)
+            sink = w(p + "sink", H, std=1.0, exact=True)
+            o = _per_request(spans, lambda *t: _attend(*t, m["scale"], sink=sink), q, k, v)
+            y = (o * torch.sigmoid(h @ w(p + "g", H, W).T)[..., None]).reshape(-1, H * dv) @ w(p + "o", W, H * dv).T
+        elif layer["type"] == "attention":
+            H, G, d = m["heads"], m["kv_heads"], m["dim"]
+            q = _unit_rms((h @ w(p + "q", H * d, W).T).view(-1, H, d), eps) * w.norm(p + "q.norm", d)
+            if m.get("kv_from") is None:
+                kept[i] = (_unit_rms((h @ w(p + "k", G * d, W).T).view(-1, G, d), eps) * w.norm(p + "k.norm", d),
+                           (h @ w(p + "v", G * d, W).T).view(-1, G, d))
+            k, v = kept[i if m.get("kv_from") is None else m["kv_from"]]
+            slope = torch.tensor([2.0 ** (-8.0 * (a + 1) / H) for a in range(H)], dtype=torch.float64, device=x.device)
+            o = _per_request(spans, lambda *t: _attend(*t, m["scale"], reach=m["mask"]["size"], slope=slope), q, k, v)
+            y = (o * torch.sigmoid(h @ w(p + "g", H, W).T)[..., None]).reshape(-1, H * d) @ w(p + "o", W, H * d).T
+        else:
+            H, d = m["heads"], m["dim"]
+            n, rank = H * d, m["decay_rank"]
+            r, k, v = ((h @ w(p + c, n, W).T).view(-1, H, d) for c in "rkv")
+            decay = torch.tanh(h @ w(p + "w1", rank, W).T) @ w(p + "w2", n, rank, std=1.0).T + w(p + "w0", n, std=1.0)
+            decay = torch.exp(-math.exp(-0.5) * torch.sigmoid(decay)).view(-1, H, d)
+            rate = torch.sigmoid(h @ w(p + "a", n, W).T + w(p + "a.b", n, std=1.0)).view(-1, H, d)
+            u = k / torch.sqrt((k * k).sum(-1, keepdim=True) + 1e-6)
+            r, k, v, decay, rate, u = (_padded(t, spans) for t in (r, k, v, decay, rate, u))
+            S, o = x.new_zeros(len(spans), H, d, d), torch.empty_like(v)
+            for t in range(len(v)):
+                seen = torch.einsum("bhk,bhkv->bhv", u[t], S)
+                S = decay[t][..., None] * S - (rate[t] * u[t])[..., None] * seen[..., None, :] \
+                    + k[t][..., None] * v[t][..., None, :]
+                o[t] = torch.einsum("bhk,bhkv->bhv", r[t], S)
+            o = _unit_rms(_packed(o, spans), eps).reshape(-1, n) * w.norm(p + "norm", n)
+            y = (o * torch.sigmoid(h @ w(p + "g", n, W).T)) @ w(p + "o", W, n).T
+        ff = layer["mlp"]["ff"]
+        y = y + (torch.relu(filtered(plain, f"l{i}.canon2") @ w(f"l{i}.mlp.up", ff, W).T) ** 2) @ w(f"l{i}.mlp.down", W, ff).T
+        x = x + cfg["residual_mult"] * y
+    z = norm(x[rows], "final.norm") @ w("embed", cfg["vocab"], W).T * cfg["logit_scale"]
+    return cfg["logit_softcap"] * torch.tanh(z / cfg["logit_softcap"])
+
+
+def exact(case, seed):
+    cfg, kind, new = MODELS[case["model"]], case["kind"], case["new"]
+    spans = _lengths(case)
+    if case["model"] == "qwen3_8b" and sum(spans) > 60000:
+        return None                         # the contexts alone would be over 20 seconds of 64-bit products
+    rows, cut = _tokens(case, seed)
+    rows = ([cut] if kind == "mixed" else []) + rows
+    model = {"qwen3": _qwen3_exact, "muvonex": _muvonex_exact, "nomudra": _nomudra_exact,
+             "ginodra": _ginodra_exact}[case["model"].split("_")[0]]
+    w = _Weights(seed, torch.bfloat16 if case["dtype"] == "bfloat16" else torch.float32)
+    found, group, size = [], [], 0
+
+    def compute():
+        ends = [sum(len(r) for r in group[:i + 1]) for i in range(len(group))]
+        spans = [(e - len(r), e) for r, e in zip(group, ends)]
+        ids = torch.tensor([t for r in group for t in r], device="cuda")
+        pos = torch.cat([torch.arange(len(r), device="cuda") for r in group])
+        wanted = torch.tensor([e - 1 - new + k for e in ends for k in range(new + 1)], device="cuda")
+        found.append(model(cfg, w, ids, pos, spans, wanted).view(len(group), new + 1, -1))
+
+    with torch.no_grad():
+        for r in rows:
+            if group and size + len(r) > 20000:
+                compute()
+                group, size = [], 0
+            group.append(r)
+            size += len(r)
+        compute()
+    out = torch.cat(found)
+    return [out[:, k] for k in range(new + 1)] if kind in ("prompt", "generate") else out[:, 0]
