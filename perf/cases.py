@@ -184,11 +184,12 @@ def prepare(case, seed):
     rows, cut = _tokens(case, seed)
     held = [len(r) for r in rows] + ([len(cut)] if cut else [])
     pages = sum(-(-(n + 1) // PAGE) for n in held) + 2
+    places = max(8, 1 << (len(held) - 1).bit_length())       # a server is set up for a round number of live requests
     with tempfile.TemporaryDirectory() as folder:
         with open(os.path.join(folder, "config.json"), "w") as f:
             json.dump(MODELS[case["model"]], f)
         llm = LLM(folder, random_weights_seed=seed, kvcache_block_size=PAGE, num_kvcache_blocks=pages,
-                  max_model_len=max(4352, max(held) + 1), max_num_seqs=max(8, len(held)), max_num_batched_tokens=BUDGET,
+                  max_model_len=max(4352, max(held) + 1), max_num_seqs=places, max_num_batched_tokens=BUDGET,
                   dtype=case["dtype"])
     runner, kind = llm.model_runner, case["kind"]
     state = dict(llm=llm, runner=runner, kind=kind, rows=rows, flight=None, new=case["new"])
