@@ -30,6 +30,8 @@
 // true positions; their chunks are visited before the window's.
 #include <math.h>
 
+#include <type_traits>
+
 #include "nhv_common.cuh"
 
 constexpr int AT_WARPS = 4;
@@ -197,6 +199,257 @@ __global__ void attn_paged_simt_kernel(const T* __restrict__ q, int q_stride, T*
   }
 }
 
+// ---------------------------------------------------------------- head sizes in steps of 4
+// The kernel above reads one float of K and one of q from shared memory per multiply-add and waits for every chunk of
+// keys: 320 us for 370 tokens (37 to 210 a request) of 16 heads of 128; this one takes 80.  For heads of up to 256
+// elements in steps of four, in rows that can be read 16 (bf16: 8) bytes at a time:
+//   - a warp takes its pairs (up to 8) through a chunk together, so that a key's four elements, read once, serve all of
+//     them, and likewise a value's; q and the probabilities are broadcast reads of four;
+//   - key rows are d + 4 floats apart: the eight lanes that are served at once read different banks;
+//   - products and sums two at a time (a score is the sum of its even and its odd elements, each in ascending order);
+//   - with fp32 storage the next chunk of keys and values travels by cp.async while this one is worked on.
+// The order of a position's operations is as fixed as above: chunks of 32 keys at absolute multiples of 32; a pair for
+// which a chunk holds no visible key is left as it is.
+static __device__ __forceinline__ void simt_copy16(float* smem, const float* gmem, bool there) {
+  const int bytes = there ? 16 : 0;                        // what is not there arrives as zeros
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"((uint32_t)__cvta_generic_to_shared(smem)), "l"(gmem),
+               "r"(bytes));
+}
+static __device__ __forceinline__ float4 simt_load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
+static __device__ __forceinline__ float4 simt_load4(const __nv_bfloat16* p) {
+  const uint2 raw = *reinterpret_cast<const uint2*>(p);
+  const float2 lo = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.x));
+  const float2 hi = __bfloat1622float2(*reinterpret_cast<const __nv_bfloat162*>(&raw.y));
+  return make_float4(lo.x, lo.y, hi.x, hi.y);
+}
+
+constexpr int AV_PAIRS = 8;             // pairs per warp
+
+// VC: groups of four output columns per lane (value heads of up to 128 VC elements)
+template <typename T, int VC>
+__global__ void __launch_bounds__(AT_WARPS * 32) attn_paged_simt_vec_kernel(
+    const T* __restrict__ q, int q_stride, T* __restrict__ out, int out_stride, const T* __restrict__ kv_pages,
+    const int* __restrict__ block_table, int bt_stride, const int* __restrict__ cu_q, const int* __restrict__ kv_len,
+    int n_seqs, int nq, int nkv, int d, int page_size, int n_pages, int window, float scale, int TQ, int GS, int dv, int row,
+    const float* __restrict__ sinks, int chunk, const float* __restrict__ slopes, int planes, int keep_first,
+    float softcap) {
+  extern __shared__ __align__(16) float smem[];
+  constexpr bool ASYNC = sizeof(T) == 4;
+  constexpr int STAGES = ASYNC ? 2 : 1;
+  pdl_prologue();
+  const int G = nq / nkv;
+  const int kvh = blockIdx.y;
+  const int g0 = blockIdx.z * GS;
+  const int gs = min(GS, G - g0);
+  int seq = -1, tile = blockIdx.x;
+  for (int s = 0; s < n_seqs; ++s) {
+    const int n = cu_q[s + 1] - cu_q[s];
+    const int nt = (n + TQ - 1) / TQ;
+    if (tile < nt) { seq = s; break; }
+    tile -= nt;
+  }
+  if (seq < 0) return;
+  const int n_new = cu_q[seq + 1] - cu_q[seq];
+  const int total = kv_len[seq];
+  const int t0 = tile * TQ;                              // first token of the tile, within the new tokens
+  const int tq_n = min(TQ, n_new - t0);
+  const int n_pairs = tq_n * gs;
+  const int pos_lo = total - n_new + t0, pos_hi = pos_lo + tq_n - 1;
+
+  const int ks = d + 4;
+  const int vs = planes == 2 ? dv : ks;                  // one plane: the values are the keys' leading elements
+  const int stage_floats = AT_CHUNK * ks + (planes == 2 ? AT_CHUNK * dv : 0);
+  float* Qs = smem + STAGES * stage_floats;              // [pairs][d]
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  float* Ps = Qs + AV_PAIRS * AT_WARPS * d + warp * AV_PAIRS * AT_CHUNK;   // [pairs of the warp][32]
+  const int d4 = d >> 2, dv4 = dv >> 2;
+
+  for (int i = tid; i < n_pairs * d4; i += AT_WARPS * 32) {
+    const int p = i / d4, c = 4 * (i - p * d4);
+    const int tq = p / gs, g = p - tq * gs;
+    const size_t tok = (size_t)cu_q[seq] + t0 + tq;
+    *reinterpret_cast<float4*>(Qs + p * d + c) = simt_load4(q + tok * q_stride + (size_t)(kvh * G + g0 + g) * d + c);
+  }
+
+  // the page row of key j (-1: there is no such key)
+  auto key_row = [&](int j) -> long {
+    if (j > pos_hi || j >= total) return -1;
+    const int page = block_table[(size_t)seq * bt_stride + j / page_size];
+    if (page < 0 || page >= n_pages) return -1;
+    return (((long)page * planes) * nkv + kvh) * page_size + j % page_size;
+  };
+  const long v_plane = (long)nkv * page_size;
+  auto fetch = [&](int c0, int stage) {
+    float* Ks = smem + stage * stage_floats;
+    float* Vs = Ks + AT_CHUNK * ks;
+    // a warp per row: its lanes take a group of four each
+    for (int r = warp; r < AT_CHUNK; r += AT_WARPS) {
+      const long at = key_row(c0 + r);
+      const bool there = at >= 0;
+      const T* src = kv_pages + (there ? at * row : 0);
+      for (int c = lane; c < d4; c += 32) {
+        if constexpr (ASYNC) simt_copy16(Ks + r * ks + 4 * c, src + 4 * c, there);
+        else *reinterpret_cast<float4*>(Ks + r * ks + 4 * c) = there ? simt_load4(src + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
+      }
+      if (planes == 2) {
+        src += there ? v_plane * row : 0;
+        for (int c = lane; c < dv4; c += 32) {
+          if constexpr (ASYNC) simt_copy16(Vs + r * dv + 4 * c, src + 4 * c, there);
+          else *reinterpret_cast<float4*>(Vs + r * dv + 4 * c) = there ? simt_load4(src + 4 * c) : make_float4(0.f, 0.f, 0.f, 0.f);
+        }
+      }
+    }
+  };
+
+  const int first_key = nhv_first_key(pos_lo, window, chunk);
+  const int c_begin = (first_key / AT_CHUNK) * AT_CHUNK;
+  const int kept_end = keep_first > 0 ? min(((keep_first + AT_CHUNK - 1) / AT_CHUNK) * AT_CHUNK, c_begin) : 0;
+  auto next_chunk = [&](int c0) {
+    c0 += AT_CHUNK;
+    return c0 >= kept_end && c0 < c_begin ? c_begin : c0;
+  };
+
+  // pair i of the warp is pair warp + i * AT_WARPS of the block; NP of them may exist
+  auto work = [&](auto np) {
+    constexpr int NP = decltype(np)::value;
+    float m[NP], l[NP];
+    f32x2 o[NP][2 * VC];
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+      const int p = warp + i * AT_WARPS;
+      const bool sink = sinks && p < n_pairs;
+      m[i] = sink ? sinks[kvh * G + g0 + (p % gs)] : -INFINITY;
+      l[i] = sink ? 1.f : 0.f;
+#pragma unroll
+      for (int c = 0; c < 2 * VC; ++c) o[i][c] = 0ull;
+    }
+    int c0 = kept_end > 0 ? 0 : c_begin, stage = 0;
+    if (ASYNC) {
+      fetch(c0, 0);
+      asm volatile("cp.async.commit_group;\n" ::);
+    }
+    for (; c0 <= pos_hi; c0 = next_chunk(c0)) {
+      if (ASYNC) {
+        asm volatile("cp.async.wait_group 0;\n" ::);
+        __syncthreads();                                   // this chunk is there, and the other stage has been read by all
+        if (next_chunk(c0) <= pos_hi) fetch(next_chunk(c0), stage ^ 1);
+        asm volatile("cp.async.commit_group;\n" ::);
+      } else {
+        __syncthreads();
+        fetch(c0, 0);
+        __syncthreads();
+      }
+      const float* Ks = smem + stage * stage_floats;
+      const float* Vs = planes == 2 ? Ks + AT_CHUNK * ks : Ks;
+      if (ASYNC) stage ^= 1;
+      const int j = c0 + lane;
+      const bool ok = key_row(j) >= 0;
+
+      f32x2 acc[NP];
+#pragma unroll
+      for (int i = 0; i < NP; ++i) acc[i] = 0ull;
+      const float* kv = Ks + lane * ks;
+#pragma unroll 2
+      for (int c = 0; c < d; c += 4) {
+        const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(kv + c);
+#pragma unroll
+        for (int i = 0; i < NP; ++i) {
+          const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(Qs + (warp + i * AT_WARPS) * d + c);
+          acc[i] = f2_fma(q4.x, k4.x, acc[i]);
+          acc[i] = f2_fma(q4.y, k4.y, acc[i]);
+        }
+      }
+      float s[NP], top[NP], alpha[NP];
+#pragma unroll
+      for (int i = 0; i < NP; ++i) {
+        const int p = warp + i * AT_WARPS, tq = p / gs, pos = pos_lo + tq;
+        const int lo = nhv_first_key(pos, window, chunk);
+        float even, odd;
+        f2_unpack(acc[i], even, odd);
+        s[i] = -INFINITY;
+        if (p < n_pairs && ok && j <= pos && (j >= lo || j < keep_first)) {
+          s[i] = (even + odd) * scale;
+          if (softcap > 0.f) s[i] = softcap * tanhf(s[i] / softcap);
+          if (slopes) s[i] -= slopes[kvh * G + g0 + (p - tq * gs)] * (float)(pos - j);
+        }
+        top[i] = s[i];
+      }
+#pragma unroll
+      for (int i = 0; i < NP; ++i) top[i] = warp_max(top[i]);
+#pragma unroll
+      for (int i = 0; i < NP; ++i) {
+        const bool any = top[i] != -INFINITY;              // no visible key: the pair stays as it is
+        const float m_new = any ? fmaxf(m[i], top[i]) : m[i];
+        alpha[i] = any ? expf(m[i] - m_new) : 1.f;         // exp(-inf) = 0 on the first chunk
+        s[i] = any ? expf(s[i] - m_new) : 0.f;             // 0 for masked keys
+        m[i] = m_new;
+        Ps[i * AT_CHUNK + lane] = s[i];
+      }
+#pragma unroll
+      for (int i = 0; i < NP; ++i) l[i] = l[i] * alpha[i] + warp_sum(s[i]);
+      __syncwarp();
+#pragma unroll
+      for (int vc = 0; vc < VC; ++vc) {
+        const int c = 4 * (lane + 32 * vc);
+        if (c >= dv) continue;
+        f32x2 sum[NP][2];
+#pragma unroll
+        for (int i = 0; i < NP; ++i) sum[i][0] = sum[i][1] = 0ull;
+#pragma unroll 1
+        for (int r = 0; r < AT_CHUNK; r += 4) {
+          ulonglong2 v[4];
+#pragma unroll
+          for (int e = 0; e < 4; ++e) v[e] = *reinterpret_cast<const ulonglong2*>(Vs + (r + e) * vs + c);
+#pragma unroll
+          for (int i = 0; i < NP; ++i) {
+            const float4 pr = *reinterpret_cast<const float4*>(Ps + i * AT_CHUNK + r);
+            const float pe[4] = {pr.x, pr.y, pr.z, pr.w};
+#pragma unroll
+            for (int e = 0; e < 4; ++e) {
+              const f32x2 pp = f2_pack(pe[e], pe[e]);
+              sum[i][0] = f2_fma(pp, v[e].x, sum[i][0]);
+              sum[i][1] = f2_fma(pp, v[e].y, sum[i][1]);
+            }
+          }
+        }
+        const f32x2 one = f2_pack(1.f, 1.f);
+#pragma unroll
+        for (int i = 0; i < NP; ++i) {
+          if (top[i] == -INFINITY) continue;               // (its zeros may have met values that are no numbers)
+          const f32x2 aa = f2_pack(alpha[i], alpha[i]);
+          o[i][2 * vc] = f2_fma(f2_mul(o[i][2 * vc], aa), one, sum[i][0]);
+          o[i][2 * vc + 1] = f2_fma(f2_mul(o[i][2 * vc + 1], aa), one, sum[i][1]);
+        }
+      }
+      __syncwarp();
+    }
+#pragma unroll
+    for (int i = 0; i < NP; ++i) {
+      const int p = warp + i * AT_WARPS;
+      if (p >= n_pairs) break;
+      const int tq = p / gs, g = p - tq * gs;
+      const size_t tok = (size_t)cu_q[seq] + t0 + tq;
+      T* dst = out + tok * out_stride + (size_t)(kvh * G + g0 + g) * dv;
+      const float inv = l[i] > 0.f ? 1.0f / l[i] : 0.f;
+#pragma unroll
+      for (int vc = 0; vc < VC; ++vc) {
+        const int c = 4 * (lane + 32 * vc);
+        if (c >= dv) continue;
+        float x[4];
+        f2_unpack(o[i][2 * vc], x[0], x[1]);
+        f2_unpack(o[i][2 * vc + 1], x[2], x[3]);
+#pragma unroll
+        for (int e = 0; e < 4; ++e) dst[c + e] = from_f32<T>(x[e] * inv);
+      }
+    }
+  };
+  // the same for all warps of the block (the loop over the chunks has barriers)
+  const int most = (n_pairs + AT_WARPS - 1) / AT_WARPS;
+  if (most <= 1) work(std::integral_constant<int, 1>());
+  else if (most <= 4) work(std::integral_constant<int, 4>());
+  else work(std::integral_constant<int, AV_PAIRS>());
+}
+
 // max_tiles: an upper bound on sum over requests of ceil(new tokens / TQ); the caller may pass
 // n_tokens / TQ + n_seqs.  Blocks beyond the true count leave at once.
 NHV_API int nhv_attention_simt_ex(int dtype, const void* q, int q_stride, void* out, int out_stride,
@@ -214,6 +467,30 @@ NHV_API int nhv_attention_simt_ex(int dtype, const void* q, int q_stride, void* 
   NHV_REQUIRE(page_size > 0 && n_pages > 0 && bt_stride > 0, "attention: bad page geometry");
   NHV_REQUIRE(planes == 2 || (planes == 1 && dv <= d), "attention: pages have a key and a value plane, or one plane whose rows' leading elements are the values");
   const int G = nq / nkv;
+  // groups of four elements wherever sizes and addresses allow them
+  const uintptr_t four = dtype == NHV_F32 ? 16 : 8;
+  if (d % 4 == 0 && dv % 4 == 0 && d <= 256 && dv <= 256 && row % 4 == 0 && q_stride % 4 == 0 && (uintptr_t)q % four == 0 &&
+      (uintptr_t)kv_pages % four == 0) {
+    const int most = AV_PAIRS * AT_WARPS, GS = G < 8 ? G : 8, TQ = most / GS, stages = dtype == NHV_F32 ? 2 : 1;
+    const size_t smem = ((size_t)stages * AT_CHUNK * (d + 4 + (planes == 2 ? dv : 0)) + (size_t)most * (d + AT_CHUNK)) * 4;
+    const dim3 grid(n_tokens / TQ + n_seqs, nkv, (G + GS - 1) / GS);
+#define LAUNCH_VEC(T, VC)                                                                                           \
+  do {                                                                                                              \
+    NHV_CUDA(cudaFuncSetAttribute(attn_paged_simt_vec_kernel<T, VC>, cudaFuncAttributeMaxDynamicSharedMemorySize,   \
+                                  (int)smem), "attention");                                                         \
+    nhv_launch(attn_paged_simt_vec_kernel<T, VC>, grid, AT_WARPS * 32, smem, stream, (const T*)q, q_stride, (T*)out, \
+               out_stride, (const T*)kv_pages, block_table, bt_stride, cu_q, kv_len, n_seqs, nq, nkv, d, page_size,  \
+               n_pages, window, scale, TQ, GS, dv, row, sinks, chunk, slopes, planes, keep_first, softcap);          \
+  } while (0)
+    if (dtype == NHV_F32 && dv <= 128) LAUNCH_VEC(float, 1);
+    else if (dtype == NHV_F32) LAUNCH_VEC(float, 2);
+    else if (dtype == NHV_BF16 && dv <= 128) LAUNCH_VEC(__nv_bfloat16, 1);
+    else if (dtype == NHV_BF16) LAUNCH_VEC(__nv_bfloat16, 2);
+    else NHV_REQUIRE(false, "attention: unknown dtype %d", dtype);
+#undef LAUNCH_VEC
+    NHV_CHECK_LAUNCH("attention");
+    return 0;
+  }
   const int cols = dv <= 256 ? 8 : dv <= 512 ? 16 : dv <= 1024 ? 32 : 64;
   const int max_pairs = AT_ACC / cols * AT_WARPS;
   const int GS = G < 8 ? (G < max_pairs ? G : max_pairs) : (8 < max_pairs ? 8 : max_pairs);
