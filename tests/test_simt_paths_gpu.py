@@ -1,5 +1,5 @@
-"""The CUDA-core product and attention at the edges of its tiles, and where sizes or addresses send it another way (operands that cannot
-be copied 16 bytes at a time), against a 64-bit reference and each other."""
+"""The CUDA-core product and attention at the edges of their tiles, and where sizes or addresses send them another way
+(what cannot be read 16 bytes at a time), against a 64-bit reference and each other."""
 import pytest
 import torch
 
