@@ -8,9 +8,9 @@
 //           same (row, column) in the same thread, so the unit is applied without leaving the registers;
 //   second: y[row, c] = act[row] . Wd[e][c]                                          128 columns;
 //   for experts without a gate, first: act[row, c] = relu(x[token(row)] . Wu[e][c])^2   128 columns.
-// A rows are gathered by token on their way into shared memory.  Operands travel by cp.async in a ring of three
-// stages of 32 columns of K (small stages: several blocks fit an SM, and the tensor pipe needs many warps to stay
-// busy); a row's sum over K runs in the same order wherever the row stands, so results do not depend on the
+// A rows are gathered by token on their way into shared memory.  Operands travel by cp.async in a ring of
+// stages, for prompts three of 32 columns of K (small stages: several blocks fit an SM, and the tensor pipe needs many
+// warps to stay busy); a row's sum over K runs in the same order wherever the row stands, so results do not depend on the
 // ordering.  BM is 16 where experts see few rows (decoding: the kernel streams each expert's weights once), 64 or
 // 128 (eight warps, each panel of weights read for twice the rows) for prompts.
 #include <cuda_bf16.h>
@@ -21,9 +21,6 @@
 
 typedef __nv_bfloat16 bf16;
 
-constexpr int MM_BK = 32;
-constexpr int MM_LDS = MM_BK + 8;       // a row of a stage in shared memory, padded against bank conflicts
-constexpr int MM_STAGES = 3;
 constexpr int MM_BROWS = 128;
 
 __device__ __forceinline__ void mm_cp_async16(void* smem, const void* gmem, int bytes) {
@@ -46,7 +43,13 @@ __device__ __forceinline__ void mm_mma(float (&c)[4], const uint32_t (&a)[4], ui
 
 __device__ __forceinline__ float mm_round(float v) { return __bfloat162float(__float2bfloat16_rn(v)); }
 
+// Tiles of 16 rows only stream the weights: what counts is how many bytes are on their way.  Their grid is about two
+// blocks an SM (16 experts, 16 panels), so a block keeps four stages of 64 columns, 64 KB, in flight (two stages of 32
+// columns left the 134 MB of 16 experts' gate and up at 40 us and the 67 MB of down at 22, half the memory's rate).
 template <int BM> struct MmShape {
+  static constexpr int BK = BM >= 64 ? 32 : 64;        // columns of K per stage
+  static constexpr int LDS = BK + 8;                   // a row of a stage in shared memory, padded against bank conflicts
+  static constexpr int STAGES = BM >= 64 ? 3 : 5;
   static constexpr int WM = BM >= 64 ? 64 : 16;        // rows per warp
   static constexpr int THREADS = (BM / WM) * 4 * 32;   // warps: BM / WM along the rows x 4 along the columns
 };
@@ -58,6 +61,7 @@ __global__ void __launch_bounds__(MmShape<BM>::THREADS) moe_gemm_mma_kernel(
     float alpha, float up_shift, const float* __restrict__ row_scale) {
   constexpr bool FIRST = MODE == 1, GATHER = MODE != 0;
   constexpr int MT = MmShape<BM>::WM / 16, MM_THREADS = MmShape<BM>::THREADS;
+  constexpr int MM_BK = MmShape<BM>::BK, MM_LDS = MmShape<BM>::LDS, MM_STAGES = MmShape<BM>::STAGES;
   extern __shared__ __align__(16) unsigned char smem_raw[];
   bf16* As = reinterpret_cast<bf16*>(smem_raw);              // [STAGES][BM][LDS]
   bf16* Bs = As + MM_STAGES * BM * MM_LDS;                   // [STAGES][BROWS][LDS]
@@ -177,7 +181,7 @@ __global__ void __launch_bounds__(MmShape<BM>::THREADS) moe_gemm_mma_kernel(
 }
 
 template <int BM>
-static size_t mm_smem_bytes() { return (size_t)MM_STAGES * (BM + MM_BROWS) * MM_LDS * sizeof(bf16); }
+static size_t mm_smem_bytes() { return (size_t)MmShape<BM>::STAGES * (BM + MM_BROWS) * MmShape<BM>::LDS * sizeof(bf16); }
 
 // tile: 16, 64 or 128, the row tile that moe_align was called with.  mode 1: out [rows, N] = glu over x [T, K] gathered
 // by sorted_slots, W0 / W1 [E, N, K]; 2: relu^2 of the same rows times W0; 0: out [rows, N] = a [rows, K] times W0 [E, N, K].
