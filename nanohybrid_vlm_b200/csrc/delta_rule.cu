@@ -23,6 +23,7 @@
 // without a slot (slot < 0) is skipped and its outputs are cleared.
 #include <math.h>
 
+#include "nhv_chunk_scan.cuh"
 #include "nhv_common.cuh"
 
 constexpr int DR_PARTS = 4;
@@ -737,17 +738,32 @@ __global__ void __launch_bounds__(DR_COLS * DR_PARTS) delta_scan_kernel(
   }
 }
 
+struct DeltaGates {
+  const float *decay, *beta;                             // [T, H]
+  int H;
+  __device__ __forceinline__ void operator()(int t, int h, float& gate, float& weight, float&) const {
+    gate = decay[(size_t)t * H + h];
+    weight = beta[(size_t)t * H + h];
+  }
+};
+
+// Floats of scratch per head and chunk for the kernels that go through prompts a chunk of tokens at a time; a step has
+// n_tokens / 32 + n_seqs chunks.
+NHV_API int nhv_chunk_scan_floats() { return CS_WORK; }
+
 // o_out [T, H, dv] fp32.  lanes: 4, 8, 16 or 32 lanes per column of the state, or 0 for the kernel's own choice.
 // group4: 1 takes four tokens per round of the chain (needs pairs [T, G, 8] as scratch), 0 one, -1 chooses by the
 // size of the step.  cpt: 2 or 4 columns of the state per lane (8 lanes a column, d up to 128), 1 one, 0 the
 // kernel's choice.
+// chunks: scratch of (n_tokens / 32 + n_seqs) * H * nhv_chunk_scan_floats() floats to go through the prompts a chunk of
+// tokens at a time (d up to 128, sizes in steps of 4; null: token by token).
 // Scratch given by the caller, all fp32: qn, kn [T, G, d]; kq [T, G]; v32 [T, H, dv]; beta,
 // decay [T, H].
 NHV_API int nhv_delta_rule(int dtype, float* o_out, const void* qkv, int qkv_stride, const float* ba,
                            const float* a_log, const float* dt_bias, float* state, long state_stride, float* qn,
                            float* kn, float* kq, float* v32, float* beta, float* decay, const int* cu_q,
                            const int* q_start, const int* slots, int n_seqs, int n_tokens, int G, int H, int d, int dv,
-                           int lanes, int group4, float* pairs, int cpt, cudaStream_t stream) {
+                           int lanes, int group4, float* pairs, int cpt, float* chunks, cudaStream_t stream) {
   if (n_tokens == 0 || n_seqs == 0) return 0;
   NHV_REQUIRE(G > 0 && H > 0 && H % G == 0, "delta_rule: %d heads do not divide into %d q/k heads", H, G);
   NHV_REQUIRE(d > 0 && d <= 256 && dv > 0, "delta_rule: a q/k head of %d is beyond the supported 256", d);
@@ -767,6 +783,22 @@ NHV_API int nhv_delta_rule(int dtype, float* o_out, const void* qkv, int qkv_str
   else if (dtype == NHV_BF16) PREP(__nv_bfloat16);
   else NHV_REQUIRE(false, "delta_rule: unknown dtype %d", dtype);
 #undef PREP
+  // prompts: a chunk of tokens at a time
+  if (chunks && fast && d <= 128) {
+    const CsPairs pp{qn, kn, (long)G * d, chunks, nullptr, cu_q, slots, n_seqs, G, H, d};
+    const DeltaGates gates{decay, beta, H};
+    const CsScan ps{o_out, qn, kn, (long)G * d, v_src, v_stride, chunks, nullptr, nullptr, nullptr, state, state_stride,
+                    cu_q, q_start, slots, G, H, d, dv};
+    if (d <= 64) {
+      NHV_CUDA((cs_launch_pairs<64, CS_DELTA>(pp, gates, n_tokens, stream)), "delta_rule");
+      NHV_CUDA((cs_launch_scan<64, CS_DELTA, float>(ps, n_seqs, stream)), "delta_rule");
+    } else {
+      NHV_CUDA((cs_launch_pairs<128, CS_DELTA>(pp, gates, n_tokens, stream)), "delta_rule");
+      NHV_CUDA((cs_launch_scan<128, CS_DELTA, float>(ps, n_seqs, stream)), "delta_rule");
+    }
+    NHV_CHECK_LAUNCH("delta_rule");
+    return 0;
+  }
   // four tokens per round of the chain: 225 against 252 ns a token for one 4,096-token request (16 heads, d = dv =
   // 128), the same at 4 or more requests.  Too little to give up sums in one fixed order for: off unless asked for.
   if (group4 < 0) group4 = 0;

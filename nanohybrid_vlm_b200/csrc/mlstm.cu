@@ -18,6 +18,7 @@
 // A request with q_start == 0 starts fresh; one without a slot (slot < 0) is skipped and its outputs are cleared.
 #include <math.h>
 
+#include "nhv_chunk_scan.cuh"
 #include "nhv_common.cuh"
 #include "nhv_vec8.cuh"
 
@@ -295,6 +296,96 @@ __global__ void __launch_bounds__(128) mlstm_step_kernel(
   }
 }
 
+// ---------------------------------------------------------------- prompts, a chunk of tokens at a time
+// (nhv_chunk_scan.cuh: the columns of S with weights exp(i_t - m_t) and decays exp(f_t + m_(t-1) - m_t); the normaliser
+// n . q of a token is gam_t (n0 . q_t) + the sum of its row of P.)  The chain of maxima comes first: with
+// (F, M)(t) = (f_t, i_t) and (F1, M1) then (F2, M2) = (F1 + F2, max(M1 + F2, M2)), m_t = max(F + m, M) of the tokens so far.
+
+constexpr int MG_TOKENS = 256;
+
+// One block per (request, head): a = decay, b = weight, em = exp(-m), top = m, all [T, H].
+__global__ void __launch_bounds__(MG_TOKENS) mlstm_gates_kernel(
+    float* __restrict__ a, float* __restrict__ b, float* __restrict__ em, float* __restrict__ top,
+    const float* __restrict__ gates, int gate_stride, const float* __restrict__ gate_bias, float cap,
+    const float* __restrict__ state, long state_stride, const int* __restrict__ cu_q, const int* __restrict__ q_start,
+    const int* __restrict__ slots, int H, int d, int dv, int n_blocks) {
+  __shared__ float wf[8], wm[8], last[MG_TOKENS + 1];
+  pdl_prologue();
+  const int s = blockIdx.x, h = blockIdx.y, tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int first = cu_q[s], n = cu_q[s + 1] - first, slot = slots[s];
+  if (slot < 0) return;
+  float m0 = q_start[s] == 0 ? 0.f : state[(size_t)slot * state_stride + (size_t)H * dv * d + (size_t)h * n_blocks * (d + 1) + d];
+  const float bi = gate_bias[h], bf = gate_bias[H + h];
+  for (int c0 = 0; c0 < n; c0 += MG_TOKENS) {
+    const bool there = c0 + tid < n;
+    float f = 0.f, i = -INFINITY;
+    if (there) {
+      const float* g = gates + (size_t)(first + c0 + tid) * gate_stride;
+      i = cap * tanhf((g[h] + bi) / cap);
+      f = ml_logsigmoid(cap * tanhf((g[H + h] + bf) / cap));
+    }
+    float F = f, M = i;
+#pragma unroll
+    for (int o = 1; o < 32; o <<= 1) {
+      const float Fl = __shfl_up_sync(0xffffffffu, F, o), Ml = __shfl_up_sync(0xffffffffu, M, o);
+      if (lane >= o) {
+        M = fmaxf(Ml + F, M);
+        F += Fl;
+      }
+    }
+    if (lane == 31) { wf[warp] = F; wm[warp] = M; }
+    __syncthreads();
+    float start = m0;                                     // m before the warp's first token
+    for (int w = 0; w < warp; ++w) start = fmaxf(wf[w] + start, wm[w]);
+    const float m = fmaxf(F + start, M);
+    last[tid + 1] = m;
+    if (tid == 0) last[0] = m0;
+    __syncthreads();
+    if (there) {
+      const float before = last[tid];
+      const size_t at = (size_t)(first + c0 + tid) * H + h;
+      a[at] = expf(f + before - m);
+      b[at] = expf(i - m);
+      em[at] = expf(-m);
+      top[at] = m;
+    }
+    m0 = last[min(MG_TOKENS, n - c0)];
+    __syncthreads();
+  }
+}
+
+// qk [2, T, H d] fp32: q times d^-1/2, then k; four elements a thread
+template <typename T>
+__global__ void mlstm_widen_kernel(float* __restrict__ qk, const T* __restrict__ proj, int proj_stride, int n_tokens, int qk_size,
+                                   float qscale) {
+  pdl_prologue();
+  const long quarter = qk_size / 4, total = (long)n_tokens * 2 * quarter;
+  for (long e = (long)blockIdx.x * blockDim.x + threadIdx.x; e < total; e += (long)gridDim.x * blockDim.x) {
+    const long t = e / (2 * quarter), c = 4 * (e - t * 2 * quarter);
+    float4 v = cs_load4(proj + (size_t)t * proj_stride + c);
+    const bool q = c < qk_size;
+    if (q) v = make_float4(v.x * qscale, v.y * qscale, v.z * qscale, v.w * qscale);
+    *reinterpret_cast<float4*>(qk + (q ? 0 : (size_t)n_tokens * qk_size - qk_size) + (size_t)t * qk_size + c) = v;
+  }
+}
+
+struct MlstmGates {
+  const float *a, *b, *em;
+  int H;
+  __device__ __forceinline__ void operator()(int t, int h, float& gate, float& weight, float& e) const {
+    const size_t at = (size_t)t * H + h;
+    gate = a[at];
+    weight = b[at];
+    e = em[at];
+  }
+};
+
+// Floats of scratch for the above: per chunk and head, and per token (nhv_mlstm_scan's `chunks`).
+NHV_API int nhv_mlstm_chunk_floats(int n_tokens, int n_seqs, int H, int d) {
+  const long floats = cs_chunks(n_tokens, n_seqs) * H * (CS_WORK + 2 * CS_C + d) + (long)n_tokens * H * (2 * d + 4);
+  return floats < (1l << 31) - 1 ? (int)floats : 0;       // 0: beyond what this counts; the step goes token by token
+}
+
 // Floats of state that one request needs (the host sizes its slots with this).
 NHV_API int nhv_mlstm_state_floats(int H, int d, int dv) {
   const int nb = (dv + ML_COLS - 1) / ML_COLS;
@@ -302,11 +393,12 @@ NHV_API int nhv_mlstm_state_floats(int H, int d, int dv) {
 }
 
 // proj [T, >= 2*H*d + H*dv] (q, then k, then v, per head), gates [T, >= 2*H] fp32 (input gates, then forget gates,
-// before bias and cap), gate_bias [2*H] fp32, y [T, H*dv] fp32.
+// before bias and cap), gate_bias [2*H] fp32, y [T, H*dv] fp32.  chunks: scratch of nhv_mlstm_chunk_floats floats to go
+// through prompts a chunk of tokens at a time (d up to 128, sizes in steps of 4; null: token by token).
 NHV_API int nhv_mlstm_scan(int dtype, float* y, const void* proj, int proj_stride, const float* gates, int gate_stride,
                            const float* gate_bias, float cap, float* state, long state_stride, const int* cu_q,
                            const int* q_start, const int* slots, int n_seqs, int n_tokens, int H, int d, int dv, int lanes,
-                           cudaStream_t stream) {
+                           float* chunks, cudaStream_t stream) {
   if (n_tokens == 0 || n_seqs == 0) return 0;
   NHV_REQUIRE(H > 0 && d > 0 && dv > 0 && cap > 0.f, "mlstm_scan: bad sizes");
   NHV_REQUIRE(d <= 512, "mlstm_scan: a key head of %d elements is beyond the supported 512", d);
@@ -331,6 +423,37 @@ NHV_API int nhv_mlstm_scan(int dtype, float* y, const void* proj, int proj_strid
     else STEP_D(__nv_bfloat16);
 #undef STEP_D
 #undef STEP
+    NHV_CHECK_LAUNCH("mlstm_scan");
+    return 0;
+  }
+  const int four = dtype == NHV_F32 ? 16 : 8;             // bytes of four elements
+  if (chunks && lanes == 0 && d % 4 == 0 && d <= 128 && dv % 4 == 0 && proj_stride % 4 == 0 && ((uintptr_t)proj % four) == 0) {
+    const int nb = (dv + ML_COLS - 1) / ML_COLS;
+    static_assert(ML_COLS == CS_COLS, "a copy of n per block of columns");
+    const long nc = cs_chunks(n_tokens, n_seqs), th = (long)n_tokens * H;
+    float* extra = chunks + nc * H * CS_WORK;
+    float* qk = extra + nc * H * (2 * CS_C + d);
+    float *a = qk + 2 * th * d, *b = a + th, *em = b + th, *top = em + th;
+    nhv_launch(mlstm_gates_kernel, dim3(n_seqs, H), MG_TOKENS, 0, stream, a, b, em, top, gates, gate_stride, gate_bias, cap,
+               (const float*)state, state_stride, cu_q, q_start, slots, H, d, dv, nb);
+    const long work = (long)n_tokens * H * d / 2;
+    const int blocks = (int)(work / 256 + 1 < 148 * 8 ? work / 256 + 1 : 148 * 8);
+    const float qscale = 1.0f / sqrtf((float)d);
+    if (dtype == NHV_F32)
+      nhv_launch(mlstm_widen_kernel<float>, blocks, 256, 0, stream, qk, (const float*)proj, proj_stride, n_tokens, H * d, qscale);
+    else
+      nhv_launch(mlstm_widen_kernel<__nv_bfloat16>, blocks, 256, 0, stream, qk, (const __nv_bfloat16*)proj, proj_stride,
+                 n_tokens, H * d, qscale);
+    const CsPairs pp{qk, qk + th * d, (long)H * d, chunks, extra, cu_q, slots, n_seqs, H, H, d};
+    const MlstmGates mg{a, b, em, H};
+    const void* v = dtype == NHV_F32 ? (const void*)((const float*)proj + 2 * H * d)
+                                     : (const void*)((const __nv_bfloat16*)proj + 2 * H * d);
+    const CsScan ps{y, pp.q, pp.k, (long)H * d, v, proj_stride, chunks, nullptr, extra, top, state, state_stride, cu_q, q_start,
+                    slots, H, H, d, dv};
+#define CHUNKS(D)                                                                                            do {                                                                                                         NHV_CUDA((cs_launch_pairs<D, CS_NORMED>(pp, mg, n_tokens, stream)), "mlstm_scan");                         if (dtype == NHV_F32) NHV_CUDA((cs_launch_scan<D, CS_NORMED, float>(ps, n_seqs, stream)), "mlstm_scan");     else NHV_CUDA((cs_launch_scan<D, CS_NORMED, __nv_bfloat16>(ps, n_seqs, stream)), "mlstm_scan");          } while (0)
+    if (d <= 64) CHUNKS(64);
+    else CHUNKS(128);
+#undef CHUNKS
     NHV_CHECK_LAUNCH("mlstm_scan");
     return 0;
   }

@@ -19,6 +19,7 @@
 // with w indexed by (column mod w_period).  gate_kind 1 puts sigmoid(z) in the place of silu(z).
 #include <math.h>
 
+#include "nhv_chunk_scan.cuh"
 #include "nhv_common.cuh"
 
 constexpr int SS_PARTS = 4;
@@ -402,15 +403,45 @@ __global__ void __launch_bounds__(SF_THREADS) ssd_scan_wide_kernel(
 
 // xbc [T, H*P + 2*G*N] (x, then B, then C), dt_raw [T, >= H] fp32, y [T, H*P] fp32.  lanes: 8, 16 or 32 lanes per
 // column of the state in the fast form, or 0 to choose by the size of the step.
+struct SsdGates {
+  const float* dt_raw;                                   // row t, head h: at t * dt_stride + h
+  int dt_stride;
+  const float *dt_bias, *a_log;
+  __device__ __forceinline__ void operator()(int t, int h, float& gate, float& weight, float&) const {
+    weight = ss_softplus(dt_raw[(size_t)t * dt_stride + h] + dt_bias[h]);
+    gate = expf(-expf(a_log[h]) * weight);
+  }
+};
+
+// chunks: scratch of (n_tokens / 32 + n_seqs) * H * nhv_chunk_scan_floats() floats to go through prompts a chunk of tokens
+// at a time (fp32 inputs, N up to 128, sizes in steps of 4; null: token by token).
 NHV_API int nhv_ssd_scan(int dtype, float* y, const void* xbc, int xbc_stride, const float* dt_raw, int dt_stride,
                          const float* dt_bias, const float* a_log, const float* d_skip, float* state,
                          long state_stride, const int* cu_q, const int* q_start, const int* slots, int n_seqs,
-                         int n_tokens, int H, int P, int N, int G, int lanes, int cpt, cudaStream_t stream) {
+                         int n_tokens, int H, int P, int N, int G, int lanes, int cpt, float* chunks,
+                         cudaStream_t stream) {
   if (n_tokens == 0 || n_seqs == 0) return 0;
   NHV_REQUIRE(G > 0 && H > 0 && H % G == 0, "ssd_scan: %d heads do not divide into %d groups", H, G);
   NHV_REQUIRE(N > 0 && N <= 256 && P > 0, "ssd_scan: a state of %d rows is beyond the supported 256", N);
   NHV_REQUIRE(state_stride >= (long)H * P * N, "ssd_scan: the state holds fewer than heads * P * N floats");
   const bool fast = dtype == NHV_F32 && N % 4 == 0 && P % 4 == 0 && xbc_stride % 4 == 0 && ((uintptr_t)xbc % 16) == 0;
+  if (chunks && fast && N <= 128) {
+    const float* rows = (const float*)xbc;
+    const CsPairs pp{rows + (size_t)H * P + (size_t)G * N, rows + (size_t)H * P, xbc_stride, chunks, nullptr, cu_q, slots,
+                     n_seqs, G, H, N};
+    const SsdGates gates{dt_raw, dt_stride, dt_bias, a_log};
+    const CsScan ps{y, pp.q, pp.k, xbc_stride, rows, xbc_stride, chunks, d_skip, nullptr, nullptr, state, state_stride, cu_q,
+                    q_start, slots, G, H, N, P};
+    if (N <= 64) {
+      NHV_CUDA((cs_launch_pairs<64, CS_PLAIN>(pp, gates, n_tokens, stream)), "ssd_scan");
+      NHV_CUDA((cs_launch_scan<64, CS_PLAIN, float>(ps, n_seqs, stream)), "ssd_scan");
+    } else {
+      NHV_CUDA((cs_launch_pairs<128, CS_PLAIN>(pp, gates, n_tokens, stream)), "ssd_scan");
+      NHV_CUDA((cs_launch_scan<128, CS_PLAIN, float>(ps, n_seqs, stream)), "ssd_scan");
+    }
+    NHV_CHECK_LAUNCH("ssd_scan");
+    return 0;
+  }
   // columns per lane (cpt: 1, 2, 4, or 0 to choose): one while the blocks of 16 columns leave SMs idle, more when
   // the SMs are full and the reads of B and C from shared memory are what costs
   if (cpt <= 0) {

@@ -213,11 +213,37 @@ SCAN_COLUMNS = 0    # columns of a scan's state per lane: 0 is the kernel's choi
 SCAN_GROUP4 = -1    # the delta rule's scan four tokens per round of its chain: -1 is the kernel's choice (off); tests set 1
 SCAN_LANES = 0      # lanes per state column in the recurrent scans: 0 is the kernels' own choice; tests set 4, 8, 16, 32
 
+# Tokens per request, on average, from which a scan goes through a step 32 tokens at a time; 0 is the rule below, tests set it
+CHUNK_SCAN_TOKENS = 0
 
-def delta_rule(o, qkv, ba, a_log, dt_bias, state, batch, G: int, H: int, d: int, dv: int) -> None:
+
+def _by_chunks(n_tokens: int, n_seqs: int, blocks: int, normed: bool) -> bool:
+    """Whether a scan goes by chunks.  ``blocks``: (request, head, 16 columns) of the step; an SM takes two at a time.
+    By chunks against by tokens, in us, on heads of 128 rows and 2,048 columns of state in all: gated delta rule 544 / 1,077
+    (one request of 4,096 tokens), 67 / 80 (200), 55 / 62 (128), 47 / 45 (64), 560 / 753 (5 of 333 to 1,501), but 399 / 326
+    (8 of 512), where a token's work for all requests fills the SMs as it is; the state space 386 / 821, 50 / 60, 43 / 45,
+    38 / 33, 401 / 499 and 282 / 244.  The mLSTM's scan by tokens costs more: 599 / 1,498, 55 / 66 (128), 45 / 43 (64),
+    519 / 1,109, 366 / 734, 8 of 32 tokens 56 / 67."""
+    if CHUNK_SCAN_TOKENS:
+        return n_tokens >= CHUNK_SCAN_TOKENS * n_seqs
+    if normed:
+        return n_tokens >= 32 * n_seqs
+    return n_tokens >= 128 * n_seqs and blocks <= 5 * 148
+
+
+def _chunk_scratch(n_tokens: int, n_seqs: int, heads: int, columns: int, device):
+    """Scratch for a scan by chunks, or None where the step goes by tokens (or a test asks for a form of that scan)."""
+    if SCAN_LANES or SCAN_GROUP4 == 1 or SCAN_COLUMNS or not _by_chunks(n_tokens, n_seqs, n_seqs * heads * -(-columns // 16), False):
+        return None
+    floats = (n_tokens // 32 + n_seqs) * heads * library.load_library().nhv_chunk_scan_floats()
+    return torch.empty(floats, dtype=torch.float32, device=device)
+
+
+def delta_rule(o, qkv, ba, a_log, dt_bias, state, batch, G: int, H: int, d: int, dv: int, fixed_order: bool = False) -> None:
     """The gated delta rule over the step's tokens.  qkv [T, 2*G*d + H*dv] (q, k, v after their convolutions), ba
     [T, 2*H] float32 (inputs of beta's sigmoid, then of the decay's softplus), a_log / dt_bias [H] float32, state
-    [slots, H*dv*d] float32 -> o [T, H*dv] float32 (before its norm and gate)."""
+    [slots, H*dv*d] float32 -> o [T, H*dv] float32 (before its norm and gate).  ``fixed_order``: token by token, so that
+    a result does not depend on how the tokens were cut into steps; else long prompts go 32 tokens at a time."""
     _need_cuda(o, qkv, ba, a_log, dt_bias, state)
     T = qkv.shape[0]
     assert qkv.stride(1) == 1 and qkv.shape[1] == 2 * G * d + H * dv
@@ -230,24 +256,28 @@ def delta_rule(o, qkv, ba, a_log, dt_bias, state, batch, G: int, H: int, d: int,
         ptrs.append(scratch.data_ptr() + 4 * at)
         at += n
     qn, kn, v32, pairs, kq, beta, decay = ptrs
+    chunks = (None if fixed_order or d > 128 or d % 4 or dv % 4 else _chunk_scratch(T, batch.n_seqs, H, dv, qkv.device))
     call("nhv_delta_rule", dtype_code(qkv), o.data_ptr(), qkv.data_ptr(), qkv.stride(0), ba.data_ptr(), a_log.data_ptr(),
          dt_bias.data_ptr(), state.data_ptr(), state.stride(0), qn, kn, kq, v32, beta, decay, batch.cu_q.data_ptr(),
          batch.q_start.data_ptr(), batch.state_slots.data_ptr(), batch.n_seqs, T, G, H, d, dv, SCAN_LANES, SCAN_GROUP4, pairs,
-         SCAN_COLUMNS, stream_ptr())
+         SCAN_COLUMNS, _ptr(chunks), stream_ptr())
 
 
-def ssd_scan(y, xbc, dt_raw, dt_bias, a_log, d_skip, state, batch, H: int, P: int, N: int, G: int) -> None:
-    """The Mamba-2 recurrence over the step's tokens.  xbc [T, H*P + 2*G*N] (x, B, C after the convolution), dt_raw
+def ssd_scan(y, xbc, dt_raw, dt_bias, a_log, d_skip, state, batch, H: int, P: int, N: int, G: int,
+             fixed_order: bool = False) -> None:
+    """The Mamba-2 recurrence over the step's tokens (``fixed_order`` as in ``delta_rule``).  xbc [T, H*P + 2*G*N] (x, B, C after the convolution), dt_raw
     [T, H] float32 (before bias and softplus), state [slots, H*P*N] float32 -> y [T, H*P] float32."""
     _need_cuda(y, xbc, dt_raw, dt_bias, a_log, d_skip, state)
     T = xbc.shape[0]
     assert xbc.stride(1) == 1 and xbc.shape[1] == H * P + 2 * G * N and dt_raw.stride(1) == 1 and dt_raw.shape == (T, H)
     assert y.dtype == dt_raw.dtype == dt_bias.dtype == a_log.dtype == d_skip.dtype == state.dtype == torch.float32
     assert y.is_contiguous() and y.shape == (T, H * P)
+    chunks = (None if fixed_order or xbc.dtype != torch.float32 or N > 128 or N % 4 or P % 4
+              else _chunk_scratch(T, batch.n_seqs, H, P, xbc.device))
     call("nhv_ssd_scan", dtype_code(xbc), y.data_ptr(), xbc.data_ptr(), xbc.stride(0), dt_raw.data_ptr(), dt_raw.stride(0),
          dt_bias.data_ptr(), a_log.data_ptr(), d_skip.data_ptr(), state.data_ptr(), state.stride(0), batch.cu_q.data_ptr(),
          batch.q_start.data_ptr(), batch.state_slots.data_ptr(), batch.n_seqs, T, H, P, N, G, SCAN_LANES,
-         SCAN_COLUMNS, stream_ptr())
+         SCAN_COLUMNS, _ptr(chunks), stream_ptr())
 
 
 def gated_rmsnorm(out, y, z, weight, n_groups: int, eps: float, gate_first: bool, gate: str = "silu") -> None:
@@ -650,8 +680,8 @@ def mlstm_state_floats(H: int, d: int, dv: int) -> int:
     return H * dv * d + H * -(-dv // MLSTM_COLUMN_BLOCK) * (d + 1)
 
 
-def mlstm_scan(y, proj, gates, gate_bias, cap: float, state, batch, H: int, d: int, dv: int) -> None:
-    """The mLSTM recurrence over the step's tokens.  proj [T, >= 2*H*d + H*dv] (q, k, v per head; a view with unit
+def mlstm_scan(y, proj, gates, gate_bias, cap: float, state, batch, H: int, d: int, dv: int, fixed_order: bool = False) -> None:
+    """The mLSTM recurrence over the step's tokens (``fixed_order`` as in ``delta_rule``).  proj [T, >= 2*H*d + H*dv] (q, k, v per head; a view with unit
     column stride), gates [T, 2*H] float32 (input then forget gates, before bias and cap), gate_bias [2*H] float32,
     state [slots, mlstm_state_floats] float32 -> y [T, H*dv] float32 (before its norm and gate)."""
     _need_cuda(y, proj, gates, gate_bias, state)
@@ -661,9 +691,13 @@ def mlstm_scan(y, proj, gates, gate_bias, cap: float, state, batch, H: int, d: i
     assert y.is_contiguous() and y.shape == (T, H * dv) and gates.stride(1) == 1 and gates.shape == (T, 2 * H)
     assert gate_bias.numel() == 2 * H and state.dim() == 2 and state.stride(1) == 1
     assert state.shape[1] >= mlstm_state_floats(H, d, dv)
+    chunks = None
+    if not fixed_order and not MLSTM_LANES and d <= 128 and d % 4 == 0 and dv % 4 == 0 and _by_chunks(T, batch.n_seqs, 0, True):
+        floats = library.load_library().nhv_mlstm_chunk_floats(T, batch.n_seqs, H, d)
+        chunks = torch.empty(floats, dtype=torch.float32, device=proj.device) if floats else None
     call("nhv_mlstm_scan", dtype_code(proj), y.data_ptr(), proj.data_ptr(), proj.stride(0), gates.data_ptr(), gates.stride(0),
          gate_bias.data_ptr(), float(cap), state.data_ptr(), state.stride(0), batch.cu_q.data_ptr(), batch.q_start.data_ptr(),
-         batch.state_slots.data_ptr(), batch.n_seqs, T, H, d, dv, MLSTM_LANES, stream_ptr())
+         batch.state_slots.data_ptr(), batch.n_seqs, T, H, d, dv, MLSTM_LANES, _ptr(chunks), stream_ptr())
 
 
 def moe_route(ids, weights, logits, correction, n_outputs: int, n_groups: int, keep: int, scores: str = "softmax",

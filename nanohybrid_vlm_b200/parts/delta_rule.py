@@ -74,7 +74,8 @@ class GatedDeltaRule(Mixer):
         qkv = self.new(T, C, dtype=torch.float32)      # what enters the recurrence stays 32-bit
         ops.short_conv_silu(qkv, proj[:, :C], self.w_conv, None, conv_state, batch)
         o = self.new(T, self.v_size, dtype=torch.float32)
-        ops.delta_rule(o, qkv, ba, self.w_A_log, self.w_dt_bias, rule_state, batch, self.G, self.H, self.d, self.dv)
+        ops.delta_rule(o, qkv, ba, self.w_A_log, self.w_dt_bias, rule_state, batch, self.G, self.H, self.d, self.dv,
+                       fixed_order=x.dtype == torch.float32)
         gated = self.new(T, self.v_size)
         ops.gated_rmsnorm(gated, o, proj[:, C:], self.w_norm, self.H, self.eps, gate_first=False)
         out = self.new(T, self.env.hidden_size)

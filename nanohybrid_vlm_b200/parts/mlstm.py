@@ -61,7 +61,8 @@ class MLSTM(Mixer):
         gates = self.new(T, 2 * self.H, dtype=torch.float32)
         ops.linear_f32(gates, x, self.w_if)
         o = self.new(T, v, dtype=torch.float32)
-        ops.mlstm_scan(o, proj, gates, self.w_if_bias, self.cap, cache.state, batch, self.H, self.d, self.dv)
+        ops.mlstm_scan(o, proj, gates, self.w_if_bias, self.cap, cache.state, batch, self.H, self.d, self.dv,
+                       fixed_order=x.dtype == torch.float32)
         gated = self.new(T, v)
         ops.gated_rmsnorm(gated, o, proj[:, 2 * qk + v:], self.w_norm, self.H, self.eps, gate_first=False, gate="sigmoid")
         out = self.new(T, self.env.hidden_size)

@@ -77,7 +77,7 @@ class Mamba2(Mixer):
         ops.short_conv_silu(xbc, zxbc[:, self.inner:], self.w_conv, self.w_conv_b, conv_state, batch)
         y = self.new(T, self.inner, dtype=torch.float32)
         ops.ssd_scan(y, xbc, dt, self.w_dt_bias, self.w_A_log, self.w_D, ssm_state, batch, self.heads, self.P, self.N,
-                     self.G)
+                     self.G, fixed_order=x.dtype == torch.float32)
         gated = self.new(T, self.inner)
         ops.gated_rmsnorm(gated, y, zxbc[:, :self.inner], self.w_norm, self.norm_groups, self.eps, gate_first=True)
         out = self.new(T, self.env.hidden_size)
