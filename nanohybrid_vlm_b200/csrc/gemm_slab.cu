@@ -22,7 +22,9 @@
 //
 // Modes: 0: y bf16.  1: y fp32, rounded through bf16 as nanovllm/layers/embed_head.py:61 with
 // nanovllm/layers/sampler.py:12 gives logits.  2: y = silu(gate) * up (nanovllm/layers/activation.py:9-11), both
-// products rounded to bf16 first.  W is [out, in] (nanovllm/layers/linear.py:40,66).
+// products rounded to bf16 first.  W is [out, in] (nanovllm/layers/linear.py:40,66).  Other units on the same layouts
+// (`unit`): 1, on mode 2: gelu_tanh(gate) * up; 2 and 3, on mode 0: relu(y)^2 and gelu_tanh(y); each of products rounded
+// to bf16 first, as a kernel of its own behind the product would read them (that launch cost a decode step 3 to 4 us).
 #include "nhv_async.cuh"
 
 // Test builds only (tests compile this file into a library of its own with a short NHV_WAIT_LIMIT): the producer
@@ -58,6 +60,9 @@ __device__ __forceinline__ void mma_bf16(float (&c)[4], const uint32_t (&a)[4], 
                : "r"(a[0]), "r"(a[1]), "r"(a[2]), "r"(a[3]), "r"(b0), "r"(b1));
 }
 __device__ __forceinline__ void consumer_sync() { asm volatile("bar.sync 1, %0;\n" ::"n"(CONSUMER_WARPS * 32) : "memory"); }
+__device__ __forceinline__ float gelu_tanh(float z) {
+  return 0.5f * z * (1.0f + tanhf(0.7978845608028654f * (z + 0.044715f * z * z * z)));
+}
 struct alignas(64) Params {
   CUtensorMap x_map;     // x [M, K]: x3d: as [K / 64][M][64], one box is a stage's columns; else box 64 columns x 8 rows
   const unsigned char* slabs;
@@ -67,6 +72,7 @@ struct alignas(64) Params {
   int rpb;               // result columns per block
   int nb;                // boxes of 64 columns per stage
   int ks;                // stages over K (K padded to ks * nb * 64 columns in the copy)
+  int unit;              // 0: the mode's own
   int x3d;               // K is a multiple of 64: a stage's columns of x come in one copy
   // a hint: the copy that the product after this one will read; block c asks its first bytes into L2 as it sends
   // for its own last stage (null: no hint)
@@ -223,7 +229,12 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_slab_kernel(const __grid_cons
         float v = value(r);
         if (p.mode == 2) {
           const float up = value(h + r);                           // the rows of up follow the rows of gate
-          v = v / (1.0f + expf(-v)) * up;
+          v = (p.unit == 1 ? gelu_tanh(v) : v / (1.0f + expf(-v))) * up;
+        } else if (p.unit == 2) {
+          const float r = fmaxf(v, 0.f);
+          v = r * r;
+        } else if (p.unit == 3) {
+          v = gelu_tanh(v);
         }
         if (p.mode == 1)
           reinterpret_cast<float*>(p.y)[(size_t)m * p.ldc + n] = v;
@@ -279,22 +290,30 @@ NHV_API int nhv_gemm_slab_geometry(int N, int K, int mode, int sms, int* blocks,
 // slabs: the copy made by ops.slab_weight for exactly this geometry (nhv_gemm_slab_geometry with the same N, K,
 // mode and SM count).
 static int gemm_slab_launch(void* y, const void* x, const void* slabs, int M, int N, int K, int lda, int ldc, int mode,
-                            int sms, const void* next_slabs, long long next_slab_bytes, int next_bytes, int next_blocks,
-                            cudaStream_t stream);
+                            int unit, int sms, const void* next_slabs, long long next_slab_bytes, int next_bytes,
+                            int next_blocks, cudaStream_t stream);
 NHV_API int nhv_gemm_slab(void* y, const void* x, const void* slabs, int M, int N, int K, int lda, int ldc, int mode,
                           int sms, cudaStream_t stream) {
-  return gemm_slab_launch(y, x, slabs, M, N, K, lda, ldc, mode, sms, nullptr, 0, 0, 0, stream);
+  return gemm_slab_launch(y, x, slabs, M, N, K, lda, ldc, mode, 0, sms, nullptr, 0, 0, 0, stream);
 }
 // The same with a hint: the copy (and its geometry: bytes per block, blocks) that the next product will read, of which
 // every block asks `next_bytes` into L2 when it has sent for its own last stage.
 NHV_API int nhv_gemm_slab_hint(void* y, const void* x, const void* slabs, int M, int N, int K, int lda, int ldc, int mode,
                                int sms, const void* next_slabs, long long next_slab_bytes, int next_bytes, int next_blocks,
                                cudaStream_t stream) {
-  return gemm_slab_launch(y, x, slabs, M, N, K, lda, ldc, mode, sms, next_slabs, next_slab_bytes, next_bytes, next_blocks, stream);
+  return gemm_slab_launch(y, x, slabs, M, N, K, lda, ldc, mode, 0, sms, next_slabs, next_slab_bytes, next_bytes, next_blocks, stream);
+}
+// The same with a unit behind the product (`next_slabs` may be null).
+NHV_API int nhv_gemm_slab_unit(void* y, const void* x, const void* slabs, int M, int N, int K, int lda, int ldc, int mode,
+                               int unit, int sms, const void* next_slabs, long long next_slab_bytes, int next_bytes,
+                               int next_blocks, cudaStream_t stream) {
+  NHV_REQUIRE(unit == 0 || (unit == 1 && mode == 2) || ((unit == 2 || unit == 3) && mode == 0),
+              "gemm_slab: no unit %d on mode %d", unit, mode);
+  return gemm_slab_launch(y, x, slabs, M, N, K, lda, ldc, mode, unit, sms, next_slabs, next_slab_bytes, next_bytes, next_blocks, stream);
 }
 static int gemm_slab_launch(void* y, const void* x, const void* slabs, int M, int N, int K, int lda, int ldc, int mode,
-                            int sms, const void* next_slabs, long long next_slab_bytes, int next_bytes, int next_blocks,
-                            cudaStream_t stream) {
+                            int unit, int sms, const void* next_slabs, long long next_slab_bytes, int next_bytes,
+                            int next_blocks, cudaStream_t stream) {
   if (M == 0 || N == 0) return 0;
   NHV_REQUIRE(M > 0 && M <= X_ROWS, "gemm_slab: takes 1 to %d tokens, got %d", X_ROWS, M);
   NHV_REQUIRE(K % 8 == 0 && lda % 8 == 0 && lda >= K && ldc >= N,
@@ -305,7 +324,7 @@ static int gemm_slab_launch(void* y, const void* x, const void* slabs, int M, in
   if (int rc = nhv_gemm_slab_geometry(N, K, mode, sms, &blocks, &p.rpb, &p.nb, &p.ks, &p.slab_bytes)) return rc;
   p.slabs = (const unsigned char*)slabs;
   p.y = y;
-  p.M = M; p.N = N; p.K = K; p.ldc = ldc; p.mode = mode;
+  p.M = M; p.N = N; p.K = K; p.ldc = ldc; p.mode = mode; p.unit = unit;
   p.next_slabs = (const unsigned char*)next_slabs;
   p.next_slab_bytes = next_slab_bytes;
   p.next_bytes = next_bytes < next_slab_bytes ? next_bytes / 16 * 16 : (int)(next_slab_bytes / 16 * 16);

@@ -1340,6 +1340,26 @@ def swiglu_first_half(act, x, gate_up_weight) -> bool:
     return True
 
 
+_SLAB_UNITS = {"gelu_tanh_mul": (2, 1), "relu_squared": (0, 2), "gelu_tanh": (0, 3)}      # layout of the copy, kernel's unit
+
+
+def product_with_unit(out, x, weight, unit: str) -> bool:
+    """out[M, I] = the feed-forward's unit of x weight^T in one kernel: ``gelu_tanh_mul`` (weight [2 I, K], gate rows first),
+    ``relu_squared`` or ``gelu_tanh`` (weight [I, K]).  For up to 8 tokens and a weight whose copy for the
+    weight-streaming kernel is laid out for that; returns False if it did not run."""
+    mode, code = _SLAB_UNITS[unit]
+    slab = _slabs.get(weight.data_ptr())
+    if (not small_m_ok(x, weight) or x.shape[0] > SLAB_MAX_M or slab is None or slab[0]() is not weight or slab[2] != mode):
+        return False
+    _need_cuda(out, x, weight)
+    _contig("out", out); _contig("weight", weight)
+    M, K = x.shape
+    N = weight.shape[0] // (2 if mode == 2 else 1)
+    assert out.shape == (M, N) and out.dtype == torch.bfloat16 and weight.shape[1] == K and x.stride(1) == 1
+    _slab_product(out, x, slab[1], M, N, K, mode, _sm_count(x.device), code)
+    return True
+
+
 _stream_k_state: dict = {}
 STREAM_K_COUNTERS = 8192
 
@@ -1367,7 +1387,7 @@ def _small_m(out, x, weight, M: int, N: int, K: int, mode: int, up_row_offset: i
          up_row_offset, scratch.data_ptr(), counters.data_ptr(), STREAM_K_COUNTERS, sms, stream_ptr())
 
 
-def _slab_product(out, x, copy, M: int, N: int, K: int, mode: int, sms: int) -> None:
+def _slab_product(out, x, copy, M: int, N: int, K: int, mode: int, sms: int, unit: int = 0) -> None:
     """The product from the per-SM copy, with a hint for the one after it.  A decode step runs the same products in
     the same order every time, so each remembers which copy was read right after its own last time; its blocks then
     ask the first bytes of that copy into L2 as they send for their own last stage, and the next product's ring
@@ -1386,10 +1406,18 @@ def _slab_product(out, x, copy, M: int, N: int, K: int, mode: int, sms: int) -> 
     nxt = hint[0]() if hint is not None else None
     if nxt is not None and nxt.data_ptr() == hint[1] and nxt.numel() * nxt.element_size() == hint[2] and SLAB_HINT_BYTES:
         blocks = min(sms, _slab_blocks.get(hint[1], 0))
+        if blocks > 0 and unit:
+            call("nhv_gemm_slab_unit", out.data_ptr(), x.data_ptr(), key, M, N, K, x.stride(0), N, mode, unit, sms, hint[1],
+                 hint[2] // blocks, SLAB_HINT_BYTES, blocks, stream_ptr())
+            return
         if blocks > 0:
             call("nhv_gemm_slab_hint", out.data_ptr(), x.data_ptr(), key, M, N, K, x.stride(0), N, mode, sms, hint[1],
                  hint[2] // blocks, SLAB_HINT_BYTES, blocks, stream_ptr())
             return
+    if unit:
+        call("nhv_gemm_slab_unit", out.data_ptr(), x.data_ptr(), key, M, N, K, x.stride(0), N, mode, unit, sms, None, 0, 0, 0,
+             stream_ptr())
+        return
     call("nhv_gemm_slab", out.data_ptr(), x.data_ptr(), key, M, N, K, x.stride(0), N, mode, sms, stream_ptr())
 
 

@@ -60,12 +60,13 @@ class GatedMLP(FeedForward):
                 ParamDecl("down", (H, I), sources=(Source(down, 0, H),))]
 
     def streamed_weights(self):
-        return [(self.w_gate_up, 2 if self.activation == "silu" else 0), (self.w_down, 0)]
+        return [(self.w_gate_up, 2), (self.w_down, 0)]
 
     def forward(self, x, batch):
         T = x.shape[0]
         act = self.new(T, self.inter)
-        if self.activation != "silu" or not ops.swiglu_first_half(act, x, self.w_gate_up):
+        if not (ops.swiglu_first_half(act, x, self.w_gate_up) if self.activation == "silu"
+                else ops.product_with_unit(act, x, self.w_gate_up, self.ACTIVATIONS[self.activation])):
             gate_up = self.new(T, 2 * self.inter)
             ops.linear(gate_up, x, self.w_gate_up)
             getattr(ops, self.ACTIVATIONS[self.activation])(act, gate_up)
@@ -99,8 +100,10 @@ class DenseMLP(FeedForward):
     def forward(self, x, batch):
         T = x.shape[0]
         act = self.new(T, self.inter)
-        ops.linear(act, x, self.w_up)
-        getattr(ops, self.ACTIVATIONS[self.activation])(act)
+        unit = self.ACTIVATIONS[self.activation]
+        if not ops.product_with_unit(act, x, self.w_up, unit):
+            ops.linear(act, x, self.w_up)
+            getattr(ops, unit)(act)
         y = self.new(T, self.env.hidden_size)
         ops.linear(y, act, self.w_down)
         return y

@@ -14,6 +14,26 @@ def ops():
     return ops
 
 
+@pytest.mark.parametrize("unit,mode", [("gelu_tanh_mul", 2), ("relu_squared", 0), ("gelu_tanh", 0)])
+@pytest.mark.parametrize("M,inter,K", [(1, 40, 64), (8, 1000, 264), (5, 5632, 2048), (3, 148 * 70, 128)])
+def test_unit_behind_the_streaming_product(ops, unit, mode, M, inter, K):
+    g = torch.Generator().manual_seed(inter)
+    rows = 2 * inter if mode == 2 else inter
+    x = dev(torch.randn(M, K, generator=g).to(torch.bfloat16))
+    w = dev((torch.randn(rows, K, generator=g) * K ** -0.5).to(torch.bfloat16))
+    out = torch.full((M, inter), float("nan"), dtype=torch.bfloat16, device="cuda")
+    assert not ops.product_with_unit(out, x, w, unit)             # no copy of the weight
+    ops.prepare_streaming(w, mode)
+    assert ops.product_with_unit(out, x, w, unit)
+    assert not ops.product_with_unit(out, torch.cat([x] * 9)[:9], w, unit)
+    y = (x.double() @ w.double().t()).to(torch.bfloat16).double()
+    a, u = (y[:, :inter], y[:, inter:]) if mode == 2 else (y, 1.0)
+    want = torch.relu(a) ** 2 if unit == "relu_squared" else torch.nn.functional.gelu(a, approximate="tanh") * u
+    # the product in bfloat16 may round the other way (2^-8 of values of size 1, doubled by the square), then once more
+    torch.testing.assert_close(out.double(), want, rtol=3 * 2 ** -8, atol=2e-3)
+    assert ops.slab_error() == 0
+
+
 @pytest.mark.parametrize("dtype", [torch.float32, torch.bfloat16])
 @pytest.mark.parametrize("C,K", [(70, 4), (129, 2), (64, 8), (33, 1)])
 def test_filters_on_single_tokens(ops, dtype, C, K):
