@@ -21,6 +21,7 @@
 
 #include "nhv_chunk_scan.cuh"
 #include "nhv_common.cuh"
+#include "nhv_vec8.cuh"
 
 constexpr int SS_PARTS = 4;
 constexpr int SS_CHUNK = 16;
@@ -575,6 +576,81 @@ __global__ void gated_rmsnorm_kernel(T* __restrict__ out, int out_stride, const 
   }
 }
 
+// Eight elements a thread, sizes in steps of 8 and rows on 16-byte boundaries: the kernels above and below read an element
+// at a time and the weight's place by a division, 46 us for 4,096 rows of 16 groups of 128 (67 MB; 19 here) and 44 us for
+// 4,096 rows of 2,048.  LANES threads (a power of two) share a group, CHUNKS pieces of eight each, which stay in
+// registers between the sum of squares and the output.
+template <typename T, int LANES, int CHUNKS>
+__global__ void __launch_bounds__(256) gated_rmsnorm_vec_kernel(
+    T* __restrict__ out, int out_stride, const float* __restrict__ y, const T* __restrict__ z, int z_stride,
+    const T* __restrict__ w, int w_period, long n_items, int n_groups, int size, float eps, int gate_first, int gate_kind) {
+  __shared__ float red[8];
+  pdl_prologue();
+  const int lane = threadIdx.x % LANES;
+  const long item = (long)blockIdx.x * (256 / LANES) + threadIdx.x / LANES;
+  const bool live = item < n_items;
+  const long t = live ? item / n_groups : 0;
+  const int gidx = (int)((live ? item : 0) - t * n_groups);
+  const float* yr = y + ((size_t)t * n_groups + gidx) * size;
+  const T* zr = z + (size_t)t * z_stride + (size_t)gidx * size;
+  float v[CHUNKS][8], g[CHUNKS][8];
+  float ss = 0.f;
+#pragma unroll
+  for (int k = 0; k < CHUNKS; ++k) {
+    const int c = 8 * (lane + k * LANES);
+    if (live && c < size) {
+      nhv_load8(v[k], yr + c);
+      nhv_load8(g[k], zr + c);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) {
+        g[k][e] = gn_gate(g[k][e], gate_kind);
+        if (gate_first) v[k][e] *= g[k][e];
+        ss = fmaf(v[k][e], v[k][e], ss);
+      }
+    }
+  }
+#pragma unroll
+  for (int o = 1; o < (LANES < 32 ? LANES : 32); o <<= 1) ss += __shfl_xor_sync(0xffffffffu, ss, o);
+  if (LANES > 32) {                                       // the block's one group
+    if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = ss;
+    __syncthreads();
+    ss = 0.f;
+#pragma unroll
+    for (int i = 0; i < LANES / 32; ++i) ss += red[i];
+  }
+  if (!live) return;
+  const float rstd = 1.0f / sqrtf(ss / (float)size + eps);
+  const int w0 = (gidx * size) % w_period;
+  T* dst = out + (size_t)t * out_stride + (size_t)gidx * size;
+#pragma unroll
+  for (int k = 0; k < CHUNKS; ++k) {
+    const int c = 8 * (lane + k * LANES);
+    if (c < size) {
+      float wv[8];
+      nhv_load8(wv, w + (w0 + c) % w_period);
+#pragma unroll
+      for (int e = 0; e < 8; ++e) v[k][e] = v[k][e] * (gate_first ? 1.0f : g[k][e]) * rstd * wv[e];
+      nhv_store8(dst + c, v[k]);
+    }
+  }
+}
+
+template <typename T>
+static void gated_rmsnorm_vec(T* out, int out_stride, const float* y, const T* z, int z_stride, const T* w, int w_period,
+                              long items, int n_groups, int size, float eps, int gate_first, int gate_kind,
+                              cudaStream_t stream) {
+  auto go = [&](auto kernel, int lanes) {
+    const int per = 256 / lanes;
+    nhv_launch(kernel, (unsigned)((items + per - 1) / per), 256, 0, stream, out, out_stride, y, z, z_stride, w, w_period,
+               items, n_groups, size, eps, gate_first, gate_kind);
+  };
+  if (size <= 64) go(gated_rmsnorm_vec_kernel<T, 8, 1>, 8);
+  else if (size <= 128) go(gated_rmsnorm_vec_kernel<T, 16, 1>, 16);
+  else if (size <= 256) go(gated_rmsnorm_vec_kernel<T, 32, 1>, 32);
+  else if (size <= 2048) go(gated_rmsnorm_vec_kernel<T, 256, 1>, 256);
+  else go(gated_rmsnorm_vec_kernel<T, 256, 4>, 256);
+}
+
 // One warp per (token, group), for groups of up to 256 elements (a head of the delta rule): no barrier, the group's values stay in registers
 // between the sum of squares and the output.
 constexpr int GN_WARPS = 8;
@@ -620,6 +696,21 @@ NHV_API int nhv_gated_rmsnorm(int dtype, void* out, int out_stride, const float*
                               int gate_first, int gate_kind, cudaStream_t stream) {
   if (n_tokens == 0) return 0;
   NHV_REQUIRE(n_groups > 0 && size > 0 && w_period > 0, "gated_rmsnorm: bad sizes");
+  const long all = (long)n_tokens * n_groups;
+  // (a weight that ends inside a group starts over at a multiple of 8 as well)
+  if ((dtype == NHV_F32 || dtype == NHV_BF16) && size % 8 == 0 && size <= 8192 && w_period % 8 == 0 && out_stride % 8 == 0 &&
+      z_stride % 8 == 0 && all < (1L << 31) &&
+      (((uintptr_t)out | (uintptr_t)y | (uintptr_t)z | (uintptr_t)w) % 16) == 0) {
+    if (dtype == NHV_F32)
+      gated_rmsnorm_vec<float>((float*)out, out_stride, y, (const float*)z, z_stride, (const float*)w, w_period, all, n_groups,
+                               size, eps, gate_first, gate_kind, stream);
+    else
+      gated_rmsnorm_vec<__nv_bfloat16>((__nv_bfloat16*)out, out_stride, y, (const __nv_bfloat16*)z, z_stride,
+                                       (const __nv_bfloat16*)w, w_period, all, n_groups, size, eps, gate_first, gate_kind,
+                                       stream);
+    NHV_CHECK_LAUNCH("gated_rmsnorm");
+    return 0;
+  }
   if (size <= GN_MAX) {           // larger groups: a block per (token, group) below
     const long items = (long)n_tokens * n_groups;
     const long wblocks = (items + GN_WARPS - 1) / GN_WARPS;

@@ -1,0 +1,123 @@
+"""Kernels that take several elements a thread where sizes and addresses allow it, against 64-bit references and against the
+same kernels' general form (reached by rows an odd number of elements apart)."""
+import pytest
+import torch
+
+import plain_muvonex as pm
+from test_muvonex_ops_gpu import F64, dev, rotary_table, step_batch, tol
+
+pytestmark = pytest.mark.gpu
+
+DTYPES = [torch.float32, torch.bfloat16]
+
+
+@pytest.fixture(scope="module")
+def ops():
+    from nanohybrid_vlm_b200.kernels import ops
+    return ops
+
+
+def odd_rows(t):
+    """The same values in rows one element further apart."""
+    wide = torch.zeros(t.shape[0], t.shape[1] + 1, dtype=t.dtype, device=t.device)
+    wide[:, :-1] = t
+    return wide[:, :-1]
+
+
+# groups of 8, 16, 32 and 256 threads, one piece and four; a weight per group, per row, and one that ends inside a group
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("groups,size,period,gate_first", [(5, 64, 64, False), (3, 72, 216, True), (16, 128, 128, False),
+                                                           (2, 256, 512, True), (3, 96, 16, True), (1, 264, 264, True),
+                                                           (1, 2048, 2048, True), (2, 2056, 4112, False), (1, 8192, 8192, True),
+                                                           (1, 8200, 8200, True), (3, 128, 192, False)])
+def test_gated_rmsnorm(ops, dtype, groups, size, period, gate_first):
+    g = torch.Generator().manual_seed(size)
+    T, n = 9, groups * size
+    y = torch.randn(T, n, generator=g) * 3
+    z = torch.randn(T, n, generator=g).to(dtype)
+    w = (1 + 0.2 * torch.randn(period, generator=g)).to(dtype)
+    full = w.repeat(n // period) if n % period == 0 else None
+    for gate in ("silu", "sigmoid"):
+        outs = []
+        for zz in (dev(z), odd_rows(dev(z))):
+            out = torch.full((T, n), float("nan"), dtype=dtype, device="cuda")
+            ops.gated_rmsnorm(out, dev(y), zz, dev(w), groups, 1e-5, gate_first, gate)
+            outs.append(out)
+        torch.testing.assert_close(outs[0].float(), outs[1].float(), **tol(dtype, bf16=2 ** -7))
+    if full is not None:
+        ops.gated_rmsnorm(out, dev(y), dev(z), dev(w), groups, 1e-5, gate_first)
+        want = pm.gated_norm(y.to(F64), z.to(F64), full.to(F64), groups, 1e-5, gate_first)
+        torch.testing.assert_close(out.cpu().to(F64), want, **tol(dtype))
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("nq,nkv,dk,dv,rot,opts", [
+    (3, 1, 128, 128, 128, {}), (4, 2, 64, 32, 32, dict(weights=True)), (2, 2, 256, 128, 64, dict(norm_first=True, weights=True)),
+    (5, 1, 72, 40, 48, dict(eps=None)), (2, 1, 128, 128, 0, dict(bias=True, values_from_keys=True)), (3, 3, 8, 8, 0, {}),
+    (2, 1, 96, 96, 40, dict(interleaved=True)), (2, 2, 128, 64, 16, dict(norm_first=True)), (1, 1, 264, 8, 16, {})])
+def test_rope_norm_store(ops, dtype, nq, nkv, dk, dv, rot, opts):
+    g = torch.Generator().manual_seed(dk + nq)
+    opts = dict(opts)
+    T, page, n_pages, row = 13, 8, 4, -(-max(dk, dv) // 8) * 8 + 8
+    vk = opts.get("values_from_keys", False)
+    qkv = torch.randn(T, (nq + nkv) * dk + (0 if vk else nkv * dv), generator=g).to(dtype).cuda()
+    kw = dict(norm_first=opts.get("norm_first", False), interleaved=opts.get("interleaved", False), values_from_keys=vk)
+    if opts.get("weights"):
+        kw.update(q_weight=dev(torch.randn(dk, generator=g).to(dtype)), k_weight=dev(torch.randn(dk, generator=g).to(dtype)))
+    if opts.get("bias"):
+        kw.update(bias=dev(torch.randn((nq + nkv) * dk, generator=g).to(dtype)))
+    table = dev(rotary_table(rot, 10000.0, None, 50)) if rot else None
+    pos = torch.randint(0, 50, (T,), generator=g, dtype=torch.int32).cuda()
+    slots = torch.randperm(n_pages * page, generator=g)[:T].to(torch.int32)
+    slots[4] = -1                                              # stored nowhere
+    got = []
+    for x in (qkv, odd_rows(qkv)):
+        q = torch.full((T, nq * dk), float("nan"), dtype=dtype, device="cuda")
+        pages = torch.full((n_pages, 2, nkv, page, row), 7.0, dtype=dtype, device="cuda")
+        ops.rope_norm_store(x, q, pages, dev(slots), pos, table, rot, nq, nkv, dk, dv, opts.get("eps", 1e-5), **kw)
+        only = torch.full((T, nq * dk), float("nan"), dtype=dtype, device="cuda")
+        ops.rope_norm_store(x, only, None, None, pos, table, rot, nq, nkv, dk, dv, opts.get("eps", 1e-5), **kw)
+        assert torch.equal(only, q)
+        got.append((q.float(), pages.float()))
+    # the sum of squares in another order: results may round the other way
+    for a, b in zip(*got):
+        torch.testing.assert_close(a, b, **tol(dtype, f32=1e-6, bf16=2 ** -7))
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("C,K", [(68, 4), (132, 3), (516, 2), (64, 1)])
+def test_short_filters_of_long_steps(ops, dtype, C, K):
+    """Requests that end inside, at and before a tile of 16 tokens and a piece of four, fresh and with a past."""
+    g = torch.Generator().manual_seed(C)
+    news, starts, slots = [1, 300, 15, 17, 2, 250, 3], [4, 0, 9, 0, 1, 2, 0], [3, 0, 1, 6, 2, -1, 5]
+    T = sum(news)
+    x = torch.randn(T, C, generator=g).to(dtype).cuda()
+    w, w2 = (dev((torch.randn(C, K, generator=g) * 0.5).to(dtype)) for _ in range(2))
+    bias = dev((torch.randn(C, generator=g) * 0.3).to(dtype))
+    first = torch.randn(7, max(K - 1, 1) * C, generator=g).cuda()
+    got, b = [], step_batch(news, starts, slots)
+    for xx in (x, odd_rows(x)):
+        s1 = first.clone()
+        y32, y = torch.empty(T, C, device="cuda"), torch.empty(T, C, dtype=dtype, device="cuda")
+        ops.short_conv_silu(y32, xx, w, bias, s1.clone(), b)
+        ops.short_conv_silu(y, xx, w, None, s1, b)
+        got.append((y32, y, s1))
+    f1, f2, f3 = (torch.empty(T, C, dtype=dtype, device="cuda") for _ in range(3))
+    ops.causal_filter_add(f1, f2, x, w, w2, first.clone(), b)
+    ops.causal_filter_add(f3, None, x, w, None, first.clone(), b)
+    for a, b in zip(*got):
+        assert torch.equal(a, b)                               # the same operations in the same order
+    # filter_add takes whole rows only: against its definition
+    past = torch.zeros(T, C, K - 1, dtype=F64, device="cuda")
+    at = 0
+    for n, start, slot in zip(news, starts, slots):
+        old = (first[slot].view(-1, C)[:K - 1].to(F64) if start > 0 and slot >= 0 and K > 1
+               else torch.zeros(K - 1, C, dtype=F64, device="cuda"))
+        seq = torch.cat([old, x[at:at + n].to(F64)])
+        for j in range(K - 1):
+            past[at:at + n, :, j] = seq[j:j + n]
+        at += n
+    for f, ww in ((f1, w), (f2, w2), (f3, w)):
+        want = x.to(F64) * (1 + ww[:, -1].to(F64)) + (past * ww[:, :-1].to(F64)).sum(-1)
+        torch.testing.assert_close(f.to(F64), want, **tol(dtype, f32=1e-5))
+    assert torch.equal(f1, f3)
