@@ -398,16 +398,17 @@ NHV_API int nhv_mlstm_state_floats(int H, int d, int dv) {
 NHV_API int nhv_mlstm_scan(int dtype, float* y, const void* proj, int proj_stride, const float* gates, int gate_stride,
                            const float* gate_bias, float cap, float* state, long state_stride, const int* cu_q,
                            const int* q_start, const int* slots, int n_seqs, int n_tokens, int H, int d, int dv, int lanes,
-                           float* chunks, cudaStream_t stream) {
+                           float* chunks, int single, cudaStream_t stream) {
   if (n_tokens == 0 || n_seqs == 0) return 0;
   NHV_REQUIRE(H > 0 && d > 0 && dv > 0 && cap > 0.f, "mlstm_scan: bad sizes");
   NHV_REQUIRE(d <= 512, "mlstm_scan: a key head of %d elements is beyond the supported 512", d);
   NHV_REQUIRE(state_stride >= (long)nhv_mlstm_state_floats(H, d, dv), "mlstm_scan: the state holds fewer floats than S, n and m need");
   NHV_REQUIRE(dtype == NHV_F32 || dtype == NHV_BF16, "mlstm_scan: unknown dtype %d", dtype);
-  // as many tokens as requests, of which each brings at least one: single tokens, and the memory is streamed through
+  // every request brings one token (the caller says so): the memory is streamed through
   // (unless a test asks for a form of the scan)
+  NHV_REQUIRE(!single || n_tokens == n_seqs, "mlstm_scan: %d requests of one token each do not have %d tokens", n_seqs, n_tokens);
   const bool st16 = d % 4 == 0 && state_stride % 4 == 0 && ((uintptr_t)state % 16) == 0;
-  if (n_tokens == n_seqs && lanes == 0 && st16) {
+  if (single && lanes == 0 && st16) {
     const int nb = (dv + ML_COLS - 1) / ML_COLS;
     const dim3 grid(n_seqs, H, (nb + 3) / 4);
 #define STEP(T, RG)                                                                                                 \

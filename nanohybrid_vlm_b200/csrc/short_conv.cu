@@ -5,8 +5,8 @@
 // where t counts within the request: inputs before the request's first token are zero, and inputs before this
 // step's portion come from the request's state, which holds its last K - 1 inputs (fp32, [slot][K - 1][C], oldest
 // first).  A first kernel computes all outputs (reading the old state), a second one moves the state on; in a step of
-// single tokens (as many tokens as requests, each of which brings at least one) the first does both, since the thread of
-// a channel then is the only one that reads the channel's state: one launch fewer per layer of a decode step, and no
+// single tokens (the caller says that every request brings exactly one) the first does both, since the thread of a
+// channel then is the only one that reads the channel's state: one launch fewer per layer of a decode step, and no
 // search for a token's request.  A request with q_start == 0 starts from zeros whatever its slot held.  Requests without a slot (slot < 0: the
 // idle entries that pad a captured batch) read zeros and write nothing.
 #include "nhv_common.cuh"
@@ -325,13 +325,13 @@ static bool sv_takes(int n_tokens, int C, int K, const void* y1, const void* y2,
 // [slots][(K - 1) * C] fp32 is read and then moved on.
 NHV_API int nhv_causal_filter_add(int dtype, void* y1, void* y2, int y_stride, const void* x, int x_stride, const void* w1,
                                   const void* w2, float* state, long state_stride, const int* cu_q, const int* q_start,
-                                  const int* slots, int n_seqs, int n_tokens, int C, int K, cudaStream_t stream) {
+                                  const int* slots, int n_seqs, int n_tokens, int C, int K, int single, cudaStream_t stream) {
   if (n_tokens == 0 || n_seqs == 0) return 0;
   NHV_REQUIRE(C > 0 && K >= 1 && K <= SC_MAX_TAPS, "causal_filter: %d taps are beyond the supported %d", K, SC_MAX_TAPS);
   NHV_REQUIRE(K == 1 || (state && state_stride >= (long)(K - 1) * C), "causal_filter: the state holds fewer than (taps - 1) * channels floats");
   NHV_REQUIRE(y1 && w1 && (!y2) == (!w2), "causal_filter: a second output comes with a second filter");
+  NHV_REQUIRE(!single || n_tokens == n_seqs, "causal_filter: %d requests of one token each do not have %d tokens", n_seqs, n_tokens);
   const int threads = 128;
-  const bool single = n_tokens == n_seqs;
   const int tokens_per_block = single || n_tokens <= 512 ? 1 : SC_TOKENS;
   dim3 grid((n_tokens + tokens_per_block - 1) / tokens_per_block, (C + threads - 1) / threads);
   dim3 grid2(n_seqs, (C + threads - 1) / threads);
@@ -364,13 +364,13 @@ NHV_API int nhv_causal_filter_add(int dtype, void* y1, void* y2, int y_stride, c
 NHV_API int nhv_short_conv_silu(int dtype, int out_dtype, void* y, int y_stride, const void* x, int x_stride, const void* w,
                                 const void* bias, float* state, long state_stride, const int* cu_q,
                                 const int* q_start, const int* slots, int n_seqs, int n_tokens, int C, int K,
-                                cudaStream_t stream) {
+                                int single, cudaStream_t stream) {
   if (n_tokens == 0 || n_seqs == 0) return 0;
   NHV_REQUIRE(out_dtype == dtype || out_dtype == NHV_F32, "short_conv: the output is of the input's type or fp32");
   NHV_REQUIRE(C > 0 && K >= 1 && K <= SC_MAX_TAPS, "short_conv: %d taps are beyond the supported %d", K, SC_MAX_TAPS);
+  NHV_REQUIRE(!single || n_tokens == n_seqs, "short_conv: %d requests of one token each do not have %d tokens", n_seqs, n_tokens);
   NHV_REQUIRE(K == 1 || (state && state_stride >= (long)(K - 1) * C), "short_conv: the state holds fewer than (taps - 1) * channels floats");
   const int threads = 128;
-  const bool single = n_tokens == n_seqs;
   const int tokens_per_block = single || n_tokens <= 512 ? 1 : SC_TOKENS;
   dim3 grid((n_tokens + tokens_per_block - 1) / tokens_per_block, (C + threads - 1) / threads);
   dim3 grid2(n_seqs, (C + threads - 1) / threads);

@@ -39,7 +39,7 @@ _SIGNATURES = {
     "nhv_embed_scaled_f32": [I, P, P, P, I, I, I, F, P],
     "nhv_rmsnorm_stream": [I, P, P, P, P, F, F, F, P, P, P, I, I, F, I, F, I, P],
     "nhv_scaled_sum": [I, P, P, P, F, F, c_size_t, P],
-    "nhv_short_conv_silu": [I, I, P, I, P, I, P, P, P, ctypes.c_long, P, P, P, I, I, I, I, P],
+    "nhv_short_conv_silu": [I, I, P, I, P, I, P, P, P, ctypes.c_long, P, P, P, I, I, I, I, I, P],
     "nhv_delta_rule": [I, P, P, I, P, P, P, P, ctypes.c_long, P, P, P, P, P, P, P, P, P, I, I, I, I, I, I, I, I, P, I, P, P],
     "nhv_chunk_scan_floats": [],
     "nhv_ssd_scan": [I, P, P, I, P, I, P, P, P, P, ctypes.c_long, P, P, P, I, I, I, I, I, I, I, I, P, P],
@@ -51,7 +51,7 @@ _SIGNATURES = {
     "nhv_sigmoid_mul": [I, P, I, P, I, P, I, I, I, P],
     "nhv_add_row_bias": [I, P, P, I, I, P],
     "nhv_clamped_glu": [I, P, P, I, I, F, F, P],
-    "nhv_mlstm_scan": [I, P, P, I, P, I, P, F, P, ctypes.c_long, P, P, P, I, I, I, I, I, I, P, P],
+    "nhv_mlstm_scan": [I, P, P, I, P, I, P, F, P, ctypes.c_long, P, P, P, I, I, I, I, I, I, P, I, P],
     "nhv_mlstm_chunk_floats": [I, I, I, I],
     "nhv_moe_route": [P, P, P, I, P, I, I, I, I, I, I, I, I, F, P],
     "nhv_moe_align": [P, I, I, I, P, P, P, P],
@@ -61,7 +61,7 @@ _SIGNATURES = {
     "nhv_moe_gemm_tcgen05": [I, P, P, P, P, I, P, P, I, I, I, F, F, F, P, P],
     "nhv_moe_combine": [I, P, P, P, P, P, I, P, P, P, I, I, I, I, P],
     "nhv_attention_simt_ex": [I, P, I, P, I, P, P, I, P, P, I, I, I, I, I, I, I, I, I, I, I, F, P, P, I, I, F, P],
-    "nhv_causal_filter_add": [I, P, P, I, P, I, P, P, P, ctypes.c_long, P, P, P, I, I, I, I, P],
+    "nhv_causal_filter_add": [I, P, P, I, P, I, P, P, P, ctypes.c_long, P, P, P, I, I, I, I, I, P],
     "nhv_latent_rope_store": [I, P, I, P, I, P, I, P, P, P, P, I, I, I, I, I, I, I, I, I, I, F, P, I, P],
     "nhv_gemm_nt_simt_batched": [I, P, P, P, I, I, I, I, I, I, I, I, ctypes.c_long, ctypes.c_long, ctypes.c_long, P],
     "nhv_general_delta": [I, P, P, I, P, I, P, P, P, P, ctypes.c_long, P, P, P, P, P, P, I, I, I, I, F, P],

@@ -194,6 +194,12 @@ def scaled_sum(out, a, b, ca: float, cb: float) -> None:
          stream_ptr())
 
 
+def _single_tokens(batch) -> int:
+    """1 if every request of the step brings exactly one token (counted on the host; a step that does not say goes the
+    general way)."""
+    return int(getattr(batch, "n_decode_seqs", -1) == batch.n_seqs == batch.n_tokens)
+
+
 def short_conv_silu(out, x, weight, bias, state, batch) -> None:
     """out [T, C] = silu(causal convolution over time of x [T, C] (a view with unit column stride) with weight [C, K]
     (+ bias)); ``state`` [slots, (K - 1) * C] float32 holds each request's last K - 1 inputs and is moved on.  ``out`` is
@@ -206,7 +212,7 @@ def short_conv_silu(out, x, weight, bias, state, batch) -> None:
     assert state.dim() == 2 and state.stride(1) == 1 and (bias is None or (bias.dtype == x.dtype and bias.numel() == C))
     call("nhv_short_conv_silu", dtype_code(x), dtype_code(out), out.data_ptr(), out.stride(0), x.data_ptr(), x.stride(0), weight.data_ptr(),
          _ptr(bias), state.data_ptr(), state.stride(0), batch.cu_q.data_ptr(), batch.q_start.data_ptr(),
-         batch.state_slots.data_ptr(), batch.n_seqs, x.shape[0], C, K, stream_ptr())
+         batch.state_slots.data_ptr(), batch.n_seqs, x.shape[0], C, K, _single_tokens(batch), stream_ptr())
 
 
 SCAN_COLUMNS = 0    # columns of a scan's state per lane: 0 is the kernel's choice; tests set 1, 2, 4
@@ -354,7 +360,7 @@ def causal_filter_add(out1, out2, x, w1, w2, state, batch) -> None:
     assert K == 1 or (state.dtype == torch.float32 and state.dim() == 2 and state.stride(1) == 1)
     call("nhv_causal_filter_add", dtype_code(x), out1.data_ptr(), _ptr(out2), C, x.data_ptr(), C, w1.data_ptr(), _ptr(w2),
          _ptr(state) if K > 1 else None, state.stride(0) if K > 1 else 0, batch.cu_q.data_ptr(), batch.q_start.data_ptr(),
-         batch.state_slots.data_ptr(), batch.n_seqs, x.shape[0], C, K, stream_ptr())
+         batch.state_slots.data_ptr(), batch.n_seqs, x.shape[0], C, K, _single_tokens(batch), stream_ptr())
 
 
 def latent_rope_store(kv, q, q_lat, pages, slot_mapping, positions, cos_sin, rotary_dim: int, H: int, dn: int, dr: int,
@@ -697,7 +703,7 @@ def mlstm_scan(y, proj, gates, gate_bias, cap: float, state, batch, H: int, d: i
         chunks = torch.empty(floats, dtype=torch.float32, device=proj.device) if floats else None
     call("nhv_mlstm_scan", dtype_code(proj), y.data_ptr(), proj.data_ptr(), proj.stride(0), gates.data_ptr(), gates.stride(0),
          gate_bias.data_ptr(), float(cap), state.data_ptr(), state.stride(0), batch.cu_q.data_ptr(), batch.q_start.data_ptr(),
-         batch.state_slots.data_ptr(), batch.n_seqs, T, H, d, dv, MLSTM_LANES, _ptr(chunks), stream_ptr())
+         batch.state_slots.data_ptr(), batch.n_seqs, T, H, d, dv, MLSTM_LANES, _ptr(chunks), _single_tokens(batch), stream_ptr())
 
 
 def moe_route(ids, weights, logits, correction, n_outputs: int, n_groups: int, keep: int, scores: str = "softmax",

@@ -63,3 +63,31 @@ def test_filters_on_single_tokens(ops, dtype, C, K):
     whole, want = run([T])
     for a, b in zip(single + (kept if K > 1 else []), whole + (want if K > 1 else [])):
         assert torch.equal(a, b)
+
+
+def test_as_many_tokens_as_requests_need_not_be_single_tokens(ops):
+    """Two tokens, none and one: three tokens of three requests, but no step of single tokens."""
+    g = torch.Generator().manual_seed(1)
+    C, K, H, d, dv = 64, 4, 2, 16, 16
+    x = dev(torch.randn(3, C, generator=g))
+    w = dev(torch.randn(C, K, generator=g))
+    proj, gates = dev(torch.randn(3, 2 * H * d + H * dv, generator=g)), dev(torch.randn(3, 2 * H, generator=g))
+    bias = dev(torch.randn(2 * H, generator=g))
+    floats = ops.mlstm_state_floats(H, d, dv)
+
+    def run(steps):
+        conv, mem = torch.zeros(3, (K - 1) * C, device="cuda"), torch.zeros(3, floats, device="cuda")
+        outs = []
+        for rows, news, starts, slots in steps:
+            b = step_batch(news, starts, slots)
+            y, f = (torch.empty(len(rows), C, device="cuda") for _ in range(2))
+            o = torch.empty(len(rows), H * dv, device="cuda")
+            ops.causal_filter_add(f, None, x[rows].contiguous(), w, None, conv.clone(), b)
+            ops.short_conv_silu(y, x[rows].contiguous(), w, None, conv, b)
+            ops.mlstm_scan(o, proj[rows].contiguous(), gates[rows].contiguous(), bias, 15.0, mem, b, H, d, dv)
+            outs.append(torch.cat([y, f, o], 1))
+        return torch.cat(outs), conv, mem
+
+    for a, b in zip(run([([0, 1, 2], [2, 0, 1], [0, 5, 0], [0, 1, 2])]),
+                    run([([0, 1], [2], [0], [0]), ([2], [1], [0], [2])])):
+        torch.testing.assert_close(a, b, rtol=1e-5, atol=1e-6)
