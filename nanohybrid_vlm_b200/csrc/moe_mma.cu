@@ -45,7 +45,8 @@ __device__ __forceinline__ float mm_round(float v) { return __bfloat162float(__f
 
 // Tiles of 16 rows only stream the weights: what counts is how many bytes are on their way.  Their grid is about two
 // blocks an SM (16 experts, 16 panels), so a block keeps four stages of 64 columns, 64 KB, in flight (two stages of 32
-// columns left the 134 MB of 16 experts' gate and up at 40 us and the 67 MB of down at 22, half the memory's rate).
+// columns left the 134 MB of 16 experts' gate and up at 40 us and the 67 MB of down at 22, half the memory's rate; now
+// 25 and 15).
 template <int BM> struct MmShape {
   static constexpr int BK = BM >= 64 ? 32 : 64;        // columns of K per stage
   static constexpr int LDS = BK + 8;                   // a row of a stage in shared memory, padded against bank conflicts
