@@ -81,6 +81,9 @@ struct alignas(64) Params {
   int next_bytes, next_blocks;
 };
 
+// UNITS: with the units of `unit`; a kernel of its own, since their code made the others' steps slower (the 8B-shaped decode
+// step of 8 requests 702 -> 712 us with one kernel for all).
+template <bool UNITS>
 __global__ void __launch_bounds__(THREADS, 1) gemm_slab_kernel(const __grid_constant__ Params p) {
   extern __shared__ unsigned char smem_unaligned[];
   unsigned char* smem = smem_unaligned + ((1024 - (smem_u32(smem_unaligned) & 1023)) & 1023);
@@ -229,11 +232,11 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_slab_kernel(const __grid_cons
         float v = value(r);
         if (p.mode == 2) {
           const float up = value(h + r);                           // the rows of up follow the rows of gate
-          v = (p.unit == 1 ? gelu_tanh(v) : v / (1.0f + expf(-v))) * up;
-        } else if (p.unit == 2) {
+          v = (UNITS && p.unit == 1 ? gelu_tanh(v) : v / (1.0f + expf(-v))) * up;
+        } else if (UNITS && p.unit == 2) {
           const float r = fmaxf(v, 0.f);
           v = r * r;
-        } else if (p.unit == 3) {
+        } else if (UNITS && p.unit == 3) {
           v = gelu_tanh(v);
         }
         if (p.mode == 1)
@@ -334,11 +337,14 @@ static int gemm_slab_launch(void* y, const void* x, const void* slabs, int M, in
               "gemm_slab: cannot encode the tensor map of x [%d, %d]", M, K);
   constexpr size_t smem = 1024 + (size_t)STAGES * STAGE_BYTES + (size_t)CONSUMER_WARPS * ROWS * X_ROWS * 4 + 2 * STAGES * 8;
   static_assert(smem <= 227 * 1024, "the ring and the reduction buffer must fit one block's shared memory");
-  static bool attr_set = false;
-  if (!attr_set) {
-    NHV_CUDA(cudaFuncSetAttribute(gemm_slab_kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "gemm_slab");
-    attr_set = true;
-  }
-  NHV_CUDA(nhv_launch(gemm_slab_kernel, dim3(blocks), dim3(THREADS), smem, stream, p), "gemm_slab");
-  return 0;
+  auto go = [&](auto kernel, bool& attr_set) -> int {
+    if (!attr_set) {
+      NHV_CUDA(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem), "gemm_slab");
+      attr_set = true;
+    }
+    NHV_CUDA(nhv_launch(kernel, dim3(blocks), dim3(THREADS), smem, stream, p), "gemm_slab");
+    return 0;
+  };
+  static bool plain_set = false, units_set = false;
+  return unit ? go(gemm_slab_kernel<true>, units_set) : go(gemm_slab_kernel<false>, plain_set);
 }
