@@ -211,7 +211,8 @@ __global__ void __launch_bounds__(ML_COLS * ML_PARTS) mlstm_scan_kernel(
 // anything: 74 us for 48 requests of 8 heads of 128 x 256 (50 MB read, 50 MB written), 38 here.  A warp takes the ML_COLS
 // columns that share a copy of n, its lanes four neighbouring rows each (RG groups of them for larger heads), with all of
 // a pass's columns on their way before the first is needed, and no barrier at all.  d in steps of 4 up to 128 RG, state
-// rows 16-byte aligned.
+// rows 16-byte aligned.  Sums over rows in another order than the scan's: a caller whose results may not depend on how
+// tokens were cut into steps does not say that they are single ones.
 template <typename T, int RG>
 __global__ void __launch_bounds__(128) mlstm_step_kernel(
     float* __restrict__ y, const T* __restrict__ proj, int proj_stride, const float* __restrict__ gates, int gate_stride,

@@ -687,7 +687,8 @@ def mlstm_state_floats(H: int, d: int, dv: int) -> int:
 
 
 def mlstm_scan(y, proj, gates, gate_bias, cap: float, state, batch, H: int, d: int, dv: int, fixed_order: bool = False) -> None:
-    """The mLSTM recurrence over the step's tokens (``fixed_order`` as in ``delta_rule``).  proj [T, >= 2*H*d + H*dv] (q, k, v per head; a view with unit
+    """The mLSTM recurrence over the step's tokens (``fixed_order`` as in ``delta_rule``: steps of single tokens take the
+    scan too then, whose sums over a column's rows have another order than the kernel for single tokens').  proj [T, >= 2*H*d + H*dv] (q, k, v per head; a view with unit
     column stride), gates [T, 2*H] float32 (input then forget gates, before bias and cap), gate_bias [2*H] float32,
     state [slots, mlstm_state_floats] float32 -> y [T, H*dv] float32 (before its norm and gate)."""
     _need_cuda(y, proj, gates, gate_bias, state)
@@ -703,7 +704,8 @@ def mlstm_scan(y, proj, gates, gate_bias, cap: float, state, batch, H: int, d: i
         chunks = torch.empty(floats, dtype=torch.float32, device=proj.device) if floats else None
     call("nhv_mlstm_scan", dtype_code(proj), y.data_ptr(), proj.data_ptr(), proj.stride(0), gates.data_ptr(), gates.stride(0),
          gate_bias.data_ptr(), float(cap), state.data_ptr(), state.stride(0), batch.cu_q.data_ptr(), batch.q_start.data_ptr(),
-         batch.state_slots.data_ptr(), batch.n_seqs, T, H, d, dv, MLSTM_LANES, _ptr(chunks), _single_tokens(batch), stream_ptr())
+         batch.state_slots.data_ptr(), batch.n_seqs, T, H, d, dv, MLSTM_LANES, _ptr(chunks),
+         0 if fixed_order else _single_tokens(batch), stream_ptr())
 
 
 def moe_route(ids, weights, logits, correction, n_outputs: int, n_groups: int, keep: int, scores: str = "softmax",

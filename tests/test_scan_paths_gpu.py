@@ -82,6 +82,31 @@ def test_mlstm_single_tokens(ops, dtype, H, d, dv, spread):
     check_mlstm(ops, dtype, H, d, dv, spread, lengths, [[1, 2, 3, 5, 6, 7, 8], [1, 2, 3, 4, 5, 6], [1, 2]])
 
 
+@pytest.mark.parametrize("pad", [0, 4])
+@pytest.mark.parametrize("H,d,dv,spread", [(2, 128, 256, 4.0), (4, 100, 36, 1.0), (4, 64, 64, 8.0), (4, 512, 20, 2.0), (1, 132, 16, 2.0)])
+def test_mlstm_in_a_fixed_order_has_the_same_bits_for_every_cutting(ops, H, d, dv, spread, pad):
+    """Whole prompts, single tokens side by side, single tokens beside a portion; slots as the engine makes them, and slots
+    that all start on 16 bytes."""
+    g = torch.Generator().manual_seed(d)
+    lengths = [70, 41, 9]
+    ins = [mlstm_inputs(g, n, H, d, dv, torch.float32, spread) for n in lengths]
+    bias = dev(torch.cat((torch.randn(H, generator=g), 2 + torch.randn(H, generator=g))))
+    floats = ops.mlstm_state_floats(H, d, dv)
+    seen = []
+    for cuts in ([[], [], []], [list(range(1, n)) for n in lengths], [[1, 2, 40, 41, 42], [1, 2, 3, 4, 40], [1, 2, 3, 4]]):
+        state = torch.full((4, -(-floats // 4) * 4 if pad else floats), float("nan"), device="cuda")
+
+        def step(o, parts, batch):
+            ops.mlstm_scan(o, rows(parts, [i[0] for i in ins]), rows(parts, [i[1] for i in ins]), bias, 15.0, state, batch,
+                           H, d, dv, fixed_order=True)
+
+        got = walk(step, H * dv, state, lengths, cuts)
+        seen.append(got + [state[SLOTS[r], :floats].cpu() for r in range(3)])
+    for other in seen[1:]:
+        for a, b in zip(seen[0], other):
+            assert torch.equal(a, b)
+
+
 # ---------------------------------------------------------------- prompts, 32 tokens at a time
 LENGTHS = [200, 129, 64, 70]
 # per step: 65, 64, 31, 1 tokens; then 1, 1, 33, 68; then 133, 64, -, 1; then a single token
