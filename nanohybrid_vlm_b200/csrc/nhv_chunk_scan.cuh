@@ -139,15 +139,16 @@ static __device__ __forceinline__ void cs_rows_by_cols(float out[4][4], const fl
     }
 }
 
-// The same for 4 rows of [32][CS_PS] and 16 columns per warp: row lane >> 3, columns (lane & 7) + 8 j, j < 2; only the
-// first 4 * k4 of a row (the rest of a triangle's row is zero).
-static __device__ __forceinline__ void cs_triangle(float out[2], const float* rows, const float* cols, int k4) {
-  const int lane = threadIdx.x & 31;
-  const float* rp = rows + (lane >> 3) * CS_PS;
+// The same for 4 rows of a triangle [32][CS_PS] and 16 columns per warp (warp w: rows 4 w to 4 w + 3): row lane >> 3,
+// columns (lane & 7) + 8 j, j < 2.  Row t takes tokens up to t and no others: a later token's value that is no number would
+// come through the triangle's zeros.
+static __device__ __forceinline__ void cs_triangle(float out[2], const float* rows, const float* cols, int warp) {
+  const int lane = threadIdx.x & 31, row = lane >> 3;
+  const float* rp = rows + (4 * warp + row) * CS_PS;
   const float* cp = cols + (lane & 7) * CS_PS;
   f32x2 acc[2][2] = {{0ull, 0ull}, {0ull, 0ull}};
 #pragma unroll 4
-  for (int k = 0; k < k4; ++k) {
+  for (int k = 0; k < warp; ++k) {
     const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(rp + 4 * k);
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
@@ -155,6 +156,13 @@ static __device__ __forceinline__ void cs_triangle(float out[2], const float* ro
       acc[j][0] = f2_fma(a.x, b.x, acc[j][0]);
       acc[j][1] = f2_fma(a.y, b.y, acc[j][1]);
     }
+  }
+  const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(rp + 4 * warp);
+#pragma unroll
+  for (int j = 0; j < 2; ++j) {
+    const float4 b = *reinterpret_cast<const float4*>(cp + 8 * j * CS_PS + 4 * warp);
+    acc[j][0] = f2_fma(a.x, f2_pack(b.x, row >= 1 ? b.y : 0.f), acc[j][0]);
+    acc[j][1] = f2_fma(a.y, f2_pack(row >= 2 ? b.z : 0.f, row >= 3 ? b.w : 0.f), acc[j][1]);
   }
 #pragma unroll
   for (int j = 0; j < 2; ++j) out[j] = f2_sum(acc[j][0], acc[j][1]);
@@ -256,7 +264,7 @@ __global__ void __launch_bounds__(CS_THREADS) chunk_pairs_kernel(const CsPairs p
 #pragma unroll
           for (int i = 0; i < t; ++i) sum[i & 3] = fmaf(-As[t * CS_PS + i], x[i], sum[i & 3]);
           x[t] = (sum[0] + sum[1]) + (sum[2] + sum[3]);
-          out[CS_T + t * CS_C + tid] = x[t] * ws[tid];
+          out[CS_T + t * CS_C + tid] = t >= tid ? x[t] * ws[tid] : 0.f;   // (0 times a beta that is no number is none)
         }
       }
     }
@@ -444,7 +452,7 @@ __global__ void __launch_bounds__(CS_THREADS, 2) chunk_scan_kernel(const CsScan 
     const float* U = Rs;
     if (DELTA) {
       float u[2] = {0.f, 0.f};
-      if (warp * 4 < cn) cs_triangle(u, Ts + warp * 4 * CS_PS, Rs, warp + 1);
+      if (warp * 4 < cn) cs_triangle(u, Ts, Rs, warp);
 #pragma unroll
       for (int j = 0; j < 2; ++j) Us[((lane & 7) + 8 * j) * CS_PS + warp * 4 + (lane >> 3)] = u[j];
       U = Us;
@@ -452,7 +460,7 @@ __global__ void __launch_bounds__(CS_THREADS, 2) chunk_scan_kernel(const CsScan 
     }
     if (warp * 4 < cn) {
       float o[2];
-      cs_triangle(o, Ps + warp * 4 * CS_PS, U, warp + 1);
+      cs_triangle(o, Ps, U, warp);
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
         const int t = warp * 4 + (lane >> 3), col = (lane & 7) + 8 * j;

@@ -163,3 +163,57 @@ def test_ssd_scan_by_chunks(ops, chunks, H, P, N, G):
 @pytest.mark.parametrize("H,d,dv,spread", [(2, 128, 256, 4.0), (3, 64, 20, 8.0), (1, 100, 36, 1.0), (2, 8, 16, 3.0)])
 def test_mlstm_by_chunks(ops, chunks, dtype, H, d, dv, spread):
     check_mlstm(ops, dtype, H, d, dv, spread, LENGTHS, CUTS)
+
+
+def scans(ops, kind, H, d, dv, T, g):
+    """One request of T tokens through one of the three scans: (its inputs, a function of them and of whether the sums are to
+    be in a fixed order, the plain recurrence in 64 bits, the places of q, k and v in a row of the first input)."""
+    if kind == "delta":
+        qkv, ba, a_log, dt_bias = delta_inputs(g, T, H, H, d, dv, torch.float32)
+
+        def run(ins, fixed):
+            o, state = torch.empty(T, H * dv, device="cuda"), torch.zeros(1, H * d * dv, device="cuda")
+            ops.delta_rule(o, dev(ins[0]), dev(ins[1]), dev(a_log), dev(dt_bias), state, step_batch([T], [0], [0]), H, H, d, dv,
+                           fixed_order=fixed)
+            return o.cpu()
+        return (qkv, ba), run, lambda ins: plain_delta(*ins, a_log, dt_bias, H, H, d, dv), (0, H * d, 2 * H * d)
+    if kind == "ssd":
+        dt_bias, a_log, skip = torch.randn(H, generator=g) * 0.5, torch.rand(H, generator=g) * 1.5 - 1.0, torch.ones(H)
+        xbc, dt = torch.randn(T, H * dv + 2 * d, generator=g), torch.randn(T, H, generator=g)
+
+        def run(ins, fixed):
+            y, state = torch.empty(T, H * dv, device="cuda"), torch.zeros(1, H * d * dv, device="cuda")
+            ops.ssd_scan(y, dev(ins[0]), dev(ins[1]), dev(dt_bias), dev(a_log), dev(skip), state, step_batch([T], [0], [0]),
+                         H, dv, d, 1, fixed_order=fixed)
+            return y.cpu()
+        return (xbc, dt), run, lambda ins: plain_ssd(*ins, dt_bias, a_log, skip, H, dv, d, 1), (H * dv + d, H * dv, 0)
+    proj, gates = mlstm_inputs(g, T, H, d, dv, torch.float32, 4.0)
+    proj = proj[:, :-3].contiguous()
+    bias = torch.cat((torch.randn(H, generator=g), 2 + torch.randn(H, generator=g)))
+
+    def run(ins, fixed):
+        o, state = torch.empty(T, H * dv, device="cuda"), torch.zeros(1, ops.mlstm_state_floats(H, d, dv), device="cuda")
+        ops.mlstm_scan(o, dev(ins[0]), dev(ins[1]), dev(bias), 15.0, state, step_batch([T], [0], [0]), H, d, dv, fixed_order=fixed)
+        return o.cpu()
+    return (proj, gates), run, lambda ins: plain_scan(*ins, bias, 15.0, H, d, dv), (0, H * d, 2 * H * d)
+
+
+@pytest.mark.parametrize("kind", ["delta", "ssd", "mlstm"])
+@pytest.mark.parametrize("bad", [float("nan"), float("inf")])
+def test_a_value_that_is_no_number_stays_with_its_token_and_later_ones(ops, chunks, kind, bad):
+    """At every place of a group of four tokens, in q, k, v and the gates: what comes before keeps its bits, and a bad value
+    of v keeps to its column."""
+    H, d, dv, T = 2, 64, 20, 70
+    ins, run, _, (q, k, v) = scans(ops, kind, H, d, dv, T, torch.Generator().manual_seed(3))
+    clean = run(ins, False)
+    assert torch.isfinite(clean).all()
+    for token in (1, 34, 47, 68):
+        for which, col in ((0, q), (0, k), (0, v), (1, 0), (1, ins[1].shape[1] - 1)):
+            broken = [t.clone() for t in ins]
+            broken[which][token, col] = bad
+            got = run(broken, False)
+            assert torch.equal(got[:token], clean[:token]), (token, which, col)
+            if which == 0 and col == v:
+                assert not torch.isfinite(got[token, 0]) and torch.equal(got[:, 1:], clean[:, 1:])
+            if which == 0 and col == q:
+                assert torch.equal(got[token + 1:], clean[token + 1:])
