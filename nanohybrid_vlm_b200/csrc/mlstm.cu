@@ -345,7 +345,7 @@ __global__ void __launch_bounds__(MG_TOKENS) mlstm_gates_kernel(
     if (there) {
       const float before = last[tid];
       const size_t at = (size_t)(first + c0 + tid) * H + h;
-      a[at] = expf(f + before - m);
+      a[at] = expf((float)((double)f + (double)before - (double)m));     // the maxima as they were rounded: no error of theirs is left
       b[at] = expf(i - m);
       em[at] = expf(-m);
       top[at] = m;

@@ -9,8 +9,10 @@
 //   u_t = beta_t (v_t - gam_t (s0^T k_t) - sum_{i < t} D(i, t) (k_i . k_t) u_i):   U = T' (V - diag(gam) K s0)
 // with T' = (I + A)^-1 diag(beta), A(t, i) = beta_t D(i, t) (k_t . k_i) below the diagonal.  Token by token a recurrence
 // is a chain of n rounds of sums over lanes and a write (delta rule, 16 heads of 128 x 128, one request of 4,096 tokens:
-// 1,042 us); chunk by chunk the chain is n / 32 rounds of small matrix products.  All products, sums and decays are fp32
-// on the CUDA cores (fused multiply-add, two at a time); decays between tokens are running products, never quotients.
+// 1,042 us); chunk by chunk the chain is n / 32 rounds of small matrix products.  Those are fp32 on the CUDA cores (fused
+// multiply-add, two at a time).  What every chunk is made from, the products q . k and k . k and the decays between
+// tokens (running products, never quotients), is summed and multiplied in 64 bits and rounded once to fp32, so that the error
+// against 64 bits is no larger than token by token.
 //
 // Two kernels.  The first has a block per (chunk, q/k head) and no chain: the products q . k and k . k, the decays, the
 // inverse.  It leaves per (chunk, head) CS_WORK floats.  The second has a block per (request, head, 16 columns of S) and
@@ -27,8 +29,9 @@ constexpr int CS_C = 32;                                  // tokens of a chunk
 constexpr int CS_COLS = 16;                               // columns of S per block
 constexpr int CS_THREADS = 256;
 constexpr int CS_PS = CS_C + 4;                           // floats of a row of P, T', V, U in shared memory
-// per (chunk, head): P, T' [32][32], gam, E [32]
-constexpr int CS_P = 0, CS_T = CS_C * CS_C, CS_GAM = 2 * CS_C * CS_C, CS_E = CS_GAM + CS_C, CS_WORK = CS_E + CS_C;
+// per (chunk, head): P, T' below their diagonals [32][32]; gam, E, the diagonals of P and of T' [32]
+constexpr int CS_P = 0, CS_T = CS_C * CS_C, CS_GAM = 2 * CS_C * CS_C, CS_E = CS_GAM + CS_C, CS_PD = CS_E + CS_C,
+              CS_TD = CS_PD + CS_C, CS_VECS = 4, CS_WORK = CS_GAM + CS_VECS * CS_C;
 
 static inline long cs_chunks(int n_tokens, int n_seqs) { return (long)n_tokens / CS_C + n_seqs; }
 
@@ -65,40 +68,35 @@ static __device__ __forceinline__ bool cs_find(int number, const int* cu_q, int 
   return c >= 0 && c * CS_C < n;
 }
 
-// Products of rows of two tiles [32][D + 4] in shared memory: out[r][c] = a_r . b_c for the 8 NC columns from c0 on, by 64
-// threads (`tid` 0..63) of 4 x NC each: rows (tid >> 3) + 8 i, columns c0 + (tid & 7) + 8 j.
-template <int D, int NC>
-static __device__ __forceinline__ void cs_products(float* out, const float* a, const float* b, int c0, int tid) {
-  const float* ar = a + (tid >> 3) * (D + 4);
-  const float* br = b + (c0 + (tid & 7)) * (D + 4);
-  f32x2 acc[4][NC];
+// Products of rows of two tiles [32][D + 4] in shared memory, out[t][i] = a_t . b_i for i <= t (and what else lies in the 8 x 8
+// tiles on the diagonal): a warp takes the eight rows from 8 `band` on.  Summed in 64 bits, on the matrix instruction for
+// them, and rounded once: every output of a chunk is made from these products, and with 32-bit sums (two chains of D / 2)
+// theirs was most of the error of a scan by chunks (state space 1.68e-7 in all, 1.06e-7 by tokens).
+template <int D>
+static __device__ __forceinline__ void cs_products(float* out, const float* a, const float* b, int band) {
+  const int lane = threadIdx.x & 31;
+  const float* ar = a + (8 * band + (lane >> 2)) * (D + 4) + (lane & 3);       // element (lane >> 2, lane & 3) of an 8 x 4 tile
+  const float* br = b + (lane >> 2) * (D + 4) + (lane & 3);
+  double acc[4][2];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < NC; ++j) acc[i][j] = 0ull;
-#pragma unroll 2
+  for (int j = 0; j < 4; ++j) acc[j][0] = acc[j][1] = 0.0;
+#pragma unroll 4
   for (int k = 0; k < D; k += 4) {
-    ulonglong2 bv[NC];
+    const double av = ar[k];
 #pragma unroll
-    for (int j = 0; j < NC; ++j) bv[j] = *reinterpret_cast<const ulonglong2*>(br + 8 * j * (D + 4) + k);
-#pragma unroll
-    for (int i = 0; i < 4; ++i) {
-      const ulonglong2 av = *reinterpret_cast<const ulonglong2*>(ar + 8 * i * (D + 4) + k);
-#pragma unroll
-      for (int j = 0; j < NC; ++j) {
-        acc[i][j] = f2_fma(av.x, bv[j].x, acc[i][j]);
-        acc[i][j] = f2_fma(av.y, bv[j].y, acc[i][j]);
+    for (int j = 0; j < 4; ++j)
+      if (j <= band) {
+        const double bv = br[8 * j * (D + 4) + k];
+        asm("mma.sync.aligned.m8n8k4.row.col.f64.f64.f64.f64 {%0, %1}, {%2}, {%3}, {%0, %1};\n"
+            : "+d"(acc[j][0]), "+d"(acc[j][1])
+            : "d"(av), "d"(bv));
       }
-    }
   }
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
-#pragma unroll
-    for (int j = 0; j < NC; ++j) {
-      float even, odd;
-      f2_unpack(acc[i][j], even, odd);
-      out[((tid >> 3) + 8 * i) * CS_PS + c0 + (tid & 7) + 8 * j] = even + odd;
-    }
+  for (int j = 0; j < 4; ++j)
+    if (j <= band)
+      *reinterpret_cast<float2*>(out + (8 * band + (lane >> 2)) * CS_PS + 8 * j + 2 * (lane & 3)) =
+          make_float2((float)acc[j][0], (float)acc[j][1]);
 }
 
 // Sums of 32 rows times 16 columns over 4 K4 elements (contiguous in both, in shared memory) by a warp: a lane's rows
@@ -139,34 +137,36 @@ static __device__ __forceinline__ void cs_rows_by_cols(float out[4][4], const fl
     }
 }
 
-// The same for 4 rows of a triangle [32][CS_PS] and 16 columns per warp (warp w: rows 4 w to 4 w + 3): row lane >> 3,
-// columns (lane & 7) + 8 j, j < 2.  Row t takes tokens up to t and no others: a later token's value that is no number would
-// come through the triangle's zeros.
-static __device__ __forceinline__ void cs_triangle(float out[2], const float* rows, const float* cols, int warp) {
+// out += the same for 4 rows of a matrix [32][CS_PS] with zeros on and above its diagonal and 16 columns per warp (warp w:
+// rows 4 w to 4 w + 3; row lane >> 3, columns (lane & 7) + 8 j, j < 2), then += diagonal[row] times the row's own token, most
+// of the sum: last, in one rounding.  A value that is no number would reach the rows before its own through the zeros:
+// MASKED leaves out what a row may not see, for chunks that hold such a value (selects in all chunks cost up to 10 % of a scan).
+template <bool MASKED>
+static __device__ __forceinline__ void cs_triangle(float out[2], const float* rows, const float* cols, const float* diagonal,
+                                                   int warp) {
   const int lane = threadIdx.x & 31, row = lane >> 3;
   const float* rp = rows + (4 * warp + row) * CS_PS;
   const float* cp = cols + (lane & 7) * CS_PS;
   f32x2 acc[2][2] = {{0ull, 0ull}, {0ull, 0ull}};
 #pragma unroll 4
-  for (int k = 0; k < warp; ++k) {
+  for (int k = 0; k <= warp; ++k) {
     const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(rp + 4 * k);
 #pragma unroll
     for (int j = 0; j < 2; ++j) {
-      const ulonglong2 b = *reinterpret_cast<const ulonglong2*>(cp + 8 * j * CS_PS + 4 * k);
+      ulonglong2 b = *reinterpret_cast<const ulonglong2*>(cp + 8 * j * CS_PS + 4 * k);
+      if (MASKED && k == warp) {
+        b.x &= row > 1 ? ~0ull : row > 0 ? 0xffffffffull : 0ull;
+        b.y &= row > 2 ? 0xffffffffull : 0ull;
+      }
       acc[j][0] = f2_fma(a.x, b.x, acc[j][0]);
       acc[j][1] = f2_fma(a.y, b.y, acc[j][1]);
     }
   }
-  const ulonglong2 a = *reinterpret_cast<const ulonglong2*>(rp + 4 * warp);
+  const float d = diagonal[4 * warp + row];
 #pragma unroll
-  for (int j = 0; j < 2; ++j) {
-    const float4 b = *reinterpret_cast<const float4*>(cp + 8 * j * CS_PS + 4 * warp);
-    acc[j][0] = f2_fma(a.x, f2_pack(b.x, row >= 1 ? b.y : 0.f), acc[j][0]);
-    acc[j][1] = f2_fma(a.y, f2_pack(row >= 2 ? b.z : 0.f, row >= 3 ? b.w : 0.f), acc[j][1]);
-  }
-#pragma unroll
-  for (int j = 0; j < 2; ++j) out[j] = f2_sum(acc[j][0], acc[j][1]);
+  for (int j = 0; j < 2; ++j) out[j] = fmaf(d, cp[8 * j * CS_PS + 4 * warp + row], out[j] + f2_sum(acc[j][0], acc[j][1]));
 }
+static __device__ __forceinline__ bool cs_no_number(float v) { return !(fabsf(v) < INFINITY); }
 
 // What kind of recurrence the second kernel walks
 enum CsKind { CS_DELTA, CS_PLAIN, CS_NORMED };           // u from T'; u = v; u = v and o divided by its normaliser
@@ -182,7 +182,7 @@ struct CsPairs {
 
 template <int D, int KIND>
 constexpr int cs_pairs_smem_floats() {
-  return 2 * CS_C * (D + 4) + (KIND == CS_DELTA ? 3 : 1) * CS_C * CS_PS + 3 * CS_C;
+  return 2 * CS_C * (D + 4) + (KIND == CS_DELTA ? 3 : 1) * CS_C * CS_PS + 4 * CS_C;
 }
 
 // Gates: decay, weight and what else a kind needs of token t (of the packed step) and head h
@@ -195,8 +195,8 @@ __global__ void __launch_bounds__(CS_THREADS) chunk_pairs_kernel(const CsPairs p
   float* QK = Qs + CS_C * (D + 4);                        // [32][CS_PS]
   float* KK = QK + CS_C * CS_PS;                          // DELTA: the same of k . k, then A
   float* As = KK + (DELTA ? CS_C * CS_PS : 0);
-  float* gs = As + (DELTA ? CS_C * CS_PS : 0);            // decay of the token
-  float* ws = gs + CS_C;                                  // weight of the token (DELTA: beta)
+  double* gd = reinterpret_cast<double*>(As + (DELTA ? CS_C * CS_PS : 0));     // decay of the token
+  float* ws = reinterpret_cast<float*>(gd + CS_C);        // weight of the token (DELTA: beta)
   float* Es = ws + CS_C;
   pdl_wait();                                             // (the scan behind it takes whole SMs: it is let in at the end)
   int s, c, first, n;
@@ -207,9 +207,10 @@ __global__ void __launch_bounds__(CS_THREADS) chunk_pairs_kernel(const CsPairs p
   cs_commit();
   cs_wait<0>();
   __syncthreads();
-  const int team = tid >> 6;
-  if (DELTA) cs_products<D, 2>(team < 2 ? QK : KK, team < 2 ? Qs : Ks, Ks, 16 * (team & 1), tid & 63);
-  else cs_products<D, 1>(QK, Qs, Ks, 8 * team, tid & 63);
+  // (a band of eight rows has one to four tiles: warps that share a quarter of the SM have five between them)
+  const int warp = tid >> 5;
+  if (warp < 4) cs_products<D>(QK, Qs, Ks, warp);
+  else if (DELTA) cs_products<D>(KK, Ks, Ks, 7 - warp);
 
   const int per = p.H / p.G, share = (per + gridDim.z - 1) / gridDim.z;       // heads of the group, of this block
   const int h_end = min((int)(blockIdx.z + 1) * share, per) + g * per;
@@ -220,31 +221,34 @@ __global__ void __launch_bounds__(CS_THREADS) chunk_pairs_kernel(const CsPairs p
     if (tid < CS_C) {
       float gate = 1.f, weight = 0.f, em = 0.f;           // behind the last token: nothing is added, nothing decays
       if (tid < cn) gates(t0 + tid, h, gate, weight, em);
-      gs[tid] = gate;
+      gd[tid] = gate;
       ws[tid] = weight;
       if (NORMED) ex[CS_C + tid] = em;
     }
     __syncthreads();
     {
       const int i = tid & 31, ta = 4 * (tid >> 5);        // a column of the triangle, four of its rows
-      float dec = 1.f;                                    // g_(i+1) .. g_t
-      for (int t = i + 1; t < ta; ++t) dec *= gs[t];
-      const float wi = DELTA ? 1.f : ws[i];
+      // (products of 64 bits, rounded once: where states last, those of 32 bits were most of what was left of the error)
+      double dec = 1.0;                                   // g_(i+1) .. g_t
+      for (int t = i + 1; t < ta; ++t) dec *= gd[t];
+      const double wi = DELTA ? 1.0 : (double)ws[i];
 #pragma unroll
       for (int t = ta; t < ta + 4; ++t) {
-        if (t > i) dec *= gs[t];
-        const float pv = t >= i ? dec * wi * QK[t * CS_PS + i] : 0.f;
-        out[CS_P + t * CS_C + i] = pv;
-        if (DELTA) As[t * CS_PS + i] = t > i ? ws[t] * dec * KK[t * CS_PS + i] : 0.f;
-        if (i == 0) out[CS_GAM + t] = gs[0] * dec;
+        if (t > i) dec *= gd[t];
+        const float pv = t >= i ? (float)(dec * wi * QK[t * CS_PS + i]) : 0.f;
+        out[CS_P + t * CS_C + i] = t > i ? pv : 0.f;
+        if (t == i) out[CS_PD + t] = pv;
+        if (DELTA) As[t * CS_PS + i] = t > i ? (float)(dec * ws[t] * KK[t * CS_PS + i]) : 0.f;
+        if (i == 0) out[CS_GAM + t] = (float)(gd[0] * dec);
         if (NORMED) {
           const float sum = warp_sum(pv);
           if (i == 0) ex[t] = sum;
         }
       }
       if (ta == CS_C - 4) {
-        out[CS_E + i] = dec * wi;
-        if (NORMED) Es[i] = dec * wi;
+        const float e = (float)(dec * wi);
+        out[CS_E + i] = e;
+        if (NORMED) Es[i] = e;
       }
     }
     __syncthreads();
@@ -264,8 +268,9 @@ __global__ void __launch_bounds__(CS_THREADS) chunk_pairs_kernel(const CsPairs p
 #pragma unroll
           for (int i = 0; i < t; ++i) sum[i & 3] = fmaf(-As[t * CS_PS + i], x[i], sum[i & 3]);
           x[t] = (sum[0] + sum[1]) + (sum[2] + sum[3]);
-          out[CS_T + t * CS_C + tid] = t >= tid ? x[t] * ws[tid] : 0.f;   // (0 times a beta that is no number is none)
+          out[CS_T + t * CS_C + tid] = t > tid ? x[t] * ws[tid] : 0.f;
         }
+        out[CS_TD + tid] = ws[tid];                       // the inverse has ones there
       }
     }
   }
@@ -303,7 +308,7 @@ constexpr int CS_PARTIAL = 8 * 32 * 20;                  // rows of 20 floats, 3
 template <int D, int KIND>
 constexpr int cs_smem_floats() {
   return CS_COLS * (D + 4) + 4 * CS_C * (D + 4) + (KIND == CS_DELTA ? 2 : 1) * CS_C * CS_PS + 2 * CS_COLS * CS_PS +
-         2 * 2 * CS_C + CS_PARTIAL + CS_C * 20 + (KIND == CS_NORMED ? D + 2 * (2 * CS_C) + CS_C : 0);
+         2 * CS_VECS * CS_C + CS_PARTIAL + CS_C * 20 + (KIND == CS_NORMED ? D + 2 * (2 * CS_C) + CS_C : 0);
 }
 
 static __device__ __forceinline__ float4 cs_load4(const float* p) { return *reinterpret_cast<const float4*>(p); }
@@ -326,8 +331,8 @@ __global__ void __launch_bounds__(CS_THREADS, 2) chunk_scan_kernel(const CsScan 
   float* Ts = Ps + CS_C * CS_PS;                          // DELTA: [64][CS_PS]
   float* Rs = Ts + (DELTA ? CS_C * CS_PS : 0);            // [16 columns][CS_PS]: V, for DELTA then V - diag(gam) K s0
   float* Us = Rs + CS_COLS * CS_PS;                       // DELTA: [16 columns][CS_PS]
-  float* Vec = Us + CS_COLS * CS_PS;                      // [2 stages][gam, E][32]
-  float* Xs = Vec + 4 * CS_C;                             // partial sums
+  float* Vec = Us + CS_COLS * CS_PS;                      // [2 stages][gam, E, P's diagonal, T' 's][32]
+  float* Xs = Vec + 2 * CS_VECS * CS_C;                   // partial sums
   float* Os = Xs + CS_PARTIAL;       // [32][20]: diag(gam) Q s0
   float* Ns = Os + CS_C * 20;                             // NORMED: [D] n, [2 stages][sum of P's row, exp(-m)][32], [32] the division
   pdl_wait();
@@ -357,7 +362,7 @@ __global__ void __launch_bounds__(CS_THREADS, 2) chunk_scan_kernel(const CsScan 
     const int cn = min(CS_C, n - c * CS_C), stage = c & 1;
     cs_fetch_rows<D>(KQ + (2 * stage) * CS_C * RS, kb + (size_t)c * CS_C * p.qk_stride, p.qk_stride, cn, d);
     cs_fetch_rows<D>(KQ + (2 * stage + 1) * CS_C * RS, qb + (size_t)c * CS_C * p.qk_stride, p.qk_stride, cn, d);
-    if (tid < 2 * CS_C / 4) cs_copy16(Vec + stage * 2 * CS_C + 4 * tid, work_of(c) + CS_GAM + 4 * tid, true);
+    if (tid < (DELTA ? 4 : 3) * CS_C / 4) cs_copy16(Vec + stage * CS_VECS * CS_C + 4 * tid, work_of(c) + CS_GAM + 4 * tid, true);
     if (NORMED && tid < 2 * CS_C / 4)
       cs_copy16(Ns + D + stage * 2 * CS_C + 4 * tid, p.extra + ((number0 + c) * p.H + h) * (2 * CS_C + d) + 4 * tid, true);
   };
@@ -398,14 +403,16 @@ __global__ void __launch_bounds__(CS_THREADS, 2) chunk_scan_kernel(const CsScan 
   for (int c = 0; c < n_chunks; ++c) {
     const int stage = c & 1, cn = min(CS_C, n - c * CS_C);
     const float* Ks = KQ + (2 * stage) * CS_C * RS;
-    const float* gam = Vec + stage * 2 * CS_C;
-    const float* E = gam + CS_C;
+    const float *gam = Vec + stage * CS_VECS * CS_C, *E = gam + CS_C, *Pd = E + CS_C, *Td = Pd + CS_C;
     cs_wait<0>();
+    // whether the chunk holds a value that is no number (DELTA: asked of V - diag(gam) K s0 and of U, below)
+    bool odd = !DELTA && (cs_no_number(v_next.x) || cs_no_number(v_next.y) || cs_no_number(v_next.z) || cs_no_number(v_next.w));
     if (tid < 4 * CS_C) {
       Rs[(vc + 0) * CS_PS + vt] = v_next.x; Rs[(vc + 1) * CS_PS + vt] = v_next.y;
       Rs[(vc + 2) * CS_PS + vt] = v_next.z; Rs[(vc + 3) * CS_PS + vt] = v_next.w;
     }
-    __syncthreads();
+    if (DELTA) __syncthreads();
+    else odd = __syncthreads_or(odd);
     fetch_pt(c);
     cs_commit();
     if (c + 1 < n_chunks) {
@@ -444,27 +451,38 @@ __global__ void __launch_bounds__(CS_THREADS, 2) chunk_scan_kernel(const CsScan 
         float sum = 0.f;
 #pragma unroll
         for (int o = 0; o < SPLIT; ++o) sum += Xs[(o * 32 * GROUPS + r) * 20 + col];
-        if (DELTA && r < CS_C) Rs[col * CS_PS + t] -= gam[t] * sum;
-        else Os[t * 20 + col] = gam[t] * sum;
+        if (DELTA && r < CS_C) {
+          const float v = Rs[col * CS_PS + t] - gam[t] * sum;
+          odd |= cs_no_number(v);
+          Rs[col * CS_PS + t] = v;
+        } else {
+          Os[t * 20 + col] = gam[t] * sum;
+        }
       }
-      __syncthreads();
+      if (DELTA) odd = __syncthreads_or(odd);
+      else __syncthreads();
     }
     const float* U = Rs;
     if (DELTA) {
       float u[2] = {0.f, 0.f};
-      if (warp * 4 < cn) cs_triangle(u, Ts, Rs, warp);
+      if (warp * 4 < cn) {
+        if (odd) cs_triangle<true>(u, Ts, Rs, Td, warp);
+        else cs_triangle<false>(u, Ts, Rs, Td, warp);
+      }
 #pragma unroll
       for (int j = 0; j < 2; ++j) Us[((lane & 7) + 8 * j) * CS_PS + warp * 4 + (lane >> 3)] = u[j];
       U = Us;
-      __syncthreads();
+      odd = __syncthreads_or(cs_no_number(u[0]) || cs_no_number(u[1]));
     }
     if (warp * 4 < cn) {
-      float o[2];
-      cs_triangle(o, Ps, U, warp);
+      const int t = warp * 4 + (lane >> 3);
+      float o[2] = {Os[t * 20 + (lane & 7)], Os[t * 20 + (lane & 7) + 8]};
+      if (odd) cs_triangle<true>(o, Ps, U, Pd, warp);
+      else cs_triangle<false>(o, Ps, U, Pd, warp);
 #pragma unroll
       for (int j = 0; j < 2; ++j) {
-        const int t = warp * 4 + (lane >> 3), col = (lane & 7) + 8 * j;
-        float out = o[j] + Os[t * 20 + col];
+        const int col = (lane & 7) + 8 * j;
+        float out = o[j];
         if (KIND == CS_PLAIN) out = fmaf(skip, U[col * CS_PS + t], out);
         if (NORMED) out /= Ns[D + 4 * CS_C + t];
         if (t < cn && col < ncol) yb[(size_t)(c * CS_C + t) * p.H * dv + col] = out;

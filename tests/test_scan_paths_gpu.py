@@ -165,11 +165,12 @@ def test_mlstm_by_chunks(ops, chunks, dtype, H, d, dv, spread):
     check_mlstm(ops, dtype, H, d, dv, spread, LENGTHS, CUTS)
 
 
-def scans(ops, kind, H, d, dv, T, g):
+def scans(ops, kind, H, d, dv, T, g, slower=0.0):
     """One request of T tokens through one of the three scans: (its inputs, a function of them and of whether the sums are to
     be in a fixed order, the plain recurrence in 64 bits, the places of q, k and v in a row of the first input)."""
     if kind == "delta":
         qkv, ba, a_log, dt_bias = delta_inputs(g, T, H, H, d, dv, torch.float32)
+        a_log -= slower
 
         def run(ins, fixed):
             o, state = torch.empty(T, H * dv, device="cuda"), torch.zeros(1, H * d * dv, device="cuda")
@@ -178,7 +179,7 @@ def scans(ops, kind, H, d, dv, T, g):
             return o.cpu()
         return (qkv, ba), run, lambda ins: plain_delta(*ins, a_log, dt_bias, H, H, d, dv), (0, H * d, 2 * H * d)
     if kind == "ssd":
-        dt_bias, a_log, skip = torch.randn(H, generator=g) * 0.5, torch.rand(H, generator=g) * 1.5 - 1.0, torch.ones(H)
+        dt_bias, a_log, skip = torch.randn(H, generator=g) * 0.5, torch.rand(H, generator=g) * 1.5 - 1.0 - slower, torch.ones(H)
         xbc, dt = torch.randn(T, H * dv + 2 * d, generator=g), torch.randn(T, H, generator=g)
 
         def run(ins, fixed):
@@ -217,3 +218,14 @@ def test_a_value_that_is_no_number_stays_with_its_token_and_later_ones(ops, chun
                 assert not torch.isfinite(got[token, 0]) and torch.equal(got[:, 1:], clean[:, 1:])
             if which == 0 and col == q:
                 assert torch.equal(got[token + 1:], clean[token + 1:])
+
+
+@pytest.mark.parametrize("kind,slower", [("delta", 0.0), ("delta", 4.0), ("ssd", 0.0), ("ssd", 4.0), ("mlstm", 0.0)])
+@pytest.mark.parametrize("H,d,dv", [(4, 128, 128), (4, 64, 64), (8, 16, 32)])
+def test_error_by_chunks_is_no_larger_than_by_tokens(ops, chunks, kind, slower, H, d, dv):
+    """Of 1,024 tokens (``slower``: decays near 1, so that many tokens add up).  The middle one of the tokens' errors: the mLSTM's
+    largest come from a few tokens whose normaliser cancels, and differ by chance."""
+    ins, run, plain, _ = scans(ops, kind, H, d, dv, 1024, torch.Generator().manual_seed(d), slower)
+    want = plain(ins)
+    by_chunks, by_tokens = (((run(ins, fixed).to(F64) - want).norm(dim=-1) / want.norm(dim=-1)).median() for fixed in (False, True))
+    assert by_chunks <= by_tokens, (by_chunks, by_tokens)
