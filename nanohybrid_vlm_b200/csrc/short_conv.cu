@@ -173,8 +173,7 @@ __global__ void filter_add_kernel(T* __restrict__ y1, T* __restrict__ y2, int y_
       fill(t);
     }
     const float xt = to_f32<T>(x[(size_t)t * x_stride + c]);
-    float a = wa[M] * xt, b = wb[M] * xt;               // oldest tap first, the current token last, then the input itself
-    float ra = 0.f, rb = 0.f;
+    float ra = 0.f, rb = 0.f;                           // oldest tap first, the current token last, then the input itself
 #pragma unroll
     for (int m = 0; m < M; ++m) {
       ra = fmaf(wa[m], win[m], ra);
@@ -187,8 +186,8 @@ __global__ void filter_add_kernel(T* __restrict__ y1, T* __restrict__ y2, int y_
 #pragma unroll
       for (int j = 0; j < M; ++j)
         if (j < K - 1) state[(size_t)slots[s] * state_stride + (size_t)j * C + c] = keep(win, j, K);
-    y1[(size_t)t * y_stride + c] = from_f32<T>(xt + (ra + a));
-    if (y2) y2[(size_t)t * y_stride + c] = from_f32<T>(xt + (rb + b));
+    y1[(size_t)t * y_stride + c] = from_f32<T>(xt + fmaf(wa[M], xt, ra));
+    if (y2) y2[(size_t)t * y_stride + c] = from_f32<T>(xt + fmaf(wb[M], xt, rb));
   }
 }
 
@@ -296,8 +295,8 @@ __global__ void __launch_bounds__(128) short_conv_vec_kernel(
             ra = fmaf(wa[m][e], win[m][e], ra);
             rb = fmaf(wb[FILTER ? m : 0][e], win[m][e], rb);
           }
-          o1[e] = xt + (ra + wa[M][e] * xt);
-          o2[e] = xt + (rb + wb[FILTER ? M : 0][e] * xt);
+          o1[e] = xt + fmaf(wa[M][e], xt, ra);
+          o2[e] = xt + fmaf(wb[FILTER ? M : 0][e], xt, rb);
         } else {
           float acc = fmaf(wa[M][e], xt, b[e]);
 #pragma unroll

@@ -4,7 +4,7 @@ import pytest
 import torch
 
 import plain_muvonex as pm
-from test_muvonex_ops_gpu import F64, dev, rotary_table, step_batch, tol
+from test_muvonex_ops_gpu import F64, dev, portions_of, rotary_table, step_batch, tol
 
 pytestmark = pytest.mark.gpu
 
@@ -121,3 +121,26 @@ def test_short_filters_of_long_steps(ops, dtype, C, K):
         want = x.to(F64) * (1 + ww[:, -1].to(F64)) + (past * ww[:, :-1].to(F64)).sum(-1)
         torch.testing.assert_close(f.to(F64), want, **tol(dtype, f32=1e-5))
     assert torch.equal(f1, f3)
+
+
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("C,K,two", [(68, 4, True), (132, 3, False), (516, 2, True), (64, 1, False)])
+def test_filter_add_has_the_same_bits_in_long_and_short_steps(ops, dtype, C, K, two):
+    """The same requests in one step of more than 512 tokens (four channels a thread) and in portions of fewer."""
+    g = torch.Generator().manual_seed(C)
+    lengths = [300, 17, 250]
+    xs = [torch.randn(n, C, generator=g).to(dtype).cuda() for n in lengths]
+    w, w2 = (dev((torch.randn(C, K, generator=g) * 0.5).to(dtype)) for _ in range(2))
+    seen = []
+    for cuts in ([[], [], []], [[1, 150], [1, 16], [1, 120]]):
+        state = torch.full((3, max(K - 1, 1) * C), float("nan"), device="cuda")
+        got = [[] for _ in lengths]
+        for who, starts, news in portions_of(lengths, cuts):
+            x = torch.cat([xs[r][s:s + n] for r, s, n in zip(who, starts, news)])
+            f1, f2 = torch.empty_like(x), torch.empty_like(x)
+            ops.causal_filter_add(f1, f2 if two else None, x, w, w2 if two else None, state, step_batch(news, starts, who))
+            for r, a, b in zip(who, f1.split(news), f2.split(news)):
+                got[r].append(torch.cat([a, b], 1) if two else a)
+        seen.append([torch.cat(p) for p in got] + ([state] if K > 1 else []))
+    for a, b in zip(*seen):
+        assert torch.equal(a, b)
