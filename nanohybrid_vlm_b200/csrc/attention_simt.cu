@@ -472,11 +472,12 @@ NHV_API int nhv_attention_simt_ex(int dtype, const void* q, int q_stride, void* 
       (uintptr_t)kv_pages % four == 0) {
     const int most = AV_PAIRS * AT_WARPS, GS = G < 8 ? G : 8, TQ = most / GS, stages = dtype == NHV_F32 ? 2 : 1;
     const size_t smem = ((size_t)stages * AT_CHUNK * (d + 4 + (planes == 2 ? dv : 0)) + (size_t)most * (d + AT_CHUNK)) * 4;
+    const int most_smem = (stages * AT_CHUNK * (256 + 4 + 256) + most * (256 + AT_CHUNK)) * 4;
     const dim3 grid(n_tokens / TQ + n_seqs, nkv, (G + GS - 1) / GS);
 #define LAUNCH_VEC(T, VC)                                                                                           \
   do {                                                                                                              \
-    NHV_CUDA(cudaFuncSetAttribute(attn_paged_simt_vec_kernel<T, VC>, cudaFuncAttributeMaxDynamicSharedMemorySize,   \
-                                  (int)smem), "attention");                                                         \
+    static std::atomic<uint64_t> done{0};                                                                           \
+    NHV_CUDA(nhv_allow_smem((const void*)attn_paged_simt_vec_kernel<T, VC>, most_smem, done), "attention");         \
     nhv_launch(attn_paged_simt_vec_kernel<T, VC>, grid, AT_WARPS * 32, smem, stream, (const T*)q, q_stride, (T*)out, \
                out_stride, (const T*)kv_pages, block_table, bt_stride, cu_q, kv_len, n_seqs, nq, nkv, d, page_size,  \
                n_pages, window, scale, TQ, GS, dv, row, sinks, chunk, slopes, planes, keep_first, softcap);          \

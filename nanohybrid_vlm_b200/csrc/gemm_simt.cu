@@ -129,15 +129,16 @@ template <typename T, typename TO, int TM, int TN, int WM, int WN, int STAGES>
 static cudaError_t launch_tile(const SimtGemm& g) {
   constexpr int GM = WM * 4 * TM, GN = WN * 8 * TN, SMEM = STAGES * (GM + GN) * GS * 4;
   const dim3 grid((g.N + GN - 1) / GN, (g.M + GM - 1) / GM, g.batch);
-  auto go = [&](auto kernel) {
-    const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, SMEM);
+  static std::atomic<uint64_t> done[2];
+  auto go = [&](auto kernel, int which) {
+    const cudaError_t e = nhv_allow_smem((const void*)kernel, SMEM, done[which]);
     if (e != cudaSuccess) return e;
     return nhv_launch(kernel, grid, WM * WN * 32, SMEM, g.stream, (TO*)g.C, (const T*)g.A, (const T*)g.W, g.M, g.N, g.K,
                       g.lda, g.ldw, g.ldc, g.batch_a, g.batch_w, g.batch_c);
   };
   if constexpr (std::is_same<T, float>::value)
-    if (g.vec) return go(gemm_nt_simt_kernel<T, TO, TM, TN, WM, WN, STAGES, true>);
-  return go(gemm_nt_simt_kernel<T, TO, TM, TN, WM, WN, STAGES, false>);
+    if (g.vec) return go(gemm_nt_simt_kernel<T, TO, TM, TN, WM, WN, STAGES, true>, 1);
+  return go(gemm_nt_simt_kernel<T, TO, TM, TN, WM, WN, STAGES, false>, 0);
 }
 
 // Which tile: an SM works through its share of the tiles, so the time goes with the tiles of the fullest SM times what

@@ -280,7 +280,8 @@ template <int D, int KIND, typename Gates>
 static cudaError_t cs_launch_pairs(const CsPairs& p, const Gates& gates, int n_tokens, cudaStream_t stream) {
   constexpr int smem = cs_pairs_smem_floats<D, KIND>() * 4;
   auto kernel = chunk_pairs_kernel<D, KIND, Gates>;
-  const cudaError_t e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  static std::atomic<uint64_t> done{0};
+  const cudaError_t e = nhv_allow_smem((const void*)kernel, smem, done);
   if (e != cudaSuccess) return e;
   // many heads on one product of q and k: several blocks compute it, each for four of them
   const int per = p.H / p.G;
@@ -561,7 +562,8 @@ template <int D, int KIND, typename TV>
 static cudaError_t cs_launch_scan(const CsScan& p, int n_seqs, cudaStream_t stream) {
   constexpr int smem = cs_smem_floats<D, KIND>() * 4;
   static_assert(smem <= 115712, "two blocks an SM");
-  const cudaError_t e = cudaFuncSetAttribute(chunk_scan_kernel<D, KIND, TV>, cudaFuncAttributeMaxDynamicSharedMemorySize, smem);
+  static std::atomic<uint64_t> done{0};
+  const cudaError_t e = nhv_allow_smem((const void*)chunk_scan_kernel<D, KIND, TV>, smem, done);
   if (e != cudaSuccess) return e;
   return nhv_launch(chunk_scan_kernel<D, KIND, TV>, dim3(n_seqs, p.H, (p.dv + CS_COLS - 1) / CS_COLS), CS_THREADS, smem, stream, p);
 }

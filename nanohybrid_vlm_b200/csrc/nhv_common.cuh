@@ -9,6 +9,8 @@
 #include <stdint.h>
 #include <stdio.h>
 
+#include <atomic>
+
 #define NHV_API extern "C" __attribute__((visibility("default")))
 
 enum NhvDtype { NHV_F32 = 0, NHV_BF16 = 1 };
@@ -83,6 +85,19 @@ inline cudaError_t nhv_launch(void (*kernel)(KArgs...), dim3 grid, dim3 block, s
   cfg.attrs = attr;
   cfg.numAttrs = 1;
   return cudaLaunchKernelEx(&cfg, kernel, static_cast<KArgs>(args)...);
+}
+
+// Lets a kernel be launched with up to `bytes` of dynamic shared memory: once per device (`done`: one bit each, beside the
+// launch), since the call costs the host about 0.6 us.
+inline cudaError_t nhv_allow_smem(const void* kernel, int bytes, std::atomic<uint64_t>& done) {
+  int device = 0;
+  cudaError_t e = cudaGetDevice(&device);
+  if (e != cudaSuccess) return e;
+  const uint64_t bit = device < 64 ? 1ull << device : 0ull;
+  if (done.load(std::memory_order_relaxed) & bit) return cudaSuccess;
+  e = cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
+  if (e == cudaSuccess) done.fetch_or(bit, std::memory_order_relaxed);
+  return e;
 }
 
 // Shared memory to ask for so that a kernel of few, long-running blocks gets its blocks spread over the SMs: the
