@@ -223,25 +223,41 @@ SCAN_LANES = 0      # lanes per state column in the recurrent scans: 0 is the ke
 CHUNK_SCAN_TOKENS = 0
 
 
-def _by_chunks(n_tokens: int, n_seqs: int, blocks: int, normed: bool) -> bool:
-    """Whether a scan goes by chunks.  ``blocks``: (request, head, 16 columns) of the step; an SM takes two at a time.
-    By chunks against by tokens, in us, on heads of 128 rows and 2,048 columns of state in all: gated delta rule 544 / 1,077
-    (one request of 4,096 tokens), 67 / 80 (200), 55 / 62 (128), 47 / 45 (64), 560 / 753 (5 of 333 to 1,501), but 399 / 326
-    (8 of 512), where a token's work for all requests fills the SMs as it is; the state space 386 / 821, 50 / 60, 43 / 45,
-    38 / 33, 401 / 499 and 282 / 244.  The mLSTM's scan by tokens costs more: 599 / 1,498, 55 / 66 (128), 45 / 43 (64),
-    519 / 1,109, 366 / 734, 8 of 32 tokens 56 / 67."""
+def _by_chunks(n_tokens: int, n_seqs: int, longest: int, blocks: int, sms: int, normed: bool) -> bool:
+    """Whether a scan goes by chunks.  ``blocks``: (head, 16 columns) of a request, ``longest``: tokens of its longest portion.
+
+    Device time (heads of 128 rows, 2,048 columns of state in all, us by chunks / by tokens).  By tokens a request's chain
+    costs 0.3 us a token as long as all blocks run at once; by chunks 0.13, but a third more of the SMs' time.  So chunks
+    win where few requests make a long chain.  Delta rule, requests of 512 tokens: 75 / 135 (one), 115 / 165 (2), 214 / 187 (4),
+    369 / 303 (8); 560 / 753 (5 of 333 to 1,501); the state space 54 / 103, 81 / 139, 151 / 154 and 262 / 226 alike.  Hence a bound
+    on all blocks' tokens over the longest.  The mLSTM's scan by tokens costs more, and chunks win everywhere from 32
+    tokens a request on: 27 / 22 (2 of 32), 41 / 52 (8 of 32), 162 / 271 (48 of 32), 84 / 265 (one of 512).
+
+    Short steps wait for the host, not for the device, and chunks take one to three launches more per layer, 15 to 60 us
+    a step of four layers.  Whole steps, widths 1,024 and 2,048: Muvonex, one prompt of 512 tokens 1,337 / 1,273 and 1,363 /
+    1,381, of 768 1,353 / 1,454 and 1,380 / 1,676, two of 512 1,373 / 1,348 and 1,497 / 1,682, four of 400 1,452 / 1,441 and
+    2,021 / 1,920; Nomudra, one of 512 1,712 / 1,689
+    and 1,707 / 1,717, of 768 1,730 / 1,778 and 1,724 / 1,880, four of 400 1,843 / 1,826 and 2,015 / 2,412, eight of 128 1,867 /
+    1,844 and 1,875 / 1,891.  Hence a long chain, or much work in all."""
     if CHUNK_SCAN_TOKENS:
         return n_tokens >= CHUNK_SCAN_TOKENS * n_seqs
+    work = n_tokens * blocks
     if normed:
-        return n_tokens >= 32 * n_seqs
-    return n_tokens >= 128 * n_seqs and blocks <= 5 * 148
+        return n_tokens >= 32 * n_seqs and (longest >= 640 or work >= 110000)
+    return (n_tokens >= 128 * n_seqs and work <= 2.75 * sms * longest
+            and (longest >= 640 or (longest >= 384 and work >= 110000)))
 
 
-def _chunk_scratch(n_tokens: int, n_seqs: int, heads: int, columns: int, device):
+def _longest(batch, n_tokens: int) -> int:
+    return max(getattr(batch, "max_new_tokens", 0), -(-n_tokens // batch.n_seqs))
+
+
+def _chunk_scratch(n_tokens: int, batch, heads: int, columns: int, device):
     """Scratch for a scan by chunks, or None where the step goes by tokens (or a test asks for a form of that scan)."""
-    if SCAN_LANES or SCAN_GROUP4 == 1 or SCAN_COLUMNS or not _by_chunks(n_tokens, n_seqs, n_seqs * heads * -(-columns // 16), False):
+    if SCAN_LANES or SCAN_GROUP4 == 1 or SCAN_COLUMNS or not _by_chunks(
+            n_tokens, batch.n_seqs, _longest(batch, n_tokens), heads * -(-columns // 16), _sm_count(device), False):
         return None
-    floats = (n_tokens // 32 + n_seqs) * heads * library.load_library().nhv_chunk_scan_floats()
+    floats = (n_tokens // 32 + batch.n_seqs) * heads * library.load_library().nhv_chunk_scan_floats()
     return torch.empty(floats, dtype=torch.float32, device=device)
 
 
@@ -262,7 +278,7 @@ def delta_rule(o, qkv, ba, a_log, dt_bias, state, batch, G: int, H: int, d: int,
         ptrs.append(scratch.data_ptr() + 4 * at)
         at += n
     qn, kn, v32, pairs, kq, beta, decay = ptrs
-    chunks = (None if fixed_order or d > 128 or d % 4 or dv % 4 else _chunk_scratch(T, batch.n_seqs, H, dv, qkv.device))
+    chunks = (None if fixed_order or d > 128 or d % 4 or dv % 4 else _chunk_scratch(T, batch, H, dv, qkv.device))
     call("nhv_delta_rule", dtype_code(qkv), o.data_ptr(), qkv.data_ptr(), qkv.stride(0), ba.data_ptr(), a_log.data_ptr(),
          dt_bias.data_ptr(), state.data_ptr(), state.stride(0), qn, kn, kq, v32, beta, decay, batch.cu_q.data_ptr(),
          batch.q_start.data_ptr(), batch.state_slots.data_ptr(), batch.n_seqs, T, G, H, d, dv, SCAN_LANES, SCAN_GROUP4, pairs,
@@ -279,7 +295,7 @@ def ssd_scan(y, xbc, dt_raw, dt_bias, a_log, d_skip, state, batch, H: int, P: in
     assert y.dtype == dt_raw.dtype == dt_bias.dtype == a_log.dtype == d_skip.dtype == state.dtype == torch.float32
     assert y.is_contiguous() and y.shape == (T, H * P)
     chunks = (None if fixed_order or xbc.dtype != torch.float32 or N > 128 or N % 4 or P % 4
-              else _chunk_scratch(T, batch.n_seqs, H, P, xbc.device))
+              else _chunk_scratch(T, batch, H, P, xbc.device))
     call("nhv_ssd_scan", dtype_code(xbc), y.data_ptr(), xbc.data_ptr(), xbc.stride(0), dt_raw.data_ptr(), dt_raw.stride(0),
          dt_bias.data_ptr(), a_log.data_ptr(), d_skip.data_ptr(), state.data_ptr(), state.stride(0), batch.cu_q.data_ptr(),
          batch.q_start.data_ptr(), batch.state_slots.data_ptr(), batch.n_seqs, T, H, P, N, G, SCAN_LANES,
@@ -699,7 +715,8 @@ def mlstm_scan(y, proj, gates, gate_bias, cap: float, state, batch, H: int, d: i
     assert gate_bias.numel() == 2 * H and state.dim() == 2 and state.stride(1) == 1
     assert state.shape[1] >= mlstm_state_floats(H, d, dv)
     chunks = None
-    if not fixed_order and not MLSTM_LANES and d <= 128 and d % 4 == 0 and dv % 4 == 0 and _by_chunks(T, batch.n_seqs, 0, True):
+    if not fixed_order and not MLSTM_LANES and d <= 128 and d % 4 == 0 and dv % 4 == 0 and _by_chunks(
+            T, batch.n_seqs, _longest(batch, T), H * -(-dv // MLSTM_COLUMN_BLOCK), _sm_count(proj.device), True):
         floats = library.load_library().nhv_mlstm_chunk_floats(T, batch.n_seqs, H, d)
         chunks = torch.empty(floats, dtype=torch.float32, device=proj.device) if floats else None
     call("nhv_mlstm_scan", dtype_code(proj), y.data_ptr(), proj.data_ptr(), proj.stride(0), gates.data_ptr(), gates.stride(0),
