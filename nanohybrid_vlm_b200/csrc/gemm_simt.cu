@@ -151,7 +151,7 @@ static cudaError_t launch_simt(const SimtGemm& g) {
     const long tiles = (long)((g.M + gm - 1) / gm) * ((g.N + gn - 1) / gn) * g.batch;
     return (float)((tiles + 147) / 148) * gm * gn * per_output;
   };
-  const float large = cost(64, 64, 1.0f), medium = cost(32, 64, 1.25f), small = cost(16, 32, 1.6f);
+  const float large = cost(64, 64, 1.0f), medium = cost(32, 64, 1.25f), small = cost(16, 32, 1.7f);
   // (M / 64 blocks fit the grid's second dimension, the caller checks; finer cuts of so many rows might not)
   if ((large <= medium && large <= small) || g.M > 16 * 65535) return launch_tile<T, TO, 8, 4, 2, 2, 3>(g);
   if (medium <= small) return launch_tile<T, TO, 4, 4, 2, 2, 4>(g);
