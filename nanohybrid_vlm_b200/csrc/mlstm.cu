@@ -207,11 +207,12 @@ __global__ void __launch_bounds__(ML_COLS * ML_PARTS) mlstm_scan_kernel(
 
 // ---------------------------------------------------------------- steps of single tokens
 // A step in which every request brings one token only streams the memory through: read, one multiply-add per element,
-// written back.  The scan above goes through seven barriers and reads its columns a float at a time before it can write
+// written back.  The scan above goes through five barriers and reads its columns a float at a time before it can write
 // anything: 74 us for 48 requests of 8 heads of 128 x 256 (50 MB read, 50 MB written), 38 here.  A warp takes the ML_COLS
 // columns that share a copy of n, its lanes four neighbouring rows each (RG groups of them for larger heads), with all of
 // a pass's columns on their way before the first is needed, and no barrier at all.  d in steps of 4 up to 128 RG, state
-// rows 16-byte aligned.  Sums over rows in another order than the scan's: a caller whose results may not depend on how
+// rows 16-byte aligned (with d in steps of 4, slots of nhv_mlstm_state_floats are where H * ceil(dv / ML_COLS) is a
+// multiple of 4; the others take the scan).  Sums over rows in another order than the scan's: a caller whose results may not depend on how
 // tokens were cut into steps does not say that they are single ones.
 template <typename T, int RG>
 __global__ void __launch_bounds__(128) mlstm_step_kernel(
@@ -452,7 +453,12 @@ NHV_API int nhv_mlstm_scan(int dtype, float* y, const void* proj, int proj_strid
                                      : (const void*)((const __nv_bfloat16*)proj + 2 * H * d);
     const CsScan ps{y, pp.q, pp.k, (long)H * d, v, proj_stride, chunks, nullptr, extra, top, state, state_stride, cu_q, q_start,
                     slots, H, H, d, dv};
-#define CHUNKS(D)                                                                                            do {                                                                                                         NHV_CUDA((cs_launch_pairs<D, CS_NORMED>(pp, mg, n_tokens, stream)), "mlstm_scan");                         if (dtype == NHV_F32) NHV_CUDA((cs_launch_scan<D, CS_NORMED, float>(ps, n_seqs, stream)), "mlstm_scan");     else NHV_CUDA((cs_launch_scan<D, CS_NORMED, __nv_bfloat16>(ps, n_seqs, stream)), "mlstm_scan");          } while (0)
+#define CHUNKS(D)                                                                                              \
+  do {                                                                                                         \
+    NHV_CUDA((cs_launch_pairs<D, CS_NORMED>(pp, mg, n_tokens, stream)), "mlstm_scan");                         \
+    if (dtype == NHV_F32) NHV_CUDA((cs_launch_scan<D, CS_NORMED, float>(ps, n_seqs, stream)), "mlstm_scan");   \
+    else NHV_CUDA((cs_launch_scan<D, CS_NORMED, __nv_bfloat16>(ps, n_seqs, stream)), "mlstm_scan");            \
+  } while (0)
     if (d <= 64) CHUNKS(64);
     else CHUNKS(128);
 #undef CHUNKS

@@ -17,9 +17,9 @@
 // Two kernels.  The first has a block per (chunk, q/k head) and no chain: the products q . k and k . k, the decays, the
 // inverse.  It leaves per (chunk, head) CS_WORK floats.  The second has a block per (request, head, 16 columns of S) and
 // walks the request's chunks; K and Q of the next chunk, and P and T' of this one, arrive by cp.async meanwhile.  It is
-// bound by reading shared memory (eight values for sixteen multiply-adds in the largest product) and, between its five
-// barriers a chunk, by latency; chunks of 32 tokens let two blocks share an SM, so that one computes while the other
-// waits (chunks of 64, one block an SM, kept the shared memory's pipe 58% busy).
+// bound by reading shared memory (eight values for sixteen multiply-adds in the largest product) and, between its barriers
+// (six a chunk for the delta rule, five for the others), by latency; chunks of 32 tokens let two blocks share an SM, so
+// that one computes while the other waits.
 // Chunks are numbered over the step: chunk c of request s (first token `first`) is number first / 32 + s + c, which
 // leaves no two requests the same number.
 #pragma once
@@ -329,7 +329,7 @@ __global__ void __launch_bounds__(CS_THREADS, 2) chunk_scan_kernel(const CsScan 
   float* Ss = smem;                                       // [16 columns][RS]
   float* KQ = Ss + CS_COLS * RS;                          // [2 stages][K, Q][32][RS]
   float* Ps = KQ + 4 * CS_C * RS;                         // [32][CS_PS]
-  float* Ts = Ps + CS_C * CS_PS;                          // DELTA: [64][CS_PS]
+  float* Ts = Ps + CS_C * CS_PS;                          // DELTA: [32][CS_PS]
   float* Rs = Ts + (DELTA ? CS_C * CS_PS : 0);            // [16 columns][CS_PS]: V, for DELTA then V - diag(gam) K s0
   float* Us = Rs + CS_COLS * CS_PS;                       // DELTA: [16 columns][CS_PS]
   float* Vec = Us + CS_COLS * CS_PS;                      // [2 stages][gam, E, P's diagonal, T' 's][32]

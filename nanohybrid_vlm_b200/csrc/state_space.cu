@@ -401,9 +401,6 @@ __global__ void __launch_bounds__(SF_THREADS) ssd_scan_wide_kernel(
     }
 }
 
-
-// xbc [T, H*P + 2*G*N] (x, then B, then C), dt_raw [T, >= H] fp32, y [T, H*P] fp32.  lanes: 8, 16 or 32 lanes per
-// column of the state in the fast form, or 0 to choose by the size of the step.
 struct SsdGates {
   const float* dt_raw;                                   // row t, head h: at t * dt_stride + h
   int dt_stride;
@@ -414,6 +411,8 @@ struct SsdGates {
   }
 };
 
+// xbc [T, H*P + 2*G*N] (x, then B, then C), dt_raw [T, >= H] fp32, y [T, H*P] fp32.  lanes: 8, 16 or 32 lanes per
+// column of the state in the fast form, or 0 to choose by the size of the step.
 // chunks: scratch of (n_tokens / 32 + n_seqs) * H * nhv_chunk_scan_floats() floats to go through prompts a chunk of tokens
 // at a time (fp32 inputs, N up to 128, sizes in steps of 4; null: token by token).
 NHV_API int nhv_ssd_scan(int dtype, float* y, const void* xbc, int xbc_stride, const float* dt_raw, int dt_stride,

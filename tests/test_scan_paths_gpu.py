@@ -1,4 +1,4 @@
-"""The recurrent kernels' other ways through a step (single tokens of the mLSTM streamed through; prompts 64 tokens at a
+"""The recurrent kernels' other ways through a step (single tokens of the mLSTM streamed through; prompts 32 tokens at a
 time), against plain recurrences in 64 bits: portions that end at, before and behind a chunk, single tokens beside them,
 states handed from one way to the other, heads of less than a kernel's width, columns that are no multiple of 16."""
 import pytest
