@@ -160,38 +160,80 @@ NHV_API int nhv_moe_route(int* ids, float* weights, const float* logits, int ld,
 // ---------------------------------------------------------------- order by expert
 constexpr int MA_THREADS = 1024;
 constexpr int MA_MAX_EXPERTS = 2048;
+constexpr int MA_BLOCKS = 8;                             // of a cluster, where a step has many slots
 
+__device__ __forceinline__ void ma_cluster_sync() {
+  asm volatile("barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;\n" ::: "memory");
+}
+__device__ __forceinline__ int ma_read(const int* mine, int rank) {      // the same variable of another block of the cluster
+  uint32_t at;
+  int v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(at) : "r"((uint32_t)__cvta_generic_to_shared(mine)), "r"(rank));
+  asm volatile("ld.shared::cluster.s32 %0, [%1];\n" : "=r"(v) : "r"(at) : "memory");
+  return v;
+}
+
+// CLUSTER blocks share the slots: each counts its own part, reads the others' counts and places its part behind those of
+// the blocks before it.  The counting and the placing are atomics in shared memory, many to one address: that is what the
+// time goes into (18,340 slots of 16 experts: 12.5 us by one block, 7.5 by eight; up to 2,048 slots, two a thread, one
+// block is as fast).
+template <int CLUSTER>
 __global__ void __launch_bounds__(MA_THREADS) moe_align_kernel(
     const int* __restrict__ ids, int n_slots, int E, int BM, int cap, int max_tiles, int* __restrict__ sorted_slots,
     int* __restrict__ slot_pos, int* __restrict__ tile_expert) {
   __shared__ int count[MA_MAX_EXPERTS];
+  __shared__ int total[CLUSTER > 1 ? MA_MAX_EXPERTS : 1];
   __shared__ int start[MA_MAX_EXPERTS + 1];
   pdl_prologue();
-  const int tid = threadIdx.x;
+  const int tid = threadIdx.x, rank = CLUSTER > 1 ? blockIdx.x : 0;
+  const int lo = (int)((long)n_slots * rank / CLUSTER), hi = (int)((long)n_slots * (rank + 1) / CLUSTER);
+  const int* all = CLUSTER > 1 ? total : count;
   for (int e = tid; e < E; e += MA_THREADS) count[e] = 0;
-  for (int i = tid; i < cap; i += MA_THREADS) sorted_slots[i] = -1;
-  for (int i = tid; i < max_tiles; i += MA_THREADS) tile_expert[i] = -1;
   __syncthreads();
-  for (int i = tid; i < n_slots; i += MA_THREADS) {
+  for (int i = lo + tid; i < hi; i += MA_THREADS) {
     const int e = ids[i];
     if (e >= 0 && e < E) atomicAdd(&count[e], 1);
+  }
+  if (CLUSTER > 1) {
+    ma_cluster_sync();
+    for (int e = tid; e < E; e += MA_THREADS) {
+      int sum = 0, before = 0;
+      for (int r = 0; r < CLUSTER; ++r) {
+        const int c = ma_read(&count[e], r);
+        if (r == rank) before = sum;
+        sum += c;
+      }
+      total[e] = sum;
+      start[e] = before;                                       // of this block's part in the expert's run, for now
+    }
+    ma_cluster_sync();                                         // (the counts are overwritten below)
+    for (int e = tid; e < E; e += MA_THREADS) count[e] = start[e];
   }
   __syncthreads();
   if (tid == 0) {
     int at = 0;
     for (int e = 0; e < E; ++e) {
       start[e] = at;
-      at += (count[e] + BM - 1) / BM * BM;
+      at += (all[e] + BM - 1) / BM * BM;
     }
     start[E] = at;
   }
   __syncthreads();
-  for (int e = tid; e < E; e += MA_THREADS) {
-    for (int r = start[e]; r < start[e + 1]; r += BM) tile_expert[r / BM] = e;
-    count[e] = 0;                                              // now the cursor of the expert's run
+  // block 0: which tile is whose, and the padding (behind each expert's slots, and behind the last expert's)
+  if (rank == 0) {
+    for (int i = start[E] / BM + tid; i < max_tiles; i += MA_THREADS) tile_expert[i] = -1;
+    for (int i = start[E] + tid; i < cap; i += MA_THREADS) sorted_slots[i] = -1;
+    for (int e = tid >> 5; e < E; e += MA_THREADS / 32) {
+      for (int r = start[e] + BM * (tid & 31); r < start[e + 1]; r += BM * 32) tile_expert[r / BM] = e;
+      for (int r = start[e] + all[e] + (tid & 31); r < start[e + 1]; r += 32) sorted_slots[r] = -1;
+    }
+    __syncthreads();
   }
-  __syncthreads();
-  for (int i = tid; i < n_slots; i += MA_THREADS) {
+  if (CLUSTER == 1) {
+    for (int e = tid; e < E; e += MA_THREADS) count[e] = 0;    // now the cursor of the expert's run
+    __syncthreads();
+  }
+  for (int i = lo + tid; i < hi; i += MA_THREADS) {
     const int e = ids[i];
     int pos = -1;
     if (e >= 0 && e < E) {
@@ -214,8 +256,11 @@ NHV_API int nhv_moe_align(const int* ids, int n_slots, int E, int BM, int* sorte
   if (n_slots == 0) return 0;
   NHV_REQUIRE(E > 0 && E <= MA_MAX_EXPERTS && BM > 0, "moe_align: %d experts are beyond the supported %d", E, MA_MAX_EXPERTS);
   const int cap = nhv_moe_sorted_rows(n_slots, E, BM);
-  nhv_launch(moe_align_kernel, 1, MA_THREADS, 0, stream, ids, n_slots, E, BM, cap, cap / BM, sorted_slots, slot_pos,
-             tile_expert);
+  if (n_slots <= 2 * MA_THREADS)
+    nhv_launch(moe_align_kernel<1>, 1, MA_THREADS, 0, stream, ids, n_slots, E, BM, cap, cap / BM, sorted_slots, slot_pos, tile_expert);
+  else
+    NHV_CUDA(nhv_launch_cluster(moe_align_kernel<MA_BLOCKS>, MA_BLOCKS, MA_THREADS, 0, stream, MA_BLOCKS, ids, n_slots, E, BM, cap,
+                                cap / BM, sorted_slots, slot_pos, tile_expert), "moe_align");
   NHV_CHECK_LAUNCH("moe_align");
   return 0;
 }

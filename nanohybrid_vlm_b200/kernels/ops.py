@@ -800,12 +800,12 @@ def _first_product(gate, up):
 MOE_ON_TENSOR_CORES = True      # tests switch it off to compare with the CUDA-core products at the same shapes
 MOE_TILE = 0                    # rows per tile of the mma.sync products: 0 chooses by the step; tests set 16, 64, 128
 MOE_TCGEN05 = None              # the tcgen05 products: None where an expert sees many rows; tests set True (always) or False
-MOE_TCGEN05_TILE = 128          # rows per tile of the tcgen05 products (ROWS of csrc/moe_tcgen05.cu)
+MOE_TCGEN05_TILE = 256          # rows per tile of the tcgen05 products (ROWS of csrc/moe_tcgen05.cu)
 
 
 def moe_experts(x, gate, up, down, ids, limit: float, alpha: float, up_shift: float = 1.0, row_scale=None):
     """Every chosen expert's output for every token: orders the slots of ids [T, top] by expert and runs the experts' two
-    products over that order: bfloat16 with sizes in steps of 8 on the tensor cores (tcgen05 with tiles of 128 rows
+    products over that order: bfloat16 with sizes in steps of 8 on the tensor cores (tcgen05 with tiles of 256 rows
     where an expert sees about a hundred rows or more; mma.sync with tiles of 64 rows below that and of 16 where it
     sees few and the products stream the weights), everything else on the CUDA cores.
     The experts' unit is g' sigmoid(alpha g') (u' + up_shift) with g' = min(g, limit), u' = clamp(u, -limit, limit)
@@ -850,7 +850,7 @@ def _check_experts(x, gate, up, down) -> None:
 
 
 def _moe_experts_tcgen05(x, gate, up, down, ids, limit: float, alpha: float, up_shift: float = 1.0, row_scale=None):
-    """``moe_experts`` for prompts in bfloat16: tiles of 128 rows per expert, the tokens' rows gathered into that order
+    """``moe_experts`` for prompts in bfloat16: tiles of 256 rows per expert, the tokens' rows gathered into that order
     (so that a tile is one TMA box), both products with tcgen05.mma and tensor-memory accumulators."""
     _need_cuda(x, gate, up, down, ids)
     _check_experts(x, gate, up, down)
