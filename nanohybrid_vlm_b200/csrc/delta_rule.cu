@@ -747,15 +747,15 @@ struct DeltaGates {
   }
 };
 
-// Floats of scratch per head and chunk for the kernels that go through prompts a chunk of tokens at a time; a step has
-// n_tokens / 32 + n_seqs chunks.
-NHV_API int nhv_chunk_scan_floats() { return CS_WORK; }
+// Floats of scratch per chunk for the kernels that go through prompts a chunk of tokens at a time (H heads of d rows of state, G
+// q/k heads); a step has n_tokens / 32 + n_seqs chunks.
+NHV_API int nhv_chunk_scan_floats(int G, int H, int d) { return (int)cs_floats(1, G, H, d); }
 
 // o_out [T, H, dv] fp32.  lanes: 4, 8, 16 or 32 lanes per column of the state, or 0 for the kernel's own choice.
 // group4: 1 takes four tokens per round of the chain (needs pairs [T, G, 8] as scratch), 0 one, -1 chooses by the
 // size of the step.  cpt: 2 or 4 columns of the state per lane (8 lanes a column, d up to 128), 1 one, 0 the
 // kernel's choice.
-// chunks: scratch of (n_tokens / 32 + n_seqs) * H * nhv_chunk_scan_floats() floats to go through the prompts a chunk of
+// chunks: scratch of (n_tokens / 32 + n_seqs) * nhv_chunk_scan_floats(G, H, d) floats to go through the prompts a chunk of
 // tokens at a time (d up to 128, sizes in steps of 4; null: token by token).
 // Scratch given by the caller, all fp32: qn, kn [T, G, d]; kq [T, G]; v32 [T, H, dv]; beta,
 // decay [T, H].
@@ -785,9 +785,10 @@ NHV_API int nhv_delta_rule(int dtype, float* o_out, const void* qkv, int qkv_str
 #undef PREP
   // prompts: a chunk of tokens at a time
   if (chunks && fast && d <= 128) {
-    const CsPairs pp{qn, kn, (long)G * d, chunks, nullptr, cu_q, slots, n_seqs, G, H, d};
+    float* work = chunks + cs_chunks(n_tokens, n_seqs) * G * cs_image_floats(cs_width(d));
+    const CsPairs pp{qn, kn, (long)G * d, chunks, work, nullptr, cu_q, slots, n_seqs, G, H, d};
     const DeltaGates gates{decay, beta, H};
-    const CsScan ps{o_out, qn, kn, (long)G * d, v_src, v_stride, chunks, nullptr, nullptr, nullptr, state, state_stride,
+    const CsScan ps{o_out, v_src, v_stride, chunks, work, nullptr, nullptr, nullptr, state, state_stride,
                     cu_q, q_start, slots, G, H, d, dv};
     if (d <= 64) {
       NHV_CUDA((cs_launch_pairs<64, CS_DELTA>(pp, gates, n_tokens, stream)), "delta_rule");

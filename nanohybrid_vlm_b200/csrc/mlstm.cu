@@ -384,7 +384,7 @@ struct MlstmGates {
 
 // Floats of scratch for the above: per chunk and head, and per token (nhv_mlstm_scan's `chunks`).
 NHV_API int nhv_mlstm_chunk_floats(int n_tokens, int n_seqs, int H, int d) {
-  const long floats = cs_chunks(n_tokens, n_seqs) * H * (CS_WORK + 2 * CS_C + d) + (long)n_tokens * H * (2 * d + 4);
+  const long floats = cs_floats(cs_chunks(n_tokens, n_seqs), H, H, d) + cs_chunks(n_tokens, n_seqs) * H * (2 * CS_C + d) + (long)n_tokens * H * (2 * d + 4);
   return floats < (1l << 31) - 1 ? (int)floats : 0;       // 0: beyond what this counts; the step goes token by token
 }
 
@@ -434,24 +434,25 @@ NHV_API int nhv_mlstm_scan(int dtype, float* y, const void* proj, int proj_strid
     const int nb = (dv + ML_COLS - 1) / ML_COLS;
     static_assert(ML_COLS == CS_COLS, "a copy of n per block of columns");
     const long nc = cs_chunks(n_tokens, n_seqs), th = (long)n_tokens * H;
-    float* extra = chunks + nc * H * CS_WORK;
+    float* work = chunks + nc * H * cs_image_floats(cs_width(d));
+    float* extra = work + nc * H * CS_WORK;
     float* qk = extra + nc * H * (2 * CS_C + d);
     float *a = qk + 2 * th * d, *b = a + th, *em = b + th, *top = em + th;
     nhv_launch(mlstm_gates_kernel, dim3(n_seqs, H), MG_TOKENS, 0, stream, a, b, em, top, gates, gate_stride, gate_bias, cap,
                (const float*)state, state_stride, cu_q, q_start, slots, H, d, dv, nb);
-    const long work = (long)n_tokens * H * d / 2;
-    const int blocks = (int)(work / 256 + 1 < 148 * 8 ? work / 256 + 1 : 148 * 8);
+    const long quarters = (long)n_tokens * H * d / 2;
+    const int blocks = (int)(quarters / 256 + 1 < 148 * 8 ? quarters / 256 + 1 : 148 * 8);
     const float qscale = 1.0f / sqrtf((float)d);
     if (dtype == NHV_F32)
       nhv_launch(mlstm_widen_kernel<float>, blocks, 256, 0, stream, qk, (const float*)proj, proj_stride, n_tokens, H * d, qscale);
     else
       nhv_launch(mlstm_widen_kernel<__nv_bfloat16>, blocks, 256, 0, stream, qk, (const __nv_bfloat16*)proj, proj_stride,
                  n_tokens, H * d, qscale);
-    const CsPairs pp{qk, qk + th * d, (long)H * d, chunks, extra, cu_q, slots, n_seqs, H, H, d};
+    const CsPairs pp{qk, qk + th * d, (long)H * d, chunks, work, extra, cu_q, slots, n_seqs, H, H, d};
     const MlstmGates mg{a, b, em, H};
     const void* v = dtype == NHV_F32 ? (const void*)((const float*)proj + 2 * H * d)
                                      : (const void*)((const __nv_bfloat16*)proj + 2 * H * d);
-    const CsScan ps{y, pp.q, pp.k, (long)H * d, v, proj_stride, chunks, nullptr, extra, top, state, state_stride, cu_q, q_start,
+    const CsScan ps{y, v, proj_stride, chunks, work, nullptr, extra, top, state, state_stride, cu_q, q_start,
                     slots, H, H, d, dv};
 #define CHUNKS(D)                                                                                              \
   do {                                                                                                         \

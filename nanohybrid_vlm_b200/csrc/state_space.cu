@@ -413,7 +413,7 @@ struct SsdGates {
 
 // xbc [T, H*P + 2*G*N] (x, then B, then C), dt_raw [T, >= H] fp32, y [T, H*P] fp32.  lanes: 8, 16 or 32 lanes per
 // column of the state in the fast form, or 0 to choose by the size of the step.
-// chunks: scratch of (n_tokens / 32 + n_seqs) * H * nhv_chunk_scan_floats() floats to go through prompts a chunk of tokens
+// chunks: scratch of (n_tokens / 32 + n_seqs) * nhv_chunk_scan_floats(G, H, N) floats to go through prompts a chunk of tokens
 // at a time (fp32 inputs, N up to 128, sizes in steps of 4; null: token by token).
 NHV_API int nhv_ssd_scan(int dtype, float* y, const void* xbc, int xbc_stride, const float* dt_raw, int dt_stride,
                          const float* dt_bias, const float* a_log, const float* d_skip, float* state,
@@ -427,10 +427,11 @@ NHV_API int nhv_ssd_scan(int dtype, float* y, const void* xbc, int xbc_stride, c
   const bool fast = dtype == NHV_F32 && N % 4 == 0 && P % 4 == 0 && xbc_stride % 4 == 0 && ((uintptr_t)xbc % 16) == 0;
   if (chunks && fast && N <= 128) {
     const float* rows = (const float*)xbc;
-    const CsPairs pp{rows + (size_t)H * P + (size_t)G * N, rows + (size_t)H * P, xbc_stride, chunks, nullptr, cu_q, slots,
+    float* work = chunks + cs_chunks(n_tokens, n_seqs) * G * cs_image_floats(cs_width(N));
+    const CsPairs pp{rows + (size_t)H * P + (size_t)G * N, rows + (size_t)H * P, xbc_stride, chunks, work, nullptr, cu_q, slots,
                      n_seqs, G, H, N};
     const SsdGates gates{dt_raw, dt_stride, dt_bias, a_log};
-    const CsScan ps{y, pp.q, pp.k, xbc_stride, rows, xbc_stride, chunks, d_skip, nullptr, nullptr, state, state_stride, cu_q,
+    const CsScan ps{y, rows, xbc_stride, chunks, work, d_skip, nullptr, nullptr, state, state_stride, cu_q,
                     q_start, slots, G, H, N, P};
     if (N <= 64) {
       NHV_CUDA((cs_launch_pairs<64, CS_PLAIN>(pp, gates, n_tokens, stream)), "ssd_scan");

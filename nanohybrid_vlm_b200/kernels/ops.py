@@ -227,14 +227,15 @@ def _by_chunks(n_tokens: int, n_seqs: int, longest: int, blocks: int, sms: int, 
     """Whether a scan goes by chunks.  ``blocks``: (head, 16 columns) of a request, ``longest``: tokens of its longest portion.
 
     Device time (heads of 128 rows, 2,048 columns of state in all, us by chunks / by tokens).  By tokens a request's chain
-    costs 0.3 us a token as long as all blocks run at once; by chunks 0.13, but a third more of the SMs' time.  So chunks
-    win where few requests make a long chain.  Delta rule, requests of 512 tokens: 75 / 135 (one), 115 / 165 (2), 214 / 187 (4),
-    369 / 303 (8); 560 / 753 (5 of 333 to 1,501); the state space 54 / 103, 81 / 139, 151 / 154 and 262 / 226 alike.  Hence a bound
-    on all blocks' tokens over the longest.  The mLSTM's scan by tokens costs more, and chunks win everywhere from 32
-    tokens a request on: 27 / 22 (2 of 32), 41 / 52 (8 of 32), 162 / 271 (48 of 32), 84 / 265 (one of 512).
+    costs 0.25 us a token as long as all blocks run at once; by chunks 0.08, but all of the SMs' time.  So chunks
+    win where few requests make a long chain.  Delta rule, requests of 512 tokens: 50 / 135 (one), 79 / 166 (2), 147 / 189 (4),
+    279 / 303 (8); 370 / 734 (5 of 333 to 1,501); 133 / 121 (8 of 200), 314 / 243 (48 of 80); the state space 37 / 104, 54 / 140,
+    97 / 154, 189 / 227, 250 / 485, 88 / 92 and 216 / 172 alike.  Hence a bound on all blocks' tokens over the longest.  The
+    mLSTM's scan by tokens costs more, and chunks win everywhere from 32 tokens a request on: 56 / 189 (one of 512), 78 / 185 (8 of
+    128), 133 / 273 (48 of 32).
 
     Short steps wait for the host, not for the device, and chunks take one to three launches more per layer, 15 to 60 us
-    a step of four layers.  Whole steps, widths 1,024 and 2,048: Muvonex, one prompt of 512 tokens 1,337 / 1,273 and 1,363 /
+    a step of four layers.  Whole steps (with scans by chunks that took 1.5 times as long as now), widths 1,024 and 2,048: Muvonex, one prompt of 512 tokens 1,337 / 1,273 and 1,363 /
     1,381, of 768 1,353 / 1,454 and 1,380 / 1,676, two of 512 1,373 / 1,348 and 1,497 / 1,682, four of 400 1,452 / 1,441 and
     2,021 / 1,920; Nomudra, one of 512 1,712 / 1,689
     and 1,707 / 1,717, of 768 1,730 / 1,778 and 1,724 / 1,880, four of 400 1,843 / 1,826 and 2,015 / 2,412, eight of 128 1,867 /
@@ -252,12 +253,12 @@ def _longest(batch, n_tokens: int) -> int:
     return max(getattr(batch, "max_new_tokens", 0), -(-n_tokens // batch.n_seqs))
 
 
-def _chunk_scratch(n_tokens: int, batch, heads: int, columns: int, device):
+def _chunk_scratch(n_tokens: int, batch, groups: int, heads: int, rows: int, columns: int, device):
     """Scratch for a scan by chunks, or None where the step goes by tokens (or a test asks for a form of that scan)."""
     if SCAN_LANES or SCAN_GROUP4 == 1 or SCAN_COLUMNS or not _by_chunks(
             n_tokens, batch.n_seqs, _longest(batch, n_tokens), heads * -(-columns // 16), _sm_count(device), False):
         return None
-    floats = (n_tokens // 32 + batch.n_seqs) * heads * library.load_library().nhv_chunk_scan_floats()
+    floats = (n_tokens // 32 + batch.n_seqs) * library.load_library().nhv_chunk_scan_floats(groups, heads, rows)
     return torch.empty(floats, dtype=torch.float32, device=device)
 
 
@@ -278,7 +279,7 @@ def delta_rule(o, qkv, ba, a_log, dt_bias, state, batch, G: int, H: int, d: int,
         ptrs.append(scratch.data_ptr() + 4 * at)
         at += n
     qn, kn, v32, pairs, kq, beta, decay = ptrs
-    chunks = (None if fixed_order or d > 128 or d % 4 or dv % 4 else _chunk_scratch(T, batch, H, dv, qkv.device))
+    chunks = (None if fixed_order or d > 128 or d % 4 or dv % 4 else _chunk_scratch(T, batch, G, H, d, dv, qkv.device))
     call("nhv_delta_rule", dtype_code(qkv), o.data_ptr(), qkv.data_ptr(), qkv.stride(0), ba.data_ptr(), a_log.data_ptr(),
          dt_bias.data_ptr(), state.data_ptr(), state.stride(0), qn, kn, kq, v32, beta, decay, batch.cu_q.data_ptr(),
          batch.q_start.data_ptr(), batch.state_slots.data_ptr(), batch.n_seqs, T, G, H, d, dv, SCAN_LANES, SCAN_GROUP4, pairs,
@@ -295,7 +296,7 @@ def ssd_scan(y, xbc, dt_raw, dt_bias, a_log, d_skip, state, batch, H: int, P: in
     assert y.dtype == dt_raw.dtype == dt_bias.dtype == a_log.dtype == d_skip.dtype == state.dtype == torch.float32
     assert y.is_contiguous() and y.shape == (T, H * P)
     chunks = (None if fixed_order or xbc.dtype != torch.float32 or N > 128 or N % 4 or P % 4
-              else _chunk_scratch(T, batch, H, P, xbc.device))
+              else _chunk_scratch(T, batch, G, H, N, P, xbc.device))
     call("nhv_ssd_scan", dtype_code(xbc), y.data_ptr(), xbc.data_ptr(), xbc.stride(0), dt_raw.data_ptr(), dt_raw.stride(0),
          dt_bias.data_ptr(), a_log.data_ptr(), d_skip.data_ptr(), state.data_ptr(), state.stride(0), batch.cu_q.data_ptr(),
          batch.q_start.data_ptr(), batch.state_slots.data_ptr(), batch.n_seqs, T, H, P, N, G, SCAN_LANES,
