@@ -1,6 +1,6 @@
 // C[M,N] = A[M,K] * W[N,K]^T on the CUDA cores with fp32 multiply-add: the matrix
-// product of the true 32-bit path (no TF32 or other reduced-precision matrix mode), also
-// usable with bf16 storage.  W is row-major [out, in] as in nanovllm/layers/linear.py:40,66.
+// product of the true 32-bit path (no TF32 or other reduced-precision matrix mode) for sizes that
+// gemm_f32_tcgen05.cu does not take, also usable with bf16 storage.  W is row-major [out, in] as in nanovllm/layers/linear.py:40,66.
 //
 // Each output element is two accumulators, of the products at even and at odd k, each in ascending k, added at the
 // end; so the value of C[m,n] does not depend on M, on the tile that holds it or on the batch.

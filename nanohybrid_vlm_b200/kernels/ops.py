@@ -1329,8 +1329,11 @@ def linear(out, x, weight) -> None:
     assert weight.shape[1] == K and out.shape == (M, N)
     if x.dtype == torch.float32:
         assert out.dtype == torch.float32
-        call("nhv_gemm_nt_simt", F32, out.data_ptr(), x.data_ptr(), weight.data_ptr(), M, N, K, x.stride(0), K, N, 0,
-             stream_ptr())
+        if _f32_on_tensor_cores(x, weight):
+            call("nhv_gemm_f32_tcgen05", out.data_ptr(), x.data_ptr(), weight.data_ptr(), M, N, K, x.stride(0), N, stream_ptr())
+        else:
+            call("nhv_gemm_nt_simt", F32, out.data_ptr(), x.data_ptr(), weight.data_ptr(), M, N, K, x.stride(0), K, N, 0,
+                 stream_ptr())
     elif small_m_ok(x, weight):
         _small_m(out, x, weight, M, N, K, int(out.dtype == torch.float32), 0)
     elif out.dtype == torch.float32:
@@ -1341,6 +1344,19 @@ def linear(out, x, weight) -> None:
         to_f32(out, tmp)
     else:
         torch.mm(x, weight.t(), out=out)
+
+
+F32_ON_TENSOR_CORES = True      # tests switch it off to compare with the CUDA-core product at the same shapes
+
+
+def _f32_on_tensor_cores(x, weight) -> bool:
+    """Whether a float32 product runs on the tensor cores, operands cut into three bfloat16 (csrc/gemm_f32_tcgen05.cu).  By the
+    weight's sizes alone, never by the number of tokens: so a token's result does not depend on what it is computed with.
+    In us on the CUDA cores / the tensor cores: a weight of 512 x 512 13 / 13 for 1 to 128 tokens and 35 / 19 for 2,048; 256 x 256 8 / 12 (the
+    line lies where launches of either cost the same); 4,096 x 1,024 23 / 17 for 16 tokens, 90 / 43 for 370."""
+    N, K = weight.shape
+    return (F32_ON_TENSOR_CORES and N >= 512 and K >= 512 and K % 4 == 0 and x.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0
+            and weight.data_ptr() % 16 == 0)
 
 
 SMALL_M = 8     # up to this many tokens the weight-streaming kernel runs instead of the library product
@@ -1642,7 +1658,7 @@ def _register_library_sources() -> None:
     import ctypes
     from .library import load_library
     lib = load_library()
-    for name in ("gemm_slab", "gemm_stream_k", "gemm_tcgen05", "moe_tcgen05"):
+    for name in ("gemm_slab", "gemm_stream_k", "gemm_tcgen05", "moe_tcgen05", "gemm_f32_tcgen05"):
         word = getattr(lib, f"nhv_{name}_error_word")
         word.restype, word.argtypes = ctypes.c_void_p, []
         take = getattr(lib, f"nhv_{name}_error")
