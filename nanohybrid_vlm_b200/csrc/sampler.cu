@@ -67,7 +67,26 @@ __global__ void __launch_bounds__(256) sample_kernel(int* __restrict__ out, cons
   const int g_end = min(n_groups, ((int)blockIdx.y + 1) * per);
   const bool vec = (ld & 3) == 0 && ((uintptr_t)logits & 15) == 0;
   unsigned long long key = 0;
-  for (int gidx = blockIdx.y * per + threadIdx.x; gidx < g_end; gidx += blockDim.x) {
+  int gidx = blockIdx.y * per + threadIdx.x;
+  if (!(temp > 0.f) && vec) {
+    // no noise: a thread asks for four pieces of four scores at once (one at a time, eight of them took 6 us one after the other)
+    const int whole = min(g_end, vocab >> 2), step = blockDim.x;
+    for (; gidx + 3 * step < whole; gidx += 4 * step) {
+      float4 f[4];
+#pragma unroll
+      for (int j = 0; j < 4; ++j) f[j] = *reinterpret_cast<const float4*>(lg + (size_t)(gidx + j * step) * 4);
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const float v[4] = {f[j].x, f[j].y, f[j].z, f[j].w};
+#pragma unroll
+        for (int k = 0; k < 4; ++k) {
+          const unsigned long long kk = score_key(v[k], (gidx + j * step) * 4 + k);
+          key = kk > key ? kk : key;
+        }
+      }
+    }
+  }
+  for (; gidx < g_end; gidx += blockDim.x) {
     uint32_t c[4] = {(uint32_t)gidx, pos, 0u, 0u};
     if (temp > 0.f) philox4x32_10(c, k0, k1);
     float v[4];
@@ -122,9 +141,11 @@ NHV_API int nhv_sample(int* out, const float* logits, int ld, const float* tempe
                        int* status, cudaStream_t stream) {
   if (n_rows == 0) return 0;
   NHV_REQUIRE(n_rows > 0 && vocab > 0 && ld >= vocab && best && arrived, "sample: bad arguments");
-  // pieces of about 8,192 scores, but no more blocks than a few per SM
-  int pieces = (vocab + 8191) / 8192;
-  const int room = 148 * 4 / n_rows;
+  // pieces of about 4,096 scores (four reads of 16 bytes a thread), but no more blocks than an SM holds.  What
+  // it adds to a step, with pieces of 8,192 read one after the other and now: 8 rows of 32,000 13.3 and 10.6 us, 256 rows of
+  // 43,392 22.1 and 13.1.
+  int pieces = (vocab + 4095) / 4096;
+  const int room = 148 * 8 / n_rows;
   if (pieces > room) pieces = room < 1 ? 1 : room;
   nhv_launch(sample_kernel, dim3(n_rows, pieces), 256, 0, stream, out, logits, ld, temperatures, seeds, positions, vocab,
              best, arrived, error_words, error_words ? n_error_words : 0, error_words ? status : (int*)nullptr);
