@@ -203,7 +203,7 @@ __global__ void attn_paged_simt_kernel(const T* __restrict__ q, int q_stride, T*
 // The kernel above reads one float of K and one of q from shared memory per multiply-add and waits for every chunk of
 // keys: 320 us for 370 tokens (37 to 210 a request) of 16 heads of 128; this one takes 80.  For heads of up to 256
 // elements in steps of four, in rows that can be read 16 (bf16: 8) bytes at a time:
-//   - a warp takes its pairs (up to 8) through a chunk together, so that a key's four elements, read once, serve all of
+//   - a warp takes its pairs (up to 4 or 8) through a chunk together, so that a key's four elements, read once, serve all of
 //     them, and likewise a value's; q and the probabilities are broadcast reads of four;
 //   - key rows are d + 4 floats apart: the eight lanes that are served at once read different banks;
 //   - products and sums two at a time (a score is the sum of its even and its odd elements, each in ascending order);
@@ -223,11 +223,11 @@ static __device__ __forceinline__ float4 simt_load4(const __nv_bfloat16* p) {
   return make_float4(lo.x, lo.y, hi.x, hi.y);
 }
 
-constexpr int AV_PAIRS = 8;             // pairs per warp
+constexpr int AV_BLOCK = 32;            // pairs of a block, dealt to its four or eight warps
 
 // VC: groups of four output columns per lane (value heads of up to 128 VC elements)
-template <typename T, int VC>
-__global__ void __launch_bounds__(AT_WARPS * 32) attn_paged_simt_vec_kernel(
+template <typename T, int VC, int WARPS>
+__global__ void __launch_bounds__(WARPS * 32) attn_paged_simt_vec_kernel(
     const T* __restrict__ q, int q_stride, T* __restrict__ out, int out_stride, const T* __restrict__ kv_pages,
     const int* __restrict__ block_table, int bt_stride, const int* __restrict__ cu_q, const int* __restrict__ kv_len,
     int n_seqs, int nq, int nkv, int d, int page_size, int n_pages, int window, float scale, int TQ, int GS, int dv, int row,
@@ -261,10 +261,10 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attn_paged_simt_vec_kernel(
   const int stage_floats = AT_CHUNK * ks + (planes == 2 ? AT_CHUNK * dv : 0);
   float* Qs = smem + STAGES * stage_floats;              // [pairs][d]
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
-  float* Ps = Qs + AV_PAIRS * AT_WARPS * d + warp * AV_PAIRS * AT_CHUNK;   // [pairs of the warp][32]
+  float* Ps = Qs + AV_BLOCK * d + warp * (AV_BLOCK / WARPS) * AT_CHUNK;   // [pairs of the warp][32]
   const int d4 = d >> 2, dv4 = dv >> 2;
 
-  for (int i = tid; i < n_pairs * d4; i += AT_WARPS * 32) {
+  for (int i = tid; i < n_pairs * d4; i += WARPS * 32) {
     const int p = i / d4, c = 4 * (i - p * d4);
     const int tq = p / gs, g = p - tq * gs;
     const size_t tok = (size_t)cu_q[seq] + t0 + tq;
@@ -285,7 +285,7 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attn_paged_simt_vec_kernel(
   // kernel above.  Heads of 128 in fp32, 16 over 8: 293, 207 here.)
   auto fetch_plane = [&](float* to, int stride, const T* from, long row_at, int pieces) {
 #pragma unroll 4
-    for (int e = tid; e < AT_CHUNK * pieces; e += AT_WARPS * 32) {          // (32 pieces of a warp: all its lanes go along)
+    for (int e = tid; e < AT_CHUNK * pieces; e += WARPS * 32) {          // (32 pieces of a warp: all its lanes go along)
       const int r = e / pieces, c = 4 * (e - r * pieces);
       const long at = __shfl_sync(0xffffffffu, row_at, r);
       const T* src = from + (at >= 0 ? at * row + c : 0);
@@ -308,14 +308,14 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attn_paged_simt_vec_kernel(
     return c0 >= kept_end && c0 < c_begin ? c_begin : c0;
   };
 
-  // pair i of the warp is pair warp + i * AT_WARPS of the block; NP of them may exist
+  // pair i of the warp is pair warp + i * WARPS of the block; NP of them may exist
   auto work = [&](auto np) {
     constexpr int NP = decltype(np)::value;
     float m[NP], l[NP];
     f32x2 o[NP][2 * VC];
 #pragma unroll
     for (int i = 0; i < NP; ++i) {
-      const int p = warp + i * AT_WARPS;
+      const int p = warp + i * WARPS;
       const bool sink = sinks && p < n_pairs;
       m[i] = sink ? sinks[kvh * G + g0 + (p % gs)] : -INFINITY;
       l[i] = sink ? 1.f : 0.f;
@@ -353,7 +353,7 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attn_paged_simt_vec_kernel(
         const ulonglong2 k4 = *reinterpret_cast<const ulonglong2*>(kv + c);
 #pragma unroll
         for (int i = 0; i < NP; ++i) {
-          const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(Qs + (warp + i * AT_WARPS) * d + c);
+          const ulonglong2 q4 = *reinterpret_cast<const ulonglong2*>(Qs + (warp + i * WARPS) * d + c);
           acc[i] = f2_fma(q4.x, k4.x, acc[i]);
           acc[i] = f2_fma(q4.y, k4.y, acc[i]);
         }
@@ -361,7 +361,7 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attn_paged_simt_vec_kernel(
       float s[NP], top[NP], alpha[NP];
 #pragma unroll
       for (int i = 0; i < NP; ++i) {
-        const int p = warp + i * AT_WARPS, tq = p / gs, pos = pos_lo + tq;
+        const int p = warp + i * WARPS, tq = p / gs, pos = pos_lo + tq;
         const int lo = nhv_first_key(pos, window, chunk);
         float even, odd;
         f2_unpack(acc[i], even, odd);
@@ -424,7 +424,7 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attn_paged_simt_vec_kernel(
     }
 #pragma unroll
     for (int i = 0; i < NP; ++i) {
-      const int p = warp + i * AT_WARPS;
+      const int p = warp + i * WARPS;
       if (p >= n_pairs) break;
       const int tq = p / gs, g = p - tq * gs;
       const size_t tok = (size_t)cu_q[seq] + t0 + tq;
@@ -443,10 +443,10 @@ __global__ void __launch_bounds__(AT_WARPS * 32) attn_paged_simt_vec_kernel(
     }
   };
   // the same for all warps of the block (the loop over the chunks has barriers)
-  const int most = (n_pairs + AT_WARPS - 1) / AT_WARPS;
+  const int most = (n_pairs + WARPS - 1) / WARPS;
   if (most <= 1) work(std::integral_constant<int, 1>());
-  else if (most <= 4) work(std::integral_constant<int, 4>());
-  else work(std::integral_constant<int, AV_PAIRS>());
+  else if (most <= 4 && AV_BLOCK / WARPS > 4) work(std::integral_constant<int, 4>());
+  else work(std::integral_constant<int, AV_BLOCK / WARPS>());
 }
 
 // max_tiles: an upper bound on sum over requests of ceil(new tokens / TQ); the caller may pass
@@ -470,17 +470,26 @@ NHV_API int nhv_attention_simt_ex(int dtype, const void* q, int q_stride, void* 
   const uintptr_t four = dtype == NHV_F32 ? 16 : 8;
   if (d % 4 == 0 && dv % 4 == 0 && d <= 256 && dv <= 256 && row % 4 == 0 && q_stride % 4 == 0 && (uintptr_t)q % four == 0 &&
       (uintptr_t)kv_pages % four == 0) {
-    const int most = AV_PAIRS * AT_WARPS, GS = G < 8 ? G : 8, TQ = most / GS, stages = dtype == NHV_F32 ? 2 : 1;
+    const int most = AV_BLOCK, GS = G < 8 ? G : 8, TQ = most / GS, stages = dtype == NHV_F32 ? 2 : 1;
     const size_t smem = ((size_t)stages * AT_CHUNK * (d + 4 + (planes == 2 ? dv : 0)) + (size_t)most * (d + AT_CHUNK)) * 4;
     const int most_smem = (stages * AT_CHUNK * (256 + 4 + 256) + most * (256 + AT_CHUNK)) * 4;
     const dim3 grid(n_tokens / TQ + n_seqs, nkv, (G + GS - 1) / GS);
-#define LAUNCH_VEC(T, VC)                                                                                           \
+    // portions of a prompt: the block's 32 pairs over eight warps, so that one waits while another works (16 heads over 8 of 128 in
+    // fp32, prompts of 37, 123 and 210 tokens: 72 us with four warps of 8 pairs, 58 with eight of 4); few pairs a block (single
+    // tokens): four
+    const bool many = n_tokens >= 4 * n_seqs;
+#define LAUNCH_WARPS(T, VC, WARPS)                                                                                  \
   do {                                                                                                              \
     static std::atomic<uint64_t> done{0};                                                                           \
-    NHV_CUDA(nhv_allow_smem((const void*)attn_paged_simt_vec_kernel<T, VC>, most_smem, done), "attention");         \
-    nhv_launch(attn_paged_simt_vec_kernel<T, VC>, grid, AT_WARPS * 32, smem, stream, (const T*)q, q_stride, (T*)out, \
+    NHV_CUDA(nhv_allow_smem((const void*)attn_paged_simt_vec_kernel<T, VC, WARPS>, most_smem, done), "attention");  \
+    nhv_launch(attn_paged_simt_vec_kernel<T, VC, WARPS>, grid, WARPS * 32, smem, stream, (const T*)q, q_stride, (T*)out, \
                out_stride, (const T*)kv_pages, block_table, bt_stride, cu_q, kv_len, n_seqs, nq, nkv, d, page_size,  \
                n_pages, window, scale, TQ, GS, dv, row, sinks, chunk, slopes, planes, keep_first, softcap);          \
+  } while (0)
+#define LAUNCH_VEC(T, VC)                  \
+  do {                                     \
+    if (many) LAUNCH_WARPS(T, VC, 8);      \
+    else LAUNCH_WARPS(T, VC, 4);           \
   } while (0)
     if (dtype == NHV_F32 && dv <= 128) LAUNCH_VEC(float, 1);
     else if (dtype == NHV_F32) LAUNCH_VEC(float, 2);
@@ -488,6 +497,7 @@ NHV_API int nhv_attention_simt_ex(int dtype, const void* q, int q_stride, void* 
     else if (dtype == NHV_BF16) LAUNCH_VEC(__nv_bfloat16, 2);
     else NHV_REQUIRE(false, "attention: unknown dtype %d", dtype);
 #undef LAUNCH_VEC
+#undef LAUNCH_WARPS
     NHV_CHECK_LAUNCH("attention");
     return 0;
   }
