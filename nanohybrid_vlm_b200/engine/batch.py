@@ -11,6 +11,7 @@ is written into ONE pinned host buffer and crosses to the device in one copy.
 """
 from __future__ import annotations
 
+from array import array
 from dataclasses import dataclass, field
 
 import numpy as np
@@ -67,6 +68,16 @@ class StepBatch:
     carried: dict = field(default_factory=dict)
 
 
+def _int32(tokens):
+    """A list of whole numbers as 32-bit ones, a third faster than by numpy; anything else as it is."""
+    if type(tokens) is list:
+        try:
+            return np.frombuffer(array("i", tokens), dtype=np.int32)
+        except TypeError:
+            pass
+    return tokens
+
+
 def _align(n: int, a: int = 4) -> int:
     return (n + a - 1) // a * a
 
@@ -84,6 +95,7 @@ class BatchBuilder:
         self._layouts: dict = {}
         self._table_rows = None          # (layout, per row (request, table length)) of the last all-decode step
         self._windows = any(g.gives_back for g in cache_manager.groups)
+        self._iota = np.arange(max(max_pages_per_seq * self.page_size, max_seqs) + 1, dtype=np.int32)
         cap = self._layout(max_tokens, max_seqs, max_tokens, max_pages_per_seq)[1]
         self._host = torch.empty(cap, dtype=torch.int32, pin_memory=self.device.type == "cuda")
         self._np = self._host.numpy()
@@ -110,6 +122,24 @@ class BatchBuilder:
             off += _align(S * width)
         self._layouts[key] = (sections, off)
         return sections, off
+
+    def _fill_slots(self, out, table, start: int, end: int) -> None:
+        """out[i] = page * page size + offset of token start + i (-1 where the table has no page), up to token ``end``."""
+        ps = self.page_size
+        first, last = start // ps, (end - 1) // ps
+        if last - first < 64:
+            # page by page: an addition each, where quotients and remainders of every position took 45 us for 4,096 tokens
+            for lp in range(first, last + 1):
+                a, b = max(start, lp * ps), min(end, (lp + 1) * ps)
+                page = table[lp]
+                if page >= 0:
+                    np.add(self._iota[a - lp * ps:b - lp * ps], page * ps, out=out[a - start:b - start])
+                else:
+                    out[a - start:b - start] = -1
+        else:
+            p = self._iota[start:end]
+            pages = np.asarray(table, dtype=np.int32)[p // ps]
+            out[:] = np.where(pages >= 0, pages * ps + p % ps, -1)
 
     def build(self, items: list[StepItem], table_width: int | None = None, sampling=None,
               pad_to: int | None = None, views: bool = True, feed: list[int] | None = None) -> StepBatch | None:
@@ -200,12 +230,15 @@ class BatchBuilder:
             tok[:n], qs[:n], st[:n] = firsts, starts, slots_state
             pos_axes[:, :n] = starts
             kvl[:n] = qs[:n] + 1
-            cu[1:n + 1] = np.arange(1, n + 1, dtype=np.int32)
+            cu[1:n + 1] = self._iota[1:n + 1]
             rows[:n] = cu[:n]
             t = r = n
             items_loop = ()
         else:
             items_loop = items
+        # several requests that bring more than a token: their tokens, positions and slots as whole arrays behind the loop
+        together = len(items_loop) >= 8 and all(it.positions is None and type(it.tokens) is list for it in items_loop)
+        flat = []
         for s, it in enumerate(items_loop):
             n = len(it.tokens)
             if n == 0:
@@ -229,7 +262,13 @@ class BatchBuilder:
                     raise ValueError(f"request {it.req_id!r}: positions must be {n} numbers, or {self.n_axes} lists of "
                                      f"{n}, none negative")
                 pos_axes[:, t:t + n] = given
-            if n == 1:
+            if together:
+                flat += it.tokens
+                for g in range(self.n_groups):
+                    table = self.cm.block_table(it.req_id, g)
+                    k = min(len(table), width)
+                    table_views[g][s, :k] = table[:k]
+            elif n == 1:
                 # a decoded token: scalars instead of arrays (this is the hot path of every decode step)
                 tok[t] = it.tokens[0]
                 if it.positions is None:
@@ -241,16 +280,25 @@ class BatchBuilder:
                     page = table[it.start // ps]
                     slot_views[g][t] = page * ps + it.start % ps if page >= 0 else -1
             else:
-                tok[t:t + n] = it.tokens
-                p = np.arange(it.start, end, dtype=np.int32)
+                tok[t:t + n] = _int32(it.tokens)
                 if it.positions is None:
-                    pos_axes[:, t:t + n] = p
+                    pos_axes[:, t:t + n] = self._iota[it.start:end]
                 for g in range(self.n_groups):
-                    table = np.asarray(self.cm.block_table(it.req_id, g), dtype=np.int32)
-                    table_views[g][s, :min(len(table), width)] = table[:width]
-                    pages = table[p // ps]
-                    slot_views[g][t:t + n] = np.where(pages >= 0, pages * ps + p % ps, -1)
+                    table = self.cm.block_table(it.req_id, g)
+                    k = min(len(table), width)
+                    table_views[g][s, :k] = table[:k]
+                    self._fill_slots(slot_views[g][t:t + n], table, it.start, end)
             t += n
+        if together:
+            tok[:t] = _int32(flat)
+            lens = np.diff(cu[:n_real + 1])
+            pos = np.arange(t, dtype=np.int32) - np.repeat(cu[:n_real] - qs[:n_real], lens)
+            pos_axes[:, :t] = pos
+            lp, off = (pos // ps, pos % ps) if ps & (ps - 1) else (pos >> (ps.bit_length() - 1), pos & (ps - 1))
+            request = np.repeat(self._iota[:n_real], lens)
+            for g in range(self.n_groups):
+                pages = table_views[g][request, lp]
+                slot_views[g][:t] = np.where(pages >= 0, pages * ps + off, -1)
         for s in range(n_real, S):          # idle entries
             if keep and old_rows[s] is not None:
                 for tv in table_views:
@@ -286,9 +334,14 @@ class BatchBuilder:
         if not views:           # a replayed graph reads the arrays where they lie; nobody needs the views
             return None
 
-        def dev(name):
-            o, n = sec[name]
-            return self._dev[o:o + n]
+        # all views in one call: section, the rest up to its alignment, the next section, ...
+        sizes, at = [], 0
+        for o, n in sec.values():
+            sizes += [o - at, n]
+            at = o + n
+        pieces = self._dev[:at].split(sizes)
+        views_by_name = dict(zip(sec, pieces[1::2]))
+        dev = views_by_name.__getitem__
 
         groups = [GroupTables(dev(f"tables{g}").view(S, width), dev(f"slots{g}")) for g in range(self.n_groups)]
         lens = [len(it.tokens) for it in items] + [1] * pad
@@ -301,7 +354,7 @@ class BatchBuilder:
             n_tokens=T, n_seqs=S, n_logit_rows=R, token_ids=dev("token_ids"), positions=dev("positions")[:T],
             position_axes=dev("positions").view(self.n_axes, T),
             cu_q=dev("cu_q"), kv_len=dev("kv_len"), q_start=dev("q_start"), state_slots=dev("state_slots"),
-            logit_rows=dev("logit_rows"), groups=groups, host_cu_q=[int(x) for x in cu[:S + 1]],
+            logit_rows=dev("logit_rows"), groups=groups, host_cu_q=cu[:S + 1].tolist(),
             host_kv_len=ends, max_new_tokens=max(lens),
             max_kv_len=max(ends) if pad_to is None else width * ps, decode_only=max(lens) == 1,
             n_decode_seqs=sum(1 for n in lens if n == 1), n_prefill_seqs=sum(1 for n in lens if n > 1),
