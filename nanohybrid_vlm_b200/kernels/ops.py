@@ -43,8 +43,15 @@ def _ptr(t):
     return None if t is None else t.data_ptr()
 
 
-def stream_ptr() -> int:
-    return torch.cuda.current_stream().cuda_stream
+try:                # the current stream's handle without an object around it: 0.3 us instead of 4 for every launch
+    from torch._C import _cuda_getCurrentRawStream, _cuda_getDevice
+
+    def stream_ptr() -> int:
+        return _cuda_getCurrentRawStream(_cuda_getDevice())
+except ImportError:
+
+    def stream_ptr() -> int:
+        return torch.cuda.current_stream().cuda_stream
 
 
 def embed(out: torch.Tensor, table: torch.Tensor, ids: torch.Tensor) -> None:
