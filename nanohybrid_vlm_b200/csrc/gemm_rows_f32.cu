@@ -2,6 +2,9 @@
 // enter a recurrence or a gate in 32-bit (a handful of rows of w, a step of a few tokens).  One warp per output:
 // the lanes walk K in 16-byte pieces, sum in fp32 in a fixed order and meet in a shuffle tree, so an output does
 // not depend on what else is in the batch.  Large M goes to the library product instead (the caller decides).
+// Bound by latency (a step's x and these rows are a few hundred kilobytes): a warp asks for eight pieces of its row of w before it
+// waits for the kernel before, and for eight pieces of x at once (read piece by piece behind the wait, a launch added 3.7 to 4.1 us to a
+// step of 8 and of 48 rows).
 #include "nhv_common.cuh"
 
 constexpr int GR_WARPS = 4;
@@ -10,23 +13,38 @@ __global__ void __launch_bounds__(GR_WARPS * 32) gemm_rows_f32_kernel(float* __r
                                                                        const __nv_bfloat16* __restrict__ x, int x_stride,
                                                                        const __nv_bfloat16* __restrict__ w, int w_stride,
                                                                        int M, int N, int K) {
-  pdl_prologue();
+  constexpr int AHEAD = 8;                                // pieces of a row on their way at once: 2,048 columns
+  pdl_launch_dependents();
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const long item = (long)blockIdx.x * GR_WARPS + warp;
-  if (item >= (long)M * N) return;
-  const int m = (int)(item / N), n = (int)(item - (long)m * N);
+  const bool there = item < (long)M * N;
+  const int m = there ? (int)(item / N) : 0, n = there ? (int)(item - (long)m * N) : 0, pieces = K >> 3;
   const uint4* xr = reinterpret_cast<const uint4*>(x + (size_t)m * x_stride);
   const uint4* wr = reinterpret_cast<const uint4*>(w + (size_t)n * w_stride);
-  float acc[4] = {0.f, 0.f, 0.f, 0.f};
-  for (int c = lane; c < (K >> 3); c += 32) {
-    const uint4 a = xr[c], b = wr[c];
-    const __nv_bfloat162* ap = reinterpret_cast<const __nv_bfloat162*>(&a);
-    const __nv_bfloat162* bp = reinterpret_cast<const __nv_bfloat162*>(&b);
+  const uint4 zero = make_uint4(0, 0, 0, 0);
+  uint4 a[AHEAD], b[AHEAD];
 #pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const float2 fa = __bfloat1622float2(ap[e]), fb = __bfloat1622float2(bp[e]);
-      acc[e] = fmaf(fa.x, fb.x, acc[e]);
-      acc[e] = fmaf(fa.y, fb.y, acc[e]);
+  for (int i = 0; i < AHEAD; ++i) b[i] = lane + 32 * i < pieces ? wr[lane + 32 * i] : zero;
+  pdl_wait();
+  if (!there) return;
+  float acc[4] = {0.f, 0.f, 0.f, 0.f};
+  for (int c0 = lane; c0 < pieces; c0 += 32 * AHEAD) {
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i) a[i] = c0 + 32 * i < pieces ? xr[c0 + 32 * i] : zero;
+    if (c0 != lane)
+#pragma unroll
+      for (int i = 0; i < AHEAD; ++i) b[i] = c0 + 32 * i < pieces ? wr[c0 + 32 * i] : zero;
+#pragma unroll
+    for (int i = 0; i < AHEAD; ++i) {
+      if (c0 + 32 * i >= pieces) break;
+      const __nv_bfloat162* ap = reinterpret_cast<const __nv_bfloat162*>(&a[i]);
+      const __nv_bfloat162* bp = reinterpret_cast<const __nv_bfloat162*>(&b[i]);
+#pragma unroll
+      for (int e = 0; e < 4; ++e) {
+        const float2 fa = __bfloat1622float2(ap[e]), fb = __bfloat1622float2(bp[e]);
+        acc[e] = fmaf(fa.x, fb.x, acc[e]);
+        acc[e] = fmaf(fa.y, fb.y, acc[e]);
+      }
     }
   }
   const float sum = warp_sum((acc[0] + acc[1]) + (acc[2] + acc[3]));
