@@ -3,8 +3,8 @@
 // the lanes walk K in 16-byte pieces, sum in fp32 in a fixed order and meet in a shuffle tree, so an output does
 // not depend on what else is in the batch.  Large M goes to the library product instead (the caller decides).
 // Bound by latency (a step's x and these rows are a few hundred kilobytes): a warp asks for eight pieces of its row of w before it
-// waits for the kernel before, and for eight pieces of x at once (read piece by piece behind the wait, a launch added 3.7 to 4.1 us to a
-// step of 8 and of 48 rows).
+// waits for the kernel before, and for eight pieces of x at once (read piece by piece behind the wait, a launch added 3.8 and 4.1 us to a
+// step of 8 and of 48 rows; 2.0 and 2.4 now).
 #include "nhv_common.cuh"
 
 constexpr int GR_WARPS = 4;

@@ -43,7 +43,7 @@ def _ptr(t):
     return None if t is None else t.data_ptr()
 
 
-try:                # the current stream's handle without an object around it: 0.3 us instead of 4 for every launch
+try:                # the current stream's handle without an object around it: 0.2 us instead of 3.2 for every launch
     from torch._C import _cuda_getCurrentRawStream, _cuda_getDevice
 
     def stream_ptr() -> int:
