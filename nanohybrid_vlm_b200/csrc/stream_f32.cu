@@ -98,16 +98,20 @@ __global__ void rmsnorm_stream_kernel(T* __restrict__ out, const T* __restrict__
 
 // The same with eight consecutive columns a thread, held in registers: a row is width / 8 threads, a part of it a whole number
 // of warps.  Bound by memory for prompts and by latency for a step of a few rows, so: everything a thread needs is asked for at
-// once, the weight before the wait for the kernels before, and one barrier.  2,048 columns, what a launch adds to a step: 8 rows with two
-// addends 7.2 (the kernel above) and 3.2 us, 4,096 rows 32 and 17 (107 MB: 6.3 TB/s).
+// once, the weight before the wait for the kernels before, and two barriers.  The squares are added in the order of the kernel
+// above (`chains` warps of it, each lane every `stride`-th column from its own on), through shared memory: so a row's bits do not
+// depend on which of the two takes it, and a model's outputs in 16 bits, which a last bit of a norm can tip, are the same.
+// FIGURES
 template <typename T, int ADDENDS>
-__global__ void __launch_bounds__(1024) rmsnorm_stream_vec_kernel(T* __restrict__ out, const T* __restrict__ a0, const T* __restrict__ a1,
+__global__ void __launch_bounds__(1024, 1) rmsnorm_stream_vec_kernel(T* __restrict__ out, const T* __restrict__ a0, const T* __restrict__ a1,
                                                                   const T* __restrict__ a2, float c0, float c1, float c2,
                                                                   float* __restrict__ stream, const T* __restrict__ w,
                                                                   const int* __restrict__ rows, int width, float eps,
-                                                                  int write_stream, float weight_offset, int part_warps) {
+                                                                  int write_stream, float weight_offset, int groups, int chains,
+                                                                  int stride) {
+  extern __shared__ __align__(16) float row[];
   __shared__ float red[32];
-  const int r = blockIdx.x, c = threadIdx.x * 8, warp = threadIdx.x >> 5;
+  const int r = blockIdx.x, c = threadIdx.x * 8, warp = threadIdx.x >> 5, lane = threadIdx.x & 31, part = width / groups;
   float wv[8], s[8], a[8], b[8], e[8];
   nhv_load8(wv, w + c);
   pdl_prologue();
@@ -116,7 +120,6 @@ __global__ void __launch_bounds__(1024) rmsnorm_stream_vec_kernel(T* __restrict_
   if (ADDENDS > 0) nhv_load8(a, a0 + src);
   if (ADDENDS > 1) nhv_load8(b, a1 + src);
   if (ADDENDS > 2) nhv_load8(e, a2 + src);
-  float ss = 0.f;
 #pragma unroll
   for (int i = 0; i < 8; ++i) {
     if (ADDENDS > 0) {
@@ -125,16 +128,21 @@ __global__ void __launch_bounds__(1024) rmsnorm_stream_vec_kernel(T* __restrict_
       if (ADDENDS > 2) add = fmaf(c2, e[i], add);
       s[i] += add;
     }
-    ss = fmaf(s[i], s[i], ss);
   }
+  nhv_store8(row + c, s);
   if (ADDENDS > 0 && write_stream) nhv_store8(stream + src, s);
-  ss = warp_sum(ss);
-  if ((threadIdx.x & 31) == 0) red[warp] = ss;
   __syncthreads();
-  const int first = warp / part_warps * part_warps;
-  float total = red[first];
-  for (int i = 1; i < part_warps; ++i) total += red[first + i];
-  const float rstd = 1.0f / sqrtf(total / (float)(part_warps * 256) + eps);
+  for (int i = warp; i < chains; i += (int)(blockDim.x >> 5)) {
+    const int first = groups > 1 ? i * part : i * 32, end = groups > 1 ? first + part : width;
+    float ss = 0.f;
+#pragma unroll 8
+    for (int k = first + lane; k < end; k += stride) ss = fmaf(row[k], row[k], ss);
+    ss = warp_sum(ss);
+    if (lane == 0) red[i] = ss;
+  }
+  __syncthreads();
+  const float total = groups > 1 ? red[c / part] : warp_sum(lane < chains ? red[lane] : 0.f);
+  const float rstd = 1.0f / sqrtf(total / (float)part + eps);
 #pragma unroll
   for (int i = 0; i < 8; ++i) s[i] = s[i] * rstd * (wv[i] + weight_offset);
   nhv_store8(out + (size_t)r * width + c, s);
@@ -149,10 +157,14 @@ NHV_API int nhv_rmsnorm_stream(int dtype, void* out, const void* a0, const void*
   NHV_REQUIRE((a0 || !a1) && (a1 || !a2), "rmsnorm_stream: addends are given in order");
   NHV_REQUIRE(!(rows && write_stream), "rmsnorm_stream: a gathered norm cannot write the stream back");
   const uintptr_t at = (uintptr_t)out | (uintptr_t)a0 | (uintptr_t)a1 | (uintptr_t)a2 | (uintptr_t)stream_rows | (uintptr_t)w;
+  const size_t smem = (size_t)width * sizeof(float);
+  int threads = 32;                                       // of the kernel that takes a column at a time
+  while (threads < 512 && threads * 4 < width) threads <<= 1;
   if (width % (groups * 256) == 0 && width <= 8192 && at % 16 == 0) {
+    const int chains = groups > 1 ? groups : threads / 32, stride = groups > 1 ? 32 : threads;
 #define VEC(T, A)                                                                                                  \
-  nhv_launch(rmsnorm_stream_vec_kernel<T, A>, n_rows, width / 8, 0, stream, (T*)out, (const T*)a0, (const T*)a1,   \
-             (const T*)a2, c0, c1, c2, stream_rows, (const T*)w, rows, width, eps, write_stream, weight_offset, width / groups / 256)
+  nhv_launch(rmsnorm_stream_vec_kernel<T, A>, n_rows, width / 8, smem, stream, (T*)out, (const T*)a0, (const T*)a1, \
+             (const T*)a2, c0, c1, c2, stream_rows, (const T*)w, rows, width, eps, write_stream, weight_offset, groups, chains, stride)
 #define BY_ADDENDS(T)         \
   do {                        \
     if (a2) VEC(T, 3);        \
@@ -168,10 +180,7 @@ NHV_API int nhv_rmsnorm_stream(int dtype, void* out, const void* a0, const void*
     NHV_CHECK_LAUNCH("rmsnorm_stream");
     return 0;
   }
-  const size_t smem = (size_t)width * sizeof(float);
   NHV_REQUIRE(smem <= 200 * 1024, "rmsnorm_stream: width %d is beyond the %d floats a row buffer holds", width, 200 * 1024 / 4);
-  int threads = 32;
-  while (threads < 512 && threads * 4 < width) threads <<= 1;
 #define LAUNCH(T)                                                                                               \
   do {                                                                                                          \
     if (smem > 48 * 1024)                                                                                       \

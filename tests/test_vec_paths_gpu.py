@@ -144,3 +144,62 @@ def test_filter_add_has_the_same_bits_in_long_and_short_steps(ops, dtype, C, K, 
         seen.append([torch.cat(p) for p in got] + ([state] if K > 1 else []))
     for a, b in zip(*seen):
         assert torch.equal(a, b)
+
+
+def off_by_one(t):
+    """The same values, contiguous, one element behind a boundary of 16 bytes."""
+    room = torch.empty(t.numel() + 1, dtype=t.dtype, device=t.device)
+    room[1:] = t.reshape(-1)
+    return room[1:].view(t.shape)
+
+
+# a warp a row; parts of one and of several warps; odd numbers of warps; the widest row of the vector form, and wider
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("width,groups", [(256, 1), (512, 2), (768, 1), (1280, 5), (2048, 1), (2048, 4), (4096, 2), (8192, 1), (8448, 1)])
+@pytest.mark.parametrize("n_addends", [0, 1, 2, 3])
+def test_norm_over_the_stream(ops, dtype, width, groups, n_addends):
+    """Against 64 bits, and the bits of the form that takes a column at a time: a norm's last bit can tip what follows in 16 bits."""
+    g = torch.Generator().manual_seed(width + n_addends)
+    T, coefs = 5, (0.7, -1.25, 2.0)
+    stream = torch.randn(T, width, generator=g) * 3
+    stream[:, :width // groups] *= 50                       # one loud part must not quieten the others
+    adds = [torch.randn(T, width, generator=g).to(dtype) for _ in range(n_addends)]
+    w = (1 + 0.2 * torch.randn(width, generator=g)).to(dtype)
+    want_stream = stream.to(F64) + sum(c * a.to(F64) for c, a in zip(coefs, adds))
+    parts = want_stream.view(T, groups, -1)
+    want = (parts / (parts.square().mean(-1, keepdim=True) + 1e-5).sqrt()).view(T, width) * (w.to(F64) + 0.5)
+    for rows in (None, torch.tensor([4, 0, 2], dtype=torch.int32)):
+        pick, seen = slice(None) if rows is None else rows.long(), []
+        for place in (lambda t: t, off_by_one):
+            s, out = place(dev(stream)), place(torch.full((T if rows is None else 3, width), float("nan"), dtype=dtype, device="cuda"))
+            ops.rmsnorm_stream(out, s, place(dev(w)), 1e-5, [(place(dev(a)), c) for a, c in zip(adds, coefs)],
+                               rows=None if rows is None else dev(rows), weight_offset=0.5, groups=groups)
+            torch.testing.assert_close(out.cpu().to(F64), want[pick], **tol(dtype))
+            torch.testing.assert_close(s.cpu().to(F64), want_stream if rows is None else stream.to(F64), rtol=1e-6, atol=1e-4)
+            seen.append((out.cpu(), s.cpu()))
+        assert torch.equal(seen[0][0], seen[1][0]) and torch.equal(seen[0][1], seen[1][1])
+
+
+# one block across with idle threads, a last block in part, two whole blocks; more rows than blocks down
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("width,T", [(96, 9), (1028, 9), (2048, 3), (512, 1200), (1536, 700)])
+def test_dyntanh_over_the_stream(ops, dtype, width, T):
+    g = torch.Generator().manual_seed(width)
+    pre, post = ([dev(t.to(dtype)) for t in (0.3 + torch.rand(1, generator=g), 1 + 0.3 * torch.randn(width, generator=g),
+                                             0.3 * torch.randn(width, generator=g))] for _ in range(2))
+    stream, a = torch.randn(T, width, generator=g) * 2, torch.randn(T, width, generator=g).to(dtype)
+    rows = torch.randperm(T, generator=g)[:max(1, T - 1)].int()
+    f = lambda x, p: torch.tanh(p[0].cpu().to(F64) * x.to(F64)) * p[1].cpu().to(F64) + p[2].cpu().to(F64)     # noqa: E731
+    for addend, norm in ((None, None), (a, None), (a, post)):
+        for gather in (None, rows):
+            pick, seen = slice(None) if gather is None else gather.long(), []
+            want_stream = stream.to(F64) + (0 if addend is None else addend.to(F64) if norm is None else f(addend, norm))
+            for place in (lambda t: t, off_by_one):
+                s, out = place(dev(stream)), place(torch.full((T if gather is None else len(gather), width), float("nan"), dtype=dtype, device="cuda"))
+                ops.dyntanh_stream(out, s, tuple(pre), None if addend is None else place(dev(addend)), None if norm is None else tuple(norm),
+                                   rows=None if gather is None else dev(gather), write_stream=gather is None)
+                torch.testing.assert_close(out.cpu().to(F64), f(want_stream, pre)[pick], **tol(dtype))
+                kept = want_stream if gather is None else stream.to(F64)
+                torch.testing.assert_close(s.cpu().to(F64), kept, **tol(torch.float32))
+                seen.append((out.cpu(), s.cpu()))
+            assert torch.equal(seen[0][0], seen[1][0]) and torch.equal(seen[0][1], seen[1][1])
