@@ -123,6 +123,10 @@ class BatchBuilder:
         self._layouts[key] = (sections, off)
         return sections, off
 
+    def _positions(self, start: int, end: int):
+        """The whole numbers from start up to end (a caller's own table width may be less than a request's tokens need)."""
+        return self._iota[start:end] if end <= len(self._iota) else np.arange(start, end, dtype=np.int32)
+
     def _fill_slots(self, out, table, start: int, end: int) -> None:
         """out[i] = page * page size + offset of token start + i (-1 where the table has no page), up to token ``end``."""
         ps = self.page_size
@@ -137,7 +141,7 @@ class BatchBuilder:
                 else:
                     out[a - start:b - start] = -1
         else:
-            p = self._iota[start:end]
+            p = self._positions(start, end)
             pages = np.asarray(table, dtype=np.int32)[p // ps]
             out[:] = np.where(pages >= 0, pages * ps + p % ps, -1)
 
@@ -237,7 +241,9 @@ class BatchBuilder:
         else:
             items_loop = items
         # several requests that bring more than a token: their tokens, positions and slots as whole arrays behind the loop
-        together = len(items_loop) >= 8 and all(it.positions is None and type(it.tokens) is list for it in items_loop)
+        # (the slots from the step's own tables, which must hold every token's page)
+        together = len(items_loop) >= 8 and all(it.positions is None and type(it.tokens) is list
+                                                and it.start + len(it.tokens) <= width * ps for it in items_loop)
         flat = []
         for s, it in enumerate(items_loop):
             n = len(it.tokens)
@@ -282,7 +288,7 @@ class BatchBuilder:
             else:
                 tok[t:t + n] = _int32(it.tokens)
                 if it.positions is None:
-                    pos_axes[:, t:t + n] = self._iota[it.start:end]
+                    pos_axes[:, t:t + n] = self._positions(it.start, end)
                 for g in range(self.n_groups):
                     table = self.cm.block_table(it.req_id, g)
                     k = min(len(table), width)

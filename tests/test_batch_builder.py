@@ -155,3 +155,16 @@ def test_random_runs_of_steps(seed, windowed):
             for x in ok:
                 cm.release_behind_window(x, held[x])
         cm.check()
+
+
+@pytest.mark.parametrize("n", [3, 9])
+def test_tables_narrower_than_the_requests_that_the_caller_asked_for(n):
+    """The tables hold their first columns; positions and slots are the manager's all the same."""
+    cm = CacheManager([GroupSpec(None)], 4, 500)
+    b = BatchBuilder(cm, VOCAB, "cpu", max_tokens=900, max_seqs=16, max_pages_per_seq=4)
+    items = []
+    for r in range(n):
+        k = (22, 9, 300)[r % 3] if r < 3 else 9             # more than four pages; more than 64 pages
+        cm.allocate(r, k)
+        items.append(StepItem(r, [(r + i) % VOCAB for i in range(k)], 0, [k - 1]))
+    check_against_manager(cm, b, items, b.build(items, table_width=2))
