@@ -168,3 +168,32 @@ def test_tables_narrower_than_the_requests_that_the_caller_asked_for(n):
         cm.allocate(r, k)
         items.append(StepItem(r, [(r + i) % VOCAB for i in range(k)], 0, [k - 1]))
     check_against_manager(cm, b, items, b.build(items, table_width=2))
+
+
+@pytest.mark.parametrize("page_size,window", [(1, None), (3, 7), (4, None), (16, 20), (5, 6)])
+def test_steps_of_many_requests(page_size, window):
+    """Eight and more requests that bring portions and single tokens (whole arrays for the step), page sizes on and off the
+    powers of two, pages given back behind a window; a portion of more than 64 pages by itself and in company."""
+    rng = random.Random(page_size)
+    cm = CacheManager([GroupSpec(None), GroupSpec(window)] if window else [GroupSpec(None)], page_size, 4000)
+    b = BatchBuilder(cm, VOCAB, "cpu", max_tokens=2000, max_seqs=16, max_pages_per_seq=1200 // page_size + 1)
+    held = {r: 0 for r in range(14)}
+    for step in range(30):
+        who = rng.sample(sorted(held), rng.choice([1, 7, 8, 9, 14]))
+        items = []
+        for r in who:
+            n = rng.choice([1, 1, 2, page_size, page_size + 1, rng.randint(1, 40)])
+            if r == who[0] and step % 5 == 0:
+                n = 70 * page_size + rng.randint(0, 3)      # (at five a page: the division; at sixteen: across many pages)
+            if held[r] + n > 1200 or sum(len(it.tokens) for it in items) + n > 1990:
+                n = 1
+            if held[r] + n > 1200:
+                cm.free(r)
+                held[r] = 0
+            cm.allocate(r, held[r] + n)
+            items.append(StepItem(r, [rng.randrange(VOCAB) for _ in range(n)], held[r], [n - 1] if rng.random() < 0.7 else []))
+        check_against_manager(cm, b, items, b.build(items))
+        for it in items:
+            held[it.req_id] += len(it.tokens)
+            cm.release_behind_window(it.req_id, held[it.req_id])
+    cm.check()
