@@ -1,6 +1,10 @@
 // C[M,N] = A[M,K] * W[N,K]^T in fp32 on the 5th-generation tensor cores (tcgen05.mma), with no less precision than fp32
-// multiply-adds: each operand is cut into three bfloat16 of eight bits, which hold it exactly, and a product is the six products
-// of their parts down to 2^-16 of the largest (what is left out is below 2^-24 of it and of either sign).
+// multiply-adds: each operand is cut into three bfloat16 of eight bits, which hold it exactly (7.7e-34 and more), and a product is
+// the six products of their parts down to 2^-16 of the largest (what is left out is below 2^-24 of it and of either sign).
+// Rows of smaller values, sums below 1.2e-35 and sums that are no finite number are multiplied again on the CUDA cores, by
+// themselves: infinities and the whole range of fp32 give what they give there.  Looking for them costs up to 3 % for 1 to 16 rows
+// (4096 x 1024 13.6 and 14.0 us, 43392 x 1024 66.2 and 68.9); a row is looked at until it shows a larger value, which
+// ordinary rows do at once.
 //
 // Sums.  The tensor cores cut off what lies below a sum's last place.  So the products of first parts are added up over 64
 // columns only (four MMAs) in tensor memory and then added to a sum in registers, rounded to the nearest; the five kinds of
@@ -20,8 +24,8 @@
 //
 // What bounds it: the way of a stage from global memory to its parts, about 2 us for 64 columns of both operands (1.1 where A
 // has up to 32 rows), beside 1,536 cycles of the tensor pipe, whose MMAs read all that shared memory gives.  In us, on the CUDA cores
-// and here, for 370 rows: N x K = 4096 x 1024 90 and 43, 1024 x 2048 70 and 23, 6144 x 1024 117 and 43, 1024 x 3072 103 and 31; for 16
-// rows 23 and 17, 43 and 17, 25 and 17, 64 and 21; 43392 x 1024, 3 and 20 rows: 66 and 70, 88 and 72.  Not faster: W two stages
+// and here, for 370 rows: N x K = 4096 x 1024 88 and 38, 1024 x 2048 159 and 20, 6144 x 1024 115 and 39, 1024 x 3072 238 and 26; for 16
+// rows 28 and 14, 42 and 14, 34 and 15, 62 and 19; 43392 x 1024, 3 and 33 rows: 65 and 69, 140 and 89.  Not faster: W two stages
 // ahead in registers with the MMAs issued by an adding warp (41 against 37 for 370 x 4096 x 1024 in one run).
 #define NHV_WAIT_LIMIT (1u << 22)
 #include "nhv_async.cuh"
@@ -103,8 +107,16 @@ __device__ __forceinline__ float4 cluster_load4(const float* mine, uint32_t rank
   return v;
 }
 
-// Eight floats as three times eight bfloat16 (16 bytes each): what is left, rounded to eight bits, three times.  Infinities and
-// values above bfloat16's largest (3.39e38) turn into values that are no number.
+__device__ __forceinline__ uint32_t cluster_load(const uint32_t* mine, uint32_t rank) {
+  uint32_t at, v;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;\n" : "=r"(at) : "r"(smem_u32(mine)), "r"(rank));
+  asm volatile("ld.shared::cluster.u32 %0, [%1];\n" : "=r"(v) : "r"(at) : "memory");
+  return v;
+}
+
+// Eight floats as three times eight bfloat16 (16 bytes each): what is left, rounded to eight bits, three times (above bfloat16's
+// largest, 3.39e38, the first part is that).  Exact down to 7.7e-34, below which the last bits are less than bfloat16's smallest
+// number; an infinity has a part that is no number.  What that leaves wrong is done again: `by_multiply_adds`.
 __device__ __forceinline__ void cut8(uint4 (&part)[3], const float (&x)[8]) {
   float v[8];
 #pragma unroll
@@ -114,12 +126,44 @@ __device__ __forceinline__ void cut8(uint4 (&part)[3], const float (&x)[8]) {
     uint32_t p[4];
 #pragma unroll
     for (int j = 0; j < 4; ++j) {
-      asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(p[j]) : "f"(v[2 * j + 1]), "f"(v[2 * j]));
+      if (i == 0) asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;\n" : "=r"(p[j]) : "f"(v[2 * j + 1]), "f"(v[2 * j]));
+      else asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(p[j]) : "f"(v[2 * j + 1]), "f"(v[2 * j]));
       v[2 * j] -= __uint_as_float(p[j] << 16);
       v[2 * j + 1] -= __uint_as_float(p[j] & 0xffff0000u);
     }
     part[i] = make_uint4(p[0], p[1], p[2], p[3]);
   }
+}
+
+// The largest of eight floats (what is no number does not count).
+__device__ __forceinline__ float largest_of8(const float (&x)[8]) {
+  float a, b;
+  asm("max.abs.f32 %0, %1, %2, %3;\n" : "=f"(a) : "f"(x[0]), "f"(x[1]), "f"(x[2]));
+  asm("max.abs.f32 %0, %1, %2, %3;\n" : "=f"(b) : "f"(x[3]), "f"(x[4]), "f"(x[5]));
+  asm("max.abs.f32 %0, %1, %2, %3;\n" : "=f"(a) : "f"(x[6]), "f"(x[7]), "f"(a));
+  return fmaxf(a, b);
+}
+constexpr float SMALL_ROW = 0x1p-101f, SMALL_SUM = 0x1p-116f;
+// Whether the tensor cores' sum is to be done again: no finite number, or so small that fp32's last place is 2^-149 (cut off there
+// in each step, K / 64 times over); not where it is zero.
+__device__ __forceinline__ bool doubtful(float v) {
+  const uint32_t size = __float_as_uint(v) & 0x7fffffffu, least = __float_as_uint(SMALL_SUM);
+  return size - least >= 0x7f800000u - least && size != 0;
+}
+
+// One value of C on the CUDA cores, as gemm_simt.cu adds it up.  For what the tensor cores cannot give: a sum that is `doubtful` (no
+// finite number: an operand is none, or some of the parts' products are beyond fp32's range, of either sign), and rows of A
+// or W whose largest value is below SMALL_ROW (their last bits are lost in bfloat16; beside a larger value in the row they
+// are below 2^-30 of it).
+__device__ __noinline__ float by_multiply_adds(const float* a, const float* w, int K) {
+  float even = 0.f, odd = 0.f;
+  for (int k = 0; k < K; k += 4) {
+    const float4 x = *reinterpret_cast<const float4*>(a + k), y = *reinterpret_cast<const float4*>(w + k);
+    even = fmaf(x.z, y.z, fmaf(x.x, y.x, even));
+    odd = fmaf(x.w, y.w, fmaf(x.y, y.y, odd));
+    if (isnan(even) || isnan(odd)) break;                        // stays one
+  }
+  return even + odd;
 }
 
 // Order of a stage's products: (part of W, part of A), the products of first parts by themselves
@@ -146,6 +190,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tcgen05_kernel(const Para
   uint64_t* small_full = sum_empty + 2;
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(small_full + 1);
   __shared__ int s_abort;
+  // rows of W, then of A: 1 where the run holds a value of SMALL_ROW or more, 256 where one that is not zero; whether a row is small
+  __shared__ uint32_t s_size[TILE + NT], s_small[TILE + NT];
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const uint32_t rank = p.split > 1 ? cluster_rank() : 0;
@@ -204,6 +250,23 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tcgen05_kernel(const Para
         }
       }
     };
+    // bits 0 to 3: this thread's rows of W that hold a value of SMALL_ROW or more, 4 to 7: of A; 8 to 15: any that is not zero.  Once a
+    // row has such a value in this thread's columns, mostly in the first stage, it is not looked at again.
+    constexpr unsigned W_ROWS = 0xf, A_ROWS = NT == 128 ? 0xf0 : 0x10;
+    unsigned sizes = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      if (n0 + r0 + 32 * i >= p.N) sizes |= 1u << i;
+      if (i < NT / 32 && m0 + r0 + 32 * i >= p.M) sizes |= 16u << i;
+    }
+    auto look = [&](const auto& v, unsigned bit) {
+#pragma unroll
+      for (int i = 0; i < (int)(sizeof(v) / sizeof(v[0])); ++i) {
+        const float top = largest_of8(v[i]);
+        if (top >= SMALL_ROW) sizes |= bit << i;
+        if (top > 0.f) sizes |= bit << (8 + i);
+      }
+    };
     auto put = [&](const auto& v, unsigned char* tiles, int part_bytes) {
 #pragma unroll
       for (int i = 0; i < (int)(sizeof(v) / sizeof(v[0])); ++i) {
@@ -229,13 +292,23 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tcgen05_kernel(const Para
       if (s >= STAGES && !mbar_wait(&empty[slot], (uint32_t)((s / STAGES) - 1) & 1, 1)) { s_abort = 1; break; }
       unsigned char* to = smem + (size_t)slot * STAGE_BYTES;
       hint(s + 4);
+      if ((sizes & W_ROWS) != W_ROWS) look(w, 1u);
       put(w, to, W_PART);
       if (s + 1 < stages) load(w, p.W, p.N, p.K, n0, s + 1);
+      if ((sizes & A_ROWS) != A_ROWS) look(a, 16u);
       put(a, to + 3 * W_PART, A_PART);
       if (s + 1 < stages) load(a, p.A, p.M, p.lda, m0, s + 1);
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(&full[slot]);
+    }
+#pragma unroll
+    for (int d = 1; d < 8; d <<= 1) sizes |= __shfl_xor_sync(0xffffffffu, sizes, d);
+    if (c == 0) {
+#pragma unroll
+      for (int i = 0; i < 4; ++i) s_size[r0 + 32 * i] = sizes >> i & 0x101;
+#pragma unroll
+      for (int i = 0; i < NT / 32; ++i) s_size[TILE + r0 + 32 * i] = sizes >> (4 + i) & 0x101;
     }
   } else if (warp == MMA_WARP) {
     // ------------------------------------------------------------------ MMA issuer
@@ -301,21 +374,35 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tcgen05_kernel(const Para
   }
   // ------------------------------------------------------------------ out: a lane holds a row of W, neighbours in a row of C
   __syncthreads();                                               // (the ring is free: the last MMAs have read it)
+  bool again = false;                                            // whether this thread has met a value that is to be done again
+  const int share = NT / p.split, first = (int)rank * share;     // each block of the cluster its share of the tile's rows
   if (p.split == 1) {
     if (adds && !s_abort && n0 + col < p.N)
 #pragma unroll
       for (int i = 0; i < PER; ++i)
-        if (m0 + row0 + i < p.M) p.C[(size_t)(m0 + row0 + i) * p.ldc + n0 + col] = acc[i];
+        if (m0 + row0 + i < p.M) {
+          p.C[(size_t)(m0 + row0 + i) * p.ldc + n0 + col] = acc[i];
+          again |= doubtful(acc[i]);
+        }
+    if (const int t = THREADS - 1 - (int)threadIdx.x; t < TILE + NT) {
+      s_small[t] = s_size[t] == 0x100;
+      again |= s_small[t] != 0;
+    }
   } else {
     float* tile = reinterpret_cast<float*>(smem);                // [rows of A][128 rows of W]
     if (adds)
 #pragma unroll
       for (int i = 0; i < PER; ++i) tile[(row0 + i) * TILE + col] = s_abort ? __int_as_float(0x7fc00000) : acc[i];
     cluster_sync();
-    // the runs in order; each block of the cluster its share of the tile's rows
-    const int share = NT / p.split;
+    if (const int t = THREADS - 1 - (int)threadIdx.x; t < TILE + NT) {      // (threads that have the least to do below)
+      uint32_t size = 0;
+      for (int q = 0; q < p.split; ++q) size |= cluster_load(&s_size[t], (uint32_t)q);
+      s_small[t] = size == 0x100;
+      again = s_small[t];
+    }
+    // the runs in order
     for (int e = threadIdx.x; e < share * (TILE / 4); e += THREADS) {
-      const int r = (int)rank * share + e / (TILE / 4), c = 4 * (e % (TILE / 4));
+      const int r = first + e / (TILE / 4), c = 4 * (e % (TILE / 4));
       if (m0 + r >= p.M || n0 + c >= p.N) continue;
       float4 sum = cluster_load4(tile + r * TILE + c, 0);
       for (int q = 1; q < p.split; ++q) {
@@ -326,10 +413,20 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tcgen05_kernel(const Para
       const float v[4] = {sum.x, sum.y, sum.z, sum.w};
 #pragma unroll
       for (int i = 0; i < 4; ++i)
-        if (n0 + c + i < p.N) at[i] = v[i];
+        if (n0 + c + i < p.N) {
+          at[i] = v[i];
+          again |= doubtful(v[i]);
+        }
     }
     cluster_sync();                                              // the others read in here
   }
+  if (__syncthreads_or(again) && !s_abort)                       // by the row's and the column's own values: any batch, the same bits
+    for (int e = threadIdx.x; e < share * TILE; e += THREADS) {
+      const int r = first + e / TILE, c = e % TILE, m = m0 + r, n = n0 + c;
+      if (m >= p.M || n >= p.N) continue;
+      float* at = p.C + (size_t)m * p.ldc + n;
+      if (s_small[c] || s_small[TILE + r] || doubtful(*at)) *at = by_multiply_adds(p.A + (size_t)m * p.lda, p.W + (size_t)n * p.K, p.K);
+    }
   if (s_abort) give_up_delay();
   tc_fence_after();
   if (warp == ALLOC_WARP) tmem_dealloc(tmem_base, tmem_cols(NT));

@@ -1359,8 +1359,9 @@ F32_ON_TENSOR_CORES = True      # tests switch it off to compare with the CUDA-c
 def _f32_on_tensor_cores(x, weight) -> bool:
     """Whether a float32 product runs on the tensor cores, operands cut into three bfloat16 (csrc/gemm_f32_tcgen05.cu).  By the
     weight's sizes alone, never by the number of tokens: so a token's result does not depend on what it is computed with.
-    In us on the CUDA cores / the tensor cores: a weight of 512 x 512 13 / 13 for 1 to 128 tokens and 35 / 19 for 2,048; 256 x 256 8 / 12 (the
-    line lies where launches of either cost the same); 4,096 x 1,024 23 / 17 for 16 tokens, 90 / 43 for 370."""
+    In us on the CUDA cores / the tensor cores: a weight of 512 x 512 12 / 9 for 1 to 16 tokens, 16 / 13 for 128 and 35 / 19 for 2,048;
+    256 x 256 8 / 12; 4,096 x 1,024 28 / 14 for 16 tokens, 88 / 38 for 370; 43,392 x 1,024 65 / 69 for 1 to 8 tokens, 140 / 89 for 33.
+    Infinities, and values and sums of any size, give what the CUDA cores give."""
     N, K = weight.shape
     return (F32_ON_TENSOR_CORES and N >= 512 and K >= 512 and K % 4 == 0 and x.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0
             and weight.data_ptr() % 16 == 0)

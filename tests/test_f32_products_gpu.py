@@ -75,3 +75,98 @@ def test_what_the_tensor_cores_do_not_take_goes_to_the_cuda_cores(ops):
         ops.linear(out, a, b)
         ops.linear_simt(simt, a, b)
         assert torch.equal(out, simt)
+
+
+def both(ops, x, w):
+    out, simt = (torch.full((x.shape[0], w.shape[0]), float("nan"), device="cuda") for _ in range(2))
+    assert ops._f32_on_tensor_cores(x, w)
+    ops.linear(out, x, w)
+    ops.linear_simt(simt, x, w)
+    ops.raise_wait_errors()
+    return out, simt
+
+
+def same(a, b):
+    """The same values: infinities with their sign, and what is no number in the same places."""
+    return torch.equal(a.isnan(), b.isnan()) and torch.equal(a[~a.isnan()], b[~b.isnan()])
+
+
+# one run of K and four; tiles of 32 and of 128 rows
+SHAPES = pytest.mark.parametrize("M,N,K", [(20, 6400, 516), (140, 6400, 516), (20, 700, 1092), (140, 700, 1092)])
+
+
+@SHAPES
+@pytest.mark.parametrize("scale", [1e-33, 1e-36, 1e-41])
+def test_rows_below_what_three_bfloat16_hold(ops, M, N, K, scale):
+    """Rows of either operand whose last bits are below bfloat16's smallest number, down to fp32's own last numbers: what fp32
+    multiply-adds give; the rows beside them keep their bits."""
+    x, w = operands(M, N, K)
+    clean, _ = both(ops, x, w)
+    x2, w2 = x.clone(), w.clone()
+    x2[[3, M - 1]] *= scale
+    w2[[0, N - 1]] *= scale
+    out, simt = both(ops, x2, w2)
+    assert torch.equal(out[[3, M - 1]], simt[[3, M - 1]]) and torch.equal(out[:, [0, N - 1]], simt[:, [0, N - 1]])
+    rest = [i for i in range(M) if i not in (3, M - 1)]
+    assert torch.equal(out[rest][:, 1:-1], clean[rest][:, 1:-1])
+    x2[3], x2[M - 1] = 0, x[M - 1]                          # a row of zeros; a row with one ordinary value
+    x2[M - 1, 1:] *= scale
+    out, simt = both(ops, x2, w2)
+    assert (out[3] == 0).all() and torch.equal(out[rest[:3]][:, 1:-1], clean[rest[:3]][:, 1:-1])
+    # one product, of which the parts leave out 2^-24, and what is 2^-30 of it
+    torch.testing.assert_close(out[M - 1, 1:-1], (x2[M - 1, 0] * w[:, 0])[1:-1], rtol=2 ** -22, atol=0)
+
+
+@SHAPES
+def test_infinities_and_sums_beyond_the_range(ops, M, N, K):
+    x, w = operands(M, N, K)
+    clean, _ = both(ops, x, w)
+    inf = float("inf")
+    for places in ([(0, inf)], [(K - 1, -inf)], [(1, inf), (K - 2, -inf)], [(5, float("nan"))]):
+        x2, w2 = x.clone(), w.clone()
+        for k, v in places:
+            x2[M - 1, k], w2[N - 1, k] = v, v
+        out, simt = both(ops, x2, w2)
+        assert same(out[M - 1], simt[M - 1]) and same(out[:, N - 1], simt[:, N - 1])
+        assert torch.equal(out[:-1, :-1], clean[:-1, :-1])
+    x2 = x.clone()
+    x2[M - 1] *= 1e37                                       # some of the sums are beyond the range, and parts of others on the way
+    out, simt = both(ops, x2, w)
+    over = ~out[M - 1].isfinite()
+    assert over.any() and not over.all() and same(out[M - 1][over], simt[M - 1][over])
+    assert out[M - 1][simt[M - 1].isfinite()].isfinite().all() and torch.equal(out[:-1], clean[:-1])
+
+
+@SHAPES
+def test_values_above_the_largest_bfloat16(ops, M, N, K):
+    x, w = operands(M, N, K)
+    x[M - 1] = 0
+    x[M - 1, 7], x[M - 1, K - 1] = 3.395e38, -torch.finfo(torch.float32).max
+    w *= 0.01
+    out, _ = both(ops, x, w)
+    want = x[M - 1].to(F64) @ w.to(F64).T
+    size = x[M - 1].abs().to(F64) @ w.abs().to(F64).T
+    assert ((out[M - 1].to(F64) - want).abs() <= 2 ** -22 * size).all()
+
+
+@SHAPES
+def test_sums_near_the_smallest_number(ops, M, N, K):
+    """Sums that fp32 holds with fewer bits, by operands of ordinary size: what multiply-adds give."""
+    x, w = operands(M, N, K)
+    out, simt = both(ops, x * 1e-20, w * 1e-20)
+    assert simt.abs().max() < 1e-37 and torch.equal(out, simt)
+    x[1] *= 1e-20                                           # beside others: the row by itself
+    out, simt = both(ops, x, w * 1e-17)
+    want = x.to(F64) @ (w * 1e-17).to(F64).T
+    off, off_simt = ((o.to(F64) - want)[1].norm() for o in (out, simt))
+    assert off <= off_simt
+
+
+def test_operands_of_one_sign(ops):
+    """The tensor cores cut sums off instead of rounding them, always to one side: still no further off than multiply-adds."""
+    g = torch.Generator().manual_seed(1)
+    for K in (512, 4096):
+        x, w = torch.rand(40, K, generator=g).cuda(), torch.rand(516, K, generator=g).cuda()
+        want = x.to(F64) @ w.to(F64).T
+        off, off_simt = ((o.to(F64) - want).norm() for o in both(ops, x, w))
+        assert off <= off_simt
