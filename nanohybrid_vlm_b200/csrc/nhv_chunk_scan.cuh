@@ -127,14 +127,15 @@ static __device__ __forceinline__ void cs_products(float* out, const float* a, c
 }
 
 // Two floats as the three bfloat16 each that they consist of: what is left, rounded to eight bits, three times.  Exact (to the
-// nearest: cut off, the parts would all have the value's sign, and what the products leave out would add up); infinities turn into
-// values that are no number.
+// nearest: cut off, the parts would all have the value's sign, and what the products leave out would add up) from 7.7e-34 on; above
+// bfloat16's largest number, 3.39e38, the first part is that; infinities turn into values that are no number.
 struct CsParts { uint32_t part[3]; };
 static __device__ __forceinline__ CsParts cs_cut(float x, float y) {
   CsParts c;
 #pragma unroll
   for (int i = 0; i < 3; ++i) {
-    asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(c.part[i]) : "f"(y), "f"(x));
+    if (i == 0) asm("cvt.rn.satfinite.bf16x2.f32 %0, %1, %2;\n" : "=r"(c.part[i]) : "f"(y), "f"(x));
+    else asm("cvt.rn.bf16x2.f32 %0, %1, %2;\n" : "=r"(c.part[i]) : "f"(y), "f"(x));
     x -= __uint_as_float(c.part[i] << 16);
     y -= __uint_as_float(c.part[i] & 0xffff0000u);
   }

@@ -93,3 +93,25 @@ def test_a_value_that_is_no_number(ops, kind, bad):
             rest = [i for i in range(H * dv) if i != col - v]
             assert torch.equal(got[:token], clean[:token]) and torch.equal(got[:, rest], clean[:, rest])
             assert not torch.isfinite(got[token, col - v])
+
+
+@pytest.mark.parametrize("kind", ["delta", "ssd", "mlstm"])
+def test_a_value_above_the_largest_bfloat16(ops, kind):
+    """A number that a bfloat16 rounds to an infinity: it moves its column from its token on, and nothing before or beside."""
+    H, d, dv, T = 40, 64, 64, 70
+    ins, run, plain, (q, k, v) = scans(ops, kind, H, d, dv, T, torch.Generator().manual_seed(5))
+    ins[0][:, :v] *= 1e-3 if kind != "ssd" else 1           # (no product beyond the range: the sums are numbers)
+    if kind == "ssd":
+        ins[0][:, H * dv:] *= 1e-3
+    clean = run(ins, False)
+    for token in (0, 1, 34, 68):
+        for col in (v, v + 17, v + 40):
+            big = [ins[0].clone(), ins[1]]
+            big[0][token, col] = 3.4e38
+            got = run(big, False)
+            rest = [i for i in range(H * dv) if i != col - v]
+            assert torch.equal(got[:token], clean[:token]) and torch.equal(got[:, rest], clean[:, rest])
+            # (delta rule: a head may keep more than half of what it holds, so that sums may leave the range)
+            if kind == "ssd":
+                want = plain(big)[token:, col - v]
+                assert ((got[token:, col - v].to(F64) - want).abs() <= 1e-5 * want.abs().max()).all()
