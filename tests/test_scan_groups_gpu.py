@@ -3,7 +3,7 @@ part, heads of less than a kernel's width, requests that end at, before and behi
 import pytest
 import torch
 
-from test_muvonex_ops_gpu import F64, delta_inputs, dev, plain_delta, plain_ssd
+from test_muvonex_ops_gpu import F64, delta_inputs, dev, plain_delta, plain_ssd, step_batch
 from test_nomudra_ops_gpu import mlstm_inputs, plain_scan
 from test_scan_paths_gpu import TOL, cancellation, rows, scans, walk
 
@@ -115,3 +115,22 @@ def test_a_value_above_the_largest_bfloat16(ops, kind):
             if kind == "ssd":
                 want = plain(big)[token:, col - v]
                 assert ((got[token:, col - v].to(F64) - want).abs() <= 1e-5 * want.abs().max()).all()
+
+
+@pytest.mark.parametrize("length", [32, 33, 64, 5])
+def test_one_product_enters_the_state_as_it_is(ops, length):
+    """The last token alone brings a value, at full weight: the state is key times value, exact in 32 bits.  (What is given back to
+    sums that the tensor cores cut off stays below half a unit of the last place, so that exact ones stay.)"""
+    H, d, dv = 8, 64, 32
+    g = torch.Generator().manual_seed(7)
+    proj = torch.randn(length, 2 * H * d + H * dv, generator=g)
+    proj[:, H * d:2 * H * d] = 2.0 ** torch.randint(-3, 4, (length, H * d), generator=g)
+    proj[:-1, 2 * H * d:] = 0
+    gates = torch.zeros(length, 2 * H)
+    gates[-1, :H] = 40.0                                    # the largest input gate by far: its weight is exp(0)
+    state = torch.zeros(1, ops.mlstm_state_floats(H, d, dv), device="cuda")
+    o = torch.empty(length, H * dv, device="cuda")
+    ops.CHUNK_SCAN_TOKENS = 4
+    ops.mlstm_scan(o, dev(proj), dev(gates), dev(torch.zeros(2 * H)), 15.0, state, step_batch([length], [0], [0]), H, d, dv)
+    k, v = proj[-1, H * d:2 * H * d].view(H, 1, d), proj[-1, 2 * H * d:].view(H, dv, 1)
+    assert torch.equal(state[0, :H * dv * d].view(H, dv, d).cpu(), k * v)
