@@ -100,6 +100,10 @@ class CausalLM:
                     out.append((w, mode))
         return out
 
+    def scratch_bytes(self, tokens: int, requests: int) -> int:
+        """The most that one part's kernels take as scratch in a step of up to so many tokens and requests."""
+        return max((obj.scratch_bytes(tokens, requests) for _, obj in self._uses), default=0)
+
     # ------------------------------------------------------------------ cache needs
     def cache_needs(self) -> list[PagedKVNeed | FixedStateNeed | None]:
         """For every run of the order: what its layer keeps between steps (None: nothing).  A run that reads another

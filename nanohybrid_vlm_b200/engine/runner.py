@@ -118,7 +118,7 @@ class ModelRunner:
         T = self.config.max_num_batched_tokens
         per_token = (3 * widest + 6 * self.model.spec.hidden_size) * item
         logits = self.config.max_num_seqs * self.vocab_size * (4 + item)
-        return 2 * T * per_token + 2 * logits + (256 << 20)
+        return 2 * T * per_token + 2 * logits + (256 << 20) + self.model.scratch_bytes(T, min(T, self.config.max_num_seqs))
 
     def _size_pools(self, num_slots: int) -> int:
         cfg = self.config

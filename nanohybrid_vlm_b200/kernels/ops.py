@@ -269,6 +269,21 @@ def _chunk_scratch(n_tokens: int, batch, groups: int, heads: int, rows: int, col
     return torch.empty(floats, dtype=torch.float32, device=device)
 
 
+def chunk_scratch_bytes(n_tokens: int, n_seqs: int, groups: int, heads: int, rows: int) -> int:
+    """The most that ``_chunk_scratch`` takes in steps of up to so many tokens and requests (chunks: 128 tokens a request and more)."""
+    if rows > 128 or rows % 4:
+        return 0
+    chunks = n_tokens // 32 + min(n_seqs, n_tokens // 128)
+    return 4 * chunks * library.load_library().nhv_chunk_scan_floats(groups, heads, rows)
+
+
+def mlstm_chunk_scratch_bytes(n_tokens: int, n_seqs: int, heads: int, rows: int) -> int:
+    """The same for ``mlstm_scan`` (32 tokens a request and more)."""
+    if rows > 128 or rows % 4:
+        return 0
+    return 4 * library.load_library().nhv_mlstm_chunk_floats(n_tokens, min(n_seqs, n_tokens // 32), heads, rows)
+
+
 def delta_rule(o, qkv, ba, a_log, dt_bias, state, batch, G: int, H: int, d: int, dv: int, fixed_order: bool = False) -> None:
     """The gated delta rule over the step's tokens.  qkv [T, 2*G*d + H*dv] (q, k, v after their convolutions), ba
     [T, 2*H] float32 (inputs of beta's sigmoid, then of the decay's softplus), a_log / dt_bias [H] float32, state
@@ -763,6 +778,17 @@ def moe_sorted_rows(n_slots: int, n_experts: int, tile: int) -> int:
     return -(-rows // tile) * tile
 
 
+def moe_scratch_bytes(n_slots: int, n_experts: int, width: int, ff: int, dtype) -> int:
+    """The most that ``moe_experts`` takes for steps of up to ``n_slots`` (token, choice) slots: the experts' rows in their
+    order, before, between and behind the products."""
+    item = 2 if dtype == torch.bfloat16 else 4
+    mma = dtype == torch.bfloat16 and width % 8 == 0 and ff % 8 == 0
+    if mma and n_slots >= MOE_TCGEN05_SLOTS * n_experts:
+        return moe_sorted_rows(n_slots, n_experts, MOE_TCGEN05_TILE) * (2 * width + ff) * item
+    tile = (64 if n_slots >= 24 * n_experts else 16) if mma else MOE_TILE_SIMT
+    return moe_sorted_rows(n_slots, n_experts, tile) * (width + ff) * item
+
+
 def moe_align(ids, n_experts: int, tile: int):
     """Order the slots of ids [T, top] by expert (choices >= n_experts, identity experts, take no row).  Returns
     (sorted_slots [rows] int32: slot of each row or -1, slot_pos [T * top] int32: row of each slot or -1,
@@ -808,6 +834,7 @@ def _first_product(gate, up):
 MOE_ON_TENSOR_CORES = True      # tests switch it off to compare with the CUDA-core products at the same shapes
 MOE_TILE = 0                    # rows per tile of the mma.sync products: 0 chooses by the step; tests set 16, 64, 128
 MOE_TCGEN05 = None              # the tcgen05 products: None where an expert sees many rows; tests set True (always) or False
+MOE_TCGEN05_SLOTS = 96          # slots per expert from which the step takes them
 MOE_TCGEN05_TILE = 256          # rows per tile of the tcgen05 products (ROWS of csrc/moe_tcgen05.cu)
 
 
@@ -827,7 +854,7 @@ def moe_experts(x, gate, up, down, ids, limit: float, alpha: float, up_shift: fl
     tile = MOE_TILE_SIMT
     if mma:
         tile = MOE_TILE or (128 if ids.numel() >= 192 * E else 64 if ids.numel() >= 24 * E else 16)
-    if mma and (MOE_TCGEN05 or (MOE_TCGEN05 is None and not MOE_TILE and ids.numel() >= 96 * E)):
+    if mma and (MOE_TCGEN05 or (MOE_TCGEN05 is None and not MOE_TILE and ids.numel() >= MOE_TCGEN05_SLOTS * E)):
         return _moe_experts_tcgen05(x, gate, up, down, ids, limit, alpha, up_shift, row_scale)
     sorted_slots, slot_pos, tile_expert = moe_align(ids, E, tile)
     rows = sorted_slots.numel()

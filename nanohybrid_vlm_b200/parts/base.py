@@ -148,6 +148,11 @@ class Part:
         engine may keep a second copy of each, laid out for the weight-streaming kernel.  Default: none."""
         return []
 
+    def scratch_bytes(self, tokens: int, requests: int) -> int:
+        """What a step of up to so many tokens and requests takes on the device beside the tensors that are as wide as one
+        of the part's matrices (which the engine counts by itself): the kernels' scratch.  Default: none."""
+        return 0
+
     def new(self, *shape, dtype=None) -> torch.Tensor:
         return torch.empty(*shape, dtype=dtype or self.env.dtype, device=self.env.device)
 

@@ -63,6 +63,9 @@ class GatedDeltaRule(Mixer):
     def streamed_weights(self):
         return [(self.w_qkvg, 0), (self.w_o, 0)]
 
+    def scratch_bytes(self, tokens, requests):
+        return ops.chunk_scratch_bytes(tokens, requests, self.G, self.H, self.d) if self.env.dtype != torch.float32 else 0
+
     def forward(self, x, batch, cache):
         T = x.shape[0]
         C = self.conv_channels

@@ -53,6 +53,9 @@ class MLSTM(Mixer):
     def streamed_weights(self):
         return [(self.w_qkvg, 0), (self.w_o, 0)]
 
+    def scratch_bytes(self, tokens, requests):
+        return ops.mlstm_chunk_scratch_bytes(tokens, requests, self.H, self.d) if self.env.dtype != torch.float32 else 0
+
     def forward(self, x, batch, cache):
         T = x.shape[0]
         qk, v = self.qk_size, self.v_size

@@ -146,6 +146,9 @@ class RoutedMoE(FeedForward):
     def streamed_weights(self):
         return self.shared.streamed_weights() if self.shared is not None else []
 
+    def scratch_bytes(self, tokens, requests):
+        return ops.moe_scratch_bytes(tokens * self.top, self.E, self.env.hidden_size, self.inter, self.env.dtype)
+
     def forward(self, x, batch):
         T, W = x.shape
         router = self.w_router

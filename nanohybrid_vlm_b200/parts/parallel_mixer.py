@@ -52,6 +52,9 @@ class ParallelMixers(Mixer):
     def streamed_weights(self):
         return [w for side in self.sides for w in side.streamed_weights()]
 
+    def scratch_bytes(self, tokens, requests):
+        return max(side.scratch_bytes(tokens, requests) for side in self.sides)
+
     def forward_normed_terms(self, x, batch, cache):
         return tuple((side.forward(x, batch, view), scale, w)
                      for side, view, scale, w in zip(self.sides, cache.children, self.scales, self.side_weights))

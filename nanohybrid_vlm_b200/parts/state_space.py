@@ -66,6 +66,9 @@ class Mamba2(Mixer):
     def streamed_weights(self):
         return [(self.w_in_main, 0), (self.w_o, 0)]
 
+    def scratch_bytes(self, tokens, requests):
+        return ops.chunk_scratch_bytes(tokens, requests, self.G, self.heads, self.N) if self.env.dtype != torch.float32 else 0
+
     def forward(self, x, batch, cache):
         T = x.shape[0]
         conv_state, ssm_state = cache.children[0].state, cache.children[1].state
