@@ -201,7 +201,7 @@ __global__ void attn_paged_simt_kernel(const T* __restrict__ q, int q_stride, T*
 
 // ---------------------------------------------------------------- head sizes in steps of 4
 // The kernel above reads one float of K and one of q from shared memory per multiply-add and waits for every chunk of
-// keys: 320 us for 370 tokens (37 to 210 a request) of 16 heads of 128; this one takes 80.  For heads of up to 256
+// keys: 320 us for 370 tokens (37 to 210 a request) of 16 heads of 128; this one takes 55.  For heads of up to 256
 // elements in steps of four, in rows that can be read 16 (bf16: 8) bytes at a time:
 //   - a warp takes its pairs (up to 4 or 8) through a chunk together, so that a key's four elements, read once, serve all of
 //     them, and likewise a value's; q and the probabilities are broadcast reads of four;
@@ -474,10 +474,12 @@ NHV_API int nhv_attention_simt_ex(int dtype, const void* q, int q_stride, void* 
     const size_t smem = ((size_t)stages * AT_CHUNK * (d + 4 + (planes == 2 ? dv : 0)) + (size_t)most * (d + AT_CHUNK)) * 4;
     const int most_smem = (stages * AT_CHUNK * (256 + 4 + 256) + most * (256 + AT_CHUNK)) * 4;
     const dim3 grid(n_tokens / TQ + n_seqs, nkv, (G + GS - 1) / GS);
-    // portions of a prompt: the block's 32 pairs over eight warps, so that one waits while another works (16 heads over 8 of 128 in
-    // fp32, prompts of 37, 123 and 210 tokens: 72 us with four warps of 8 pairs, 58 with eight of 4); few pairs a block (single
-    // tokens): four
-    const bool many = n_tokens >= 4 * n_seqs;
+    // Portions of a prompt: a block's pairs over eight warps, so that one waits while another works, where that leaves each half as
+    // many or one: more than 16 pairs (32 is all that a block takes), or 5 to 8.  In us, four and eight warps, requests of 300 tokens
+    // that get n more, 16 heads over 8 of 128 in fp32: eight of 4 57 and 43, of 8 57 and 71, of 12 88 and 81, of 32 102 and 96; three
+    // prompts of 37, 123 and 210 tokens 63 and 55.  Single tokens, mostly: four.
+    const int per_request = (n_tokens + n_seqs - 1) / n_seqs, pairs = GS * (per_request < TQ ? per_request : TQ);
+    const bool many = n_tokens >= 4 * n_seqs && (pairs > 16 || (pairs > 4 && pairs <= 8));
 #define LAUNCH_WARPS(T, VC, WARPS)                                                                                  \
   do {                                                                                                              \
     static std::atomic<uint64_t> done{0};                                                                           \
