@@ -203,3 +203,17 @@ def test_dyntanh_over_the_stream(ops, dtype, width, T):
                 torch.testing.assert_close(s.cpu().to(F64), kept, **tol(torch.float32))
                 seen.append((out.cpu(), s.cpu()))
             assert torch.equal(seen[0][0], seen[1][0]) and torch.equal(seen[0][1], seen[1][1])
+
+
+# pieces of x and w on their way at once: one, two, four and eight, and a second round of each; few and many outputs
+@pytest.mark.parametrize("K", [8, 256, 264, 512, 520, 1024, 1032, 2048, 2056, 4104])
+@pytest.mark.parametrize("M,N", [(3, 7), (700, 8)])
+def test_small_products_with_float32_sums(ops, K, M, N):
+    g = torch.Generator().manual_seed(K)
+    x, w = torch.randn(M, K, generator=g).bfloat16(), torch.randn(N, K, generator=g).bfloat16()
+    out = torch.full((M, N), float("nan"), device="cuda")
+    ops.linear_f32(out, dev(x), dev(w))
+    want = x.to(F64) @ w.to(F64).T
+    size = x.abs().to(F64) @ w.abs().to(F64).T
+    # 32-bit sums of exact products: K / 128 of a lane one after the other, then a tree of seven
+    assert ((out.cpu().to(F64) - want).abs() <= (K / 128 + 8) * 2 ** -24 * size).all()
