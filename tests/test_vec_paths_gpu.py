@@ -205,6 +205,24 @@ def test_dyntanh_over_the_stream(ops, dtype, width, T):
             assert torch.equal(seen[0][0], seen[1][0]) and torch.equal(seen[0][1], seen[1][1])
 
 
+# the three widths of a thread per four columns of each quarter, beside the tests of the other widths above
+@pytest.mark.parametrize("dtype", DTYPES)
+@pytest.mark.parametrize("width", [512, 1024, 2048])
+@pytest.mark.parametrize("n_addends,gathered", [(0, False), (1, False), (2, True), (3, False)])
+def test_norm_over_the_stream_by_quarters_has_the_same_bits(ops, dtype, width, n_addends, gathered):
+    g = torch.Generator().manual_seed(width + n_addends)
+    T, coefs = 70, (0.7, -1.25, 2.0)
+    stream, w = torch.randn(T, width, generator=g) * 3, (1 + 0.2 * torch.randn(width, generator=g)).to(dtype)
+    adds = [torch.randn(T, width, generator=g).to(dtype) for _ in range(n_addends)]
+    rows, seen = torch.randperm(T, generator=g)[:33].int() if gathered else None, []
+    for place in (lambda t: t, off_by_one):
+        s, out = place(dev(stream)), place(torch.full((33 if gathered else T, width), float("nan"), dtype=dtype, device="cuda"))
+        ops.rmsnorm_stream(out, s, place(dev(w)), 1e-5, [(place(dev(a)), c) for a, c in zip(adds, coefs)],
+                           rows=dev(rows) if gathered else None, weight_offset=1.0)
+        seen.append((out.cpu(), s.cpu()))
+    assert seen[0][0].isfinite().all() and torch.equal(seen[0][0], seen[1][0]) and torch.equal(seen[0][1], seen[1][1])
+
+
 # pieces of x and w on their way at once: one, two, four and eight, and a second round of each; few and many outputs
 @pytest.mark.parametrize("K", [8, 256, 264, 512, 520, 1024, 1032, 2048, 2056, 4104])
 @pytest.mark.parametrize("M,N", [(3, 7), (700, 8)])
