@@ -233,20 +233,21 @@ CHUNK_SCAN_TOKENS = 0
 def _by_chunks(n_tokens: int, n_seqs: int, longest: int, blocks: int, sms: int, normed: bool) -> bool:
     """Whether a scan goes by chunks.  ``blocks``: (head, 16 columns) of a request, ``longest``: tokens of its longest portion.
 
-    Device time (heads of 128 rows, 2,048 columns of state in all, us by chunks / by tokens).  By tokens a request's chain
-    costs 0.25 us a token as long as all blocks run at once; by chunks 0.08, but all of the SMs' time.  So chunks
-    win where few requests make a long chain.  Delta rule, requests of 512 tokens: 50 / 135 (one), 79 / 166 (2), 147 / 189 (4),
-    279 / 303 (8); 370 / 734 (5 of 333 to 1,501); 133 / 121 (8 of 200), 314 / 243 (48 of 80); the state space 37 / 104, 54 / 140,
-    97 / 154, 189 / 227, 250 / 485, 88 / 92 and 216 / 172 alike.  Hence a bound on all blocks' tokens over the longest.  The
-    mLSTM's scan by tokens costs more, and chunks win everywhere from 32 tokens a request on: 56 / 189 (one of 512), 78 / 185 (8 of
-    128), 133 / 273 (48 of 32).
+    By tokens a request's chain costs 0.25 us a token as long as all blocks run at once; by chunks 0.08, but all of the SMs' time:
+    chunks win where few requests make a long chain.  Hence a bound on all blocks' tokens over the longest.  Short steps wait
+    for the host, not for the device, and chunks take one to three launches more per layer: hence a long chain, or much work in all.
 
-    Short steps wait for the host, not for the device, and chunks take one to three launches more per layer, 15 to 60 us
-    a step of four layers.  Whole steps (with scans by chunks that took 1.5 times as long as now), widths 1,024 and 2,048: Muvonex, one prompt of 512 tokens 1,337 / 1,273 and 1,363 /
-    1,381, of 768 1,353 / 1,454 and 1,380 / 1,676, two of 512 1,373 / 1,348 and 1,497 / 1,682, four of 400 1,452 / 1,441 and
-    2,021 / 1,920; Nomudra, one of 512 1,712 / 1,689
-    and 1,707 / 1,717, of 768 1,730 / 1,778 and 1,724 / 1,880, four of 400 1,843 / 1,826 and 2,015 / 2,412, eight of 128 1,867 /
-    1,844 and 1,875 / 1,891.  Hence a long chain, or much work in all."""
+    The bounds were set when the scan by chunks took 1.5 times as long as now, by whole steps (us by chunks / by tokens, widths
+    1,024 and 2,048): Muvonex, one prompt of 512 tokens 1,337 / 1,273 and 1,363 / 1,381, of 768 1,353 / 1,454 and 1,380 / 1,676, two
+    of 512 1,373 / 1,348 and 1,497 / 1,682, four of 400 1,452 / 1,441 and 2,021 / 1,920; Nomudra, one of 512 1,712 / 1,689 and 1,707 /
+    1,717, of 768 1,730 / 1,778 and 1,724 / 1,880, four of 400 1,843 / 1,826 and 2,015 / 2,412, eight of 128 1,867 / 1,844 and
+    1,875 / 1,891.  They were not moved since.  Device time now, heads of 128 rows, 2,048 columns of state in all, a layer:
+      delta rule / state space by chunks: one of 2,048 166 against 527 / 111 against 404, 5 of 333 to 1,501 374 against 734 / 250 against 485;
+      left by tokens although chunks are faster on the device: one of 512 135 against 50 / 104 against 37, 4 of 512 189 against
+        147 / 154 against 97, 8 of 512 303 against 279 / 227 against 189;
+      by tokens, and as fast or faster: 8 of 200 121 against 133 / 92 against 88, 48 of 80 243 against 314 / 172 against 216;
+      mLSTM by chunks: 8 of 128 78 against 185, 48 of 32 133 against 273; one of 512 by tokens, 189 against 56.
+    """
     if CHUNK_SCAN_TOKENS:
         return n_tokens >= CHUNK_SCAN_TOKENS * n_seqs
     work = n_tokens * blocks
@@ -1380,17 +1381,15 @@ def linear(out, x, weight) -> None:
         torch.mm(x, weight.t(), out=out)
 
 
-F32_ON_TENSOR_CORES = True      # tests switch it off to compare with the CUDA-core product at the same shapes
-
-
 def _f32_on_tensor_cores(x, weight) -> bool:
     """Whether a float32 product runs on the tensor cores, operands cut into three bfloat16 (csrc/gemm_f32_tcgen05.cu).  By the
     weight's sizes alone, never by the number of tokens: so a token's result does not depend on what it is computed with.
-    In us on the CUDA cores / the tensor cores: a weight of 512 x 512 12 / 9 for 1 to 16 tokens, 16 / 13 for 128 and 35 / 19 for 2,048;
-    256 x 256 8 / 12; 4,096 x 1,024 28 / 14 for 16 tokens, 88 / 38 for 370; 43,392 x 1,024 65 / 69 for 1 to 8 tokens, 140 / 89 for 33.
+    In us on the CUDA cores / the tensor cores, weights from memory: 512 x 512 12 / 9 for 1 to 16 tokens, 16 / 13 for 128 and 35 / 19 for
+    2,048; 256 x 256 8 / 12; 4,096 x 1,024 28 / 14 for 16 tokens, 88 / 38 for 370.  Heads of K = 1,024 lose for few rows what they gain for
+    many: 43,392 x 1,024 65 / 69 for 1 to 8, 140 / 89 for 33; 151,936 x 1,024 178 / 203 for 1, 182 / 211 for 16, 459 / 268 for 33.
     Infinities, and values and sums of any size, give what the CUDA cores give."""
     N, K = weight.shape
-    return (F32_ON_TENSOR_CORES and N >= 512 and K >= 512 and K % 4 == 0 and x.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0
+    return (N >= 512 and K >= 512 and K % 4 == 0 and x.stride(0) % 4 == 0 and x.data_ptr() % 16 == 0
             and weight.data_ptr() % 16 == 0)
 
 
