@@ -1,5 +1,7 @@
 import os
+import shutil
 import sys
+import tempfile
 
 import pytest
 
@@ -29,6 +31,17 @@ TINY_C = dict(architectures=["Qwen3ForCausalLM"], model_type="qwen3", hidden_siz
 
 def pytest_configure(config):
     config.addinivalue_line("markers", "gpu: needs a CUDA device (run on a B200)")
+    # Some 300 tests start a Python process of their own.  Where the environment forbids bytecode beside the sources, each of
+    # them compiled torch's 850 modules again (1.3 s of its 4); here they share a folder of bytecode for the session.
+    if os.environ.pop("PYTHONDONTWRITEBYTECODE", None) and "PYTHONPYCACHEPREFIX" not in os.environ:
+        config.bytecode_folder = os.environ["PYTHONPYCACHEPREFIX"] = tempfile.mkdtemp(prefix="pyc_")
+
+
+def pytest_unconfigure(config):
+    folder = getattr(config, "bytecode_folder", None)
+    if folder is not None:
+        os.environ.pop("PYTHONPYCACHEPREFIX", None)
+        shutil.rmtree(folder, ignore_errors=True)
 
 
 @pytest.fixture(scope="session")
