@@ -2,8 +2,8 @@
 // multiply-adds: each operand is cut into three bfloat16 of eight bits, which hold it exactly (7.7e-34 and more), and a product is
 // the six products of their parts down to 2^-16 of the largest (what is left out is below 2^-24 of it and of either sign).
 // Rows of smaller values, sums below 1.2e-35 and sums that are no finite number are multiplied again on the CUDA cores, by
-// themselves: infinities and the whole range of fp32 give what they give there.  Looking for them costs up to 3 % for 1 to 16 rows
-// (4096 x 1024 13.6 and 14.0 us, 43392 x 1024 66.2 and 68.9); a row is looked at until it shows a larger value, which
+// themselves: infinities and the whole range of fp32 give what they give there.  Looking for them costs up to 4 % for 1 to 16 rows
+// (6144 x 1024 14.2 and 14.5 us, 43392 x 1024 65.8 and 69.0); a row is looked at until it shows a larger value, which
 // ordinary rows do at once.
 //
 // Sums.  The tensor cores cut off what lies below a sum's last place.  So the products of first parts are added up over 64
@@ -24,8 +24,8 @@
 //
 // What bounds it: the way of a stage from global memory to its parts, about 2 us for 64 columns of both operands (1.1 where A
 // has up to 32 rows), beside 1,536 cycles of the tensor pipe, whose MMAs read all that shared memory gives.  In us, on the CUDA cores
-// and here, for 370 rows: N x K = 4096 x 1024 88 and 38, 1024 x 2048 159 and 20, 6144 x 1024 115 and 39, 1024 x 3072 238 and 26; for 16
-// rows 28 and 14, 42 and 14, 34 and 15, 62 and 19; 43392 x 1024, 3 and 33 rows: 65 and 69, 140 and 89.  Not faster: W two stages
+// and here, weights from memory, for 370 rows: N x K = 4096 x 1024 88 and 37, 1024 x 2048 159 and 19, 6144 x 1024 115 and 38, 1024 x 3072
+// 238 and 25; for 16 rows 28 and 14, 42 and 14, 34 and 15, 62 and 18; 43392 x 1024, 3 and 33 rows: 65 and 69, 140 and 89.  Not faster: W two stages
 // ahead in registers with the MMAs issued by an adding warp (41 against 37 for 370 x 4096 x 1024 in one run).
 #define NHV_WAIT_LIMIT (1u << 22)
 #include "nhv_async.cuh"
@@ -395,20 +395,24 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tcgen05_kernel(const Para
       for (int i = 0; i < PER; ++i) tile[(row0 + i) * TILE + col] = s_abort ? __int_as_float(0x7fc00000) : acc[i];
     cluster_sync();
     if (const int t = THREADS - 1 - (int)threadIdx.x; t < TILE + NT) {      // (threads that have the least to do below)
-      uint32_t size = 0;
-      for (int q = 0; q < p.split; ++q) size |= cluster_load(&s_size[t], (uint32_t)q);
-      s_small[t] = size == 0x100;
+      uint32_t size[MAX_SPLIT];                                  // (all runs' on their way at once)
+#pragma unroll
+      for (int q = 0; q < MAX_SPLIT; ++q) size[q] = q < p.split ? cluster_load(&s_size[t], (uint32_t)q) : 0u;
+      s_small[t] = (size[0] | size[1] | size[2] | size[3]) == 0x100;
       again = s_small[t];
     }
     // the runs in order
     for (int e = threadIdx.x; e < share * (TILE / 4); e += THREADS) {
       const int r = first + e / (TILE / 4), c = 4 * (e % (TILE / 4));
       if (m0 + r >= p.M || n0 + c >= p.N) continue;
-      float4 sum = cluster_load4(tile + r * TILE + c, 0);
-      for (int q = 1; q < p.split; ++q) {
-        const float4 v = cluster_load4(tile + r * TILE + c, (uint32_t)q);
-        sum.x += v.x; sum.y += v.y; sum.z += v.z; sum.w += v.w;
-      }
+      float4 run[MAX_SPLIT];
+#pragma unroll
+      for (int q = 0; q < MAX_SPLIT; ++q)
+        if (q < p.split) run[q] = cluster_load4(tile + r * TILE + c, (uint32_t)q);
+      float4 sum = run[0];
+#pragma unroll
+      for (int q = 1; q < MAX_SPLIT; ++q)
+        if (q < p.split) { sum.x += run[q].x; sum.y += run[q].y; sum.z += run[q].z; sum.w += run[q].w; }
       float* at = p.C + (size_t)(m0 + r) * p.ldc + n0 + c;
       const float v[4] = {sum.x, sum.y, sum.z, sum.w};
 #pragma unroll
