@@ -3,8 +3,7 @@
 // the six products of their parts down to 2^-16 of the largest (what is left out is below 2^-24 of it and of either sign).
 // Rows of smaller values, sums below 1.2e-35 and sums that are no finite number are multiplied again on the CUDA cores, by
 // themselves: infinities and the whole range of fp32 give what they give there.  Looking for them costs up to 4 % for 1 to 16 rows
-// (6144 x 1024 14.2 and 14.5 us, 43392 x 1024 65.8 and 69.0); a row is looked at until it shows a larger value, which
-// ordinary rows do at once.
+// (6144 x 1024 14.2 and 14.4 us, 43392 x 1024 65.8 and 68.5); ordinary rows show a larger value in their last stage.
 //
 // Sums.  The tensor cores cut off what lies below a sum's last place.  So the products of first parts are added up over 64
 // columns only (four MMAs) in tensor memory and then added to a sum in registers, rounded to the nearest; the five kinds of
@@ -250,9 +249,8 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tcgen05_kernel(const Para
         }
       }
     };
-    // bits 0 to 3: this thread's rows of W that hold a value of SMALL_ROW or more, 4 to 7: of A; 8 to 15: any that is not zero.  Once a
-    // row has such a value in this thread's columns, mostly in the first stage, it is not looked at again.
-    constexpr unsigned W_ROWS = 0xf, A_ROWS = NT == 128 ? 0xf0 : 0x10;
+    // bits 0 to 3: this thread's rows of W that hold a value of SMALL_ROW or more, 4 to 7: of A; 8 to 15: any that is not zero
+    constexpr unsigned ROWS = NT == 128 ? 0xff : 0x1f;
     unsigned sizes = 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
@@ -292,18 +290,27 @@ __global__ void __launch_bounds__(THREADS, 1) gemm_f32_tcgen05_kernel(const Para
       if (s >= STAGES && !mbar_wait(&empty[slot], (uint32_t)((s / STAGES) - 1) & 1, 1)) { s_abort = 1; break; }
       unsigned char* to = smem + (size_t)slot * STAGE_BYTES;
       hint(s + 4);
-      if ((sizes & W_ROWS) != W_ROWS) look(w, 1u);
       put(w, to, W_PART);
       if (s + 1 < stages) load(w, p.W, p.N, p.K, n0, s + 1);
-      if ((sizes & A_ROWS) != A_ROWS) look(a, 16u);
       put(a, to + 3 * W_PART, A_PART);
       if (s + 1 < stages) load(a, p.A, p.M, p.lda, m0, s + 1);
       asm volatile("fence.proxy.async.shared::cta;\n" ::: "memory");
       __syncwarp();
       if (lane == 0) mbar_arrive(&full[slot]);
     }
+    // The rows' sizes: the last stage, still in registers, says enough of ordinary rows, while its products are made; where a row
+    // has nothing but small values there, the others are read again.
+    for (int s = -1; s + 1 < stages; ++s) {
+      if (s >= 0) {
+        load(w, p.W, p.N, p.K, n0, s);
+        load(a, p.A, p.M, p.lda, m0, s);
+      }
+      look(w, 1u);
+      look(a, 16u);
 #pragma unroll
-    for (int d = 1; d < 8; d <<= 1) sizes |= __shfl_xor_sync(0xffffffffu, sizes, d);
+      for (int d = 1; d < 8; d <<= 1) sizes |= __shfl_xor_sync(0xffffffffu, sizes, d);
+      if (__all_sync(0xffffffffu, (sizes & ROWS) == ROWS)) break;
+    }
     if (c == 0) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) s_size[r0 + 32 * i] = sizes >> i & 0x101;
